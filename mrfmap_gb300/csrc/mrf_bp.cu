@@ -74,50 +74,68 @@ __global__ void __launch_bounds__(kPrepThreads)
 }
 
 // ---- ray messages ----------------------------------------------------------
-// One warp per ray.  Each lane owns kE = 4 consecutive incidences of a
-// chunk of 128 (ray offsets are padded to multiples of 4, so the streams load
-// as 16-byte vectors): the prefix over the ray is a serial sum inside the
-// lane plus one warp scan per chunk, and a lane keeps 4 gathers in flight.
+// A group of kG lanes per ray, 32 / kG rays per warp.  Each lane owns kE = 4
+// consecutive incidences of a chunk of 4 kG (ray offsets are padded to
+// multiples of 4, so the streams load as 16-byte vectors).
 //
-// Pass 1 forms the visibility exponent A_i = sum_{j<=i} l_j ln q_j,
-// V_i = exp(A_i), q_i and the Pre total T over the whole ray.  Pass 2 turns
+// With k4 = k_dyn rounded down to 4, every potential before k4 is zero: the
+// static prefix [0, k4) only contributes its sum of l ln q, which needs no
+// scan: a lane-strided sum and one group reduction, split at r0 into la
+// (before r0) and lb.  From k4 on, C_i = sum_{k4 <= j <= i} l_j ln q_j is a
+// serial prefix inside the lane plus one group scan per chunk.  Pre
+// visibility restarts at r0 (the reference restores its carried state only
+// once the accumulated tau is non-zero, gvdbkernels.cu:708-715):
+//   e_i = V^pre_i = exp(C_i + A_{k4-1} - A_{r0-1}),  V_i = exp(A_{r0-1}) e_i,
+// so one exponential per incidence serves both passes.  r0 <= k_dyn on every
+// ray in the queues; where it lies behind k4 it is in the first vector.
+//
+// Pass 1 forms the Pre total T = sum e_i (1 - q_i) mu_i.  Pass 2 turns
 // (V_i mu_i, q_i, l_i) and T into the messages p_i * l_i of the dynamic
-// range [k_dyn, n_post) only: before k_dyn every potential is zero, so
-// tau_i = 0, F_i = 0, mu1_i = 0 and p_i is exactly the clamp floor F_EPS
-// (static messages, summed once per build into the pairs).  Potentials are
-// loaded from k_dyn (rounded down to a vector) on.  Pass 2 re-reads the
-// dynamic range (a sixth of the incidences, mostly still in L1/L2) from
-// A_{k_dyn - 1} instead of keeping pass 1's slice in registers: the kernel
-// then fits 40 registers, twelve resident blocks per SM.  On rays longer
-// than kLongRay the Pre total T is summed across lanes in FP64 and the
-// running difference T - F of pass 2 is carried in FP64; each lane's share
-// of T is a compensated FP32 sum.  (GB300 issues FP64 at 1/64 of the FP32
-// rate, so FP64 stays out of the per-incidence arithmetic.)
+// range [k4, n_post) only: before k_dyn tau_i = 0, F_i = 0, mu1_i = 0 and p_i
+// is exactly the clamp floor F_EPS (static messages, summed once per build
+// into the pairs).  A warp whose rays all end inside their first chunk keeps
+// it in registers for pass 2; otherwise pass 2 re-reads the dynamic range.
+// On rays longer than kLongRay the Pre total T is summed across lanes in FP64
+// and the running difference T - F of pass 2 is carried in FP64; each lane's
+// share of T is a compensated FP32 sum.  (GB300 issues FP64 at 1/64 of the
+// FP32 rate, so FP64 stays out of the per-incidence arithmetic.)
 //
 // The ln q gathers are the kernel's cost.  Pairs are numbered brick-major
 // by first visit (mrf_build.cu), so consecutive incidences of a ray gather
 // from nearby addresses and neighbouring rays from the same ones.
 //
-// Pre visibility restarts at r0 (the reference restores its carried state
-// only once the accumulated tau is non-zero, gvdbkernels.cu:708-715):
-// V^pre_i = exp(A_i - A_{r0-1}) = V_i * exp(-A_{r0-1}); Post uses V_i.
+// Why groups of 8: a 1 cm ray holds about 60 incidences from k4 on and 30
+// loud ones before it, so a whole warp per ray (chunks of 128) left half its
+// lanes idle and paid the scans, reductions and the ticket once per ray: 850
+// warp instructions a ray, bound by issue.  Four rays a warp take 300 and
+// the kernel waits for memory (issue slots 30 % busy).  Whole Gauss-Seidel
+// iteration, 8 x 640x480 at 1 cm, third iteration on: 2.61 ms with a warp
+// per ray, 1.97 with 8 lanes, 2.25 with 16, 2.11 with 4; all rays in full
+// 3.24, 2.92, 2.94, 3.20; Jacobi, 32 views at 2 cm: 1.86, 1.44, 1.60, 1.51.
+// Eight incidences a lane (chunks of 64, fewer warps) and the next rays'
+// records fetched a ray ahead: no faster.
 constexpr int kRayWarps = 4;
+constexpr int kG = 8;                    // lanes per ray
+constexpr int kRaysPerWarp = 32 / kG;
 constexpr int kE = 4;                    // incidences per lane of a chunk
-constexpr int kChunk = 32 * kE;          // 128
-constexpr float kUnderflowGuard = -60.0f;
+constexpr int kChunk = kG * kE;
+constexpr int kLoudPer = 4;              // loud prefix incidences in flight per lane
 
-template <typename T>
-__device__ __forceinline__ T warp_excl_scan(T v, int lane) {
-  T incl = warp_incl_scan(v, lane);
-  return incl - v;
+// inclusive scan and sum over the lanes of a group (gl: lane in the group)
+__device__ __forceinline__ float group_incl_scan(float v, int gl) {
+#pragma unroll
+  for (int o = 1; o < kG; o <<= 1) {
+    const float u = __shfl_up_sync(kFull, v, o, kG);
+    if (gl >= o) v += u;
+  }
+  return v;
 }
-
-// one lane's slice of a chunk (KE incidences).  ln q is kept; q itself is
-// formed only where a potential is non-zero or a message is computed.
-template <int KE>
-struct Slice {
-  float A[KE], lq[KE], mu[KE], len[KE];
-};
+template <typename T>
+__device__ __forceinline__ T group_sum(T v) {
+#pragma unroll
+  for (int o = kG / 2; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
+  return v;
+}
 
 // streamed incidence arrays: read-only path (kPol 0) or evict-first
 // streaming loads (kPol 1) that leave L2 to the ln q gathers
@@ -127,75 +145,28 @@ __device__ __forceinline__ T ld_stream(const T* p) {
   return __ldg(p);
 }
 
-template <typename T>
-__device__ __forceinline__ T from_bits(uint32_t u);
-template <>
-__device__ __forceinline__ uint32_t from_bits<uint32_t>(uint32_t u) { return u; }
-template <>
-__device__ __forceinline__ float from_bits<float>(uint32_t u) { return __uint_as_float(u); }
-
-// KE consecutive values at element i (i a multiple of KE; KE = 2 or a
-// multiple of 4): 8-byte or 16-byte vector loads, zeros when !ok
-template <int KE, int kPol, typename T>
-__device__ __forceinline__ void ld_vec(T (&out)[KE], const T* __restrict__ base, int i, bool ok) {
-  static_assert(sizeof(T) == 4, "4-byte elements");
-  if constexpr (KE % 4 == 0) {
-#pragma unroll
-    for (int v = 0; v < KE / 4; ++v) {
-      uint4 u = make_uint4(0u, 0u, 0u, 0u);
-      if (ok) u = ld_stream<kPol>(reinterpret_cast<const uint4*>(base + i + 4 * v));
-      out[4 * v + 0] = from_bits<T>(u.x);
-      out[4 * v + 1] = from_bits<T>(u.y);
-      out[4 * v + 2] = from_bits<T>(u.z);
-      out[4 * v + 3] = from_bits<T>(u.w);
-    }
-  } else {
-    static_assert(KE == 2, "short chunks hold two incidences per lane");
-    uint2 u = make_uint2(0u, 0u);
-    if (ok) u = ld_stream<kPol>(reinterpret_cast<const uint2*>(base + i));
-    out[0] = from_bits<T>(u.x);
-    out[1] = from_bits<T>(u.y);
-  }
+// four consecutive values at element i (a multiple of 4) as one vector load,
+// zeros when !ok
+template <int kPol>
+__device__ __forceinline__ void ld4(uint32_t (&out)[kE], const uint32_t* __restrict__ base, uint32_t i, bool ok) {
+  uint4 u = make_uint4(0u, 0u, 0u, 0u);
+  if (ok) u = ld_stream<kPol>(reinterpret_cast<const uint4*>(base + i));
+  out[0] = u.x;
+  out[1] = u.y;
+  out[2] = u.z;
+  out[3] = u.w;
 }
-
-// a lane's KE pair ids at i0 (those >= n read as zero)
-template <int KE, int kPol>
-__device__ __forceinline__ void load_pids(uint32_t (&pid)[KE], uint32_t off, int i0, int n,
-                                          const uint32_t* __restrict__ inc_pair) {
-  if constexpr (KE % 4 == 0) {
-#pragma unroll
-    for (int v = 0; v < KE / 4; ++v) {
-      uint32_t t[4];
-      ld_vec<4, kPol>(t, inc_pair + off, i0 + 4 * v, i0 + 4 * v < n);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) pid[4 * v + j] = t[j];
-    }
-  } else {
-    ld_vec<KE, kPol>(pid, inc_pair + off, i0, i0 < n);
-  }
+template <int kPol>
+__device__ __forceinline__ void ld4(float (&out)[kE], const float* __restrict__ base, uint32_t i, bool ok) {
+  float4 u = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  if (ok) u = ld_stream<kPol>(reinterpret_cast<const float4*>(base + i));
+  out[0] = u.x;
+  out[1] = u.y;
+  out[2] = u.z;
+  out[3] = u.w;
 }
-
-// ln q of a lane's KE incidences (those >= n read as zero; kWhole: the
-// whole chunk lies inside the ray and nothing is checked)
-__device__ __forceinline__ float to_f(float v) { return v; }
-__device__ __forceinline__ float to_f(__half v) { return __half2float(v); }
-
-template <int KE, bool kWhole, typename TQ>
-__device__ __forceinline__ void gather_lq(float (&lq)[KE], const uint32_t (&pid)[KE], int i0, int n,
-                                          const TQ* __restrict__ lnq) {
-#pragma unroll
-  for (int j = 0; j < KE; ++j) lq[j] = (kWhole || i0 + j < n) ? to_f(__ldg(lnq + pid[j])) : 0.0f;
-}
-
-// VW lengths at element i of base (fp32: one 16-byte vector; fp16: one
-// 8-byte vector of four halves), zeros when !ok
-template <int VW, int kPol>
-__device__ __forceinline__ void ld_len(float (&out)[VW], const float* __restrict__ base, int i, bool ok) {
-  ld_vec<VW, kPol>(out, base, i, ok);
-}
-template <int VW, int kPol>
-__device__ __forceinline__ void ld_len(float (&out)[VW], const __half* __restrict__ base, int i, bool ok) {
-  static_assert(VW == 4, "fp16 lengths load four at a time");
+template <int kPol>
+__device__ __forceinline__ void ld4(float (&out)[kE], const __half* __restrict__ base, uint32_t i, bool ok) {
   uint2 u = make_uint2(0u, 0u);
   if (ok) u = ld_stream<kPol>(reinterpret_cast<const uint2*>(base + i));
   const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&u.x));
@@ -205,390 +176,322 @@ __device__ __forceinline__ void ld_len(float (&out)[VW], const __half* __restric
   out[2] = b.x;
   out[3] = b.y;
 }
+__device__ __forceinline__ float to_f(float v) { return v; }
+__device__ __forceinline__ float to_f(__half v) { return __half2float(v); }
 
-// with the lane's ln q gathered: loads lengths (and potentials at and after
-// kmu, a multiple of 4; below it they are known zeros), forms prefix
-// exponents from carryA; returns the chunk total of l ln q
-// (kLenIn: the lengths were loaded ahead into len_in)
-template <int KE, int kPol, bool kWhole, bool kLenIn = false, typename TL = float>
-__device__ __forceinline__ float slice_from_lq(Slice<KE>& s, const float (&lq)[KE], uint32_t off, int i0,
-                                               int n, int kmu, float carryA, int lane,
-                                               const TL* __restrict__ inc_len,
-                                               const float* __restrict__ inc_mu,
-                                               const float* len_in = nullptr) {
-  constexpr int VW = KE % 4 == 0 ? 4 : KE;  // vector width
+// one lane's slice of a chunk from k4 on: lengths and potentials (zeros in
+// the ray's padding and past its end), ln q, the prefix exponents C
+struct Slice {
+  float len[kE], mu[kE], lq[kE], C[kE];
+};
+
+// with the lane's pair ids: gathers ln q, loads potentials (and lengths
+// unless kLenIn gave them), forms C from carry; returns the chunk's total
+template <int kPol, bool kLenIn, typename TL, typename TQ>
+__device__ __forceinline__ float load_slice(Slice& s, const uint32_t (&pid)[kE], uint32_t off, int i0, int n,
+                                            float carry, int gl, const TL* __restrict__ inc_len,
+                                            const float* __restrict__ inc_mu, const TQ* __restrict__ lnq) {
 #pragma unroll
-  for (int v = 0; v < KE / VW; ++v) {
-    const int i = i0 + VW * v;
-    float l[VW], m[VW];
-    if constexpr (kLenIn) {
-#pragma unroll
-      for (int j = 0; j < VW; ++j) l[j] = len_in[VW * v + j];
-    } else {
-      ld_len<VW, kPol>(l, inc_len + off, i, kWhole || i < n);
-    }
-    ld_vec<VW, kPol>(m, inc_mu + off, i, (kWhole || i < n) && i >= kmu);
-#pragma unroll
-    for (int j = 0; j < VW; ++j) {
-      s.len[VW * v + j] = l[j];
-      s.mu[VW * v + j] = m[j];
-    }
-  }
+  for (int j = 0; j < kE; ++j) s.lq[j] = i0 + j < n ? to_f(__ldg(lnq + pid[j])) : 0.0f;
+  if (!kLenIn) ld4<kPol>(s.len, inc_len, off + i0, i0 < n);
+  ld4<kPol>(s.mu, inc_mu, off + i0, i0 < n);
   float run = 0.0f;
 #pragma unroll
-  for (int j = 0; j < KE; ++j) {
-    const bool ok = kWhole || i0 + j < n;
-    s.lq[j] = ok ? lq[j] : 0.0f;
-    if (!ok) {
-      s.len[j] = 0.0f;
-      s.mu[j] = 0.0f;
-    }
-    run += s.len[j] * lq[j];
-    s.A[j] = run;  // lane-local inclusive prefix, rebased below
+  for (int j = 0; j < kE; ++j) {
+    run += s.len[j] * s.lq[j];
+    s.C[j] = run;
   }
-  float ex = warp_excl_scan(run, lane);
-  float b = carryA + ex;
+  const float incl = group_incl_scan(run, gl);
+  const float b = carry + (incl - run);
 #pragma unroll
-  for (int j = 0; j < KE; ++j) s.A[j] += b;
-  return __shfl_sync(kFull, ex + run, 31);
+  for (int j = 0; j < kE; ++j) s.C[j] += b;
+  return __shfl_sync(kFull, incl, kG - 1, kG);
 }
 
-template <int KE, int kPol, bool kWhole, bool kLenIn = false, typename TL = float, typename TQ = float>
-__device__ __forceinline__ float slice_from_pids(Slice<KE>& s, const uint32_t (&pid)[KE], uint32_t off,
-                                                 int i0, int n, int kmu, float carryA, int lane,
-                                                 const TL* __restrict__ inc_len,
-                                                 const float* __restrict__ inc_mu,
-                                                 const TQ* __restrict__ lnq,
-                                                 const float* len_in = nullptr) {
-  float lq[KE];
-  gather_lq<KE, kWhole>(lq, pid, i0, n, lnq);
-  return slice_from_lq<KE, kPol, kWhole, kLenIn, TL>(s, lq, off, i0, n, kmu, carryA, lane, inc_len, inc_mu,
-                                                    len_in);
-}
-
-template <int KE, int kPol, bool kWhole, typename TL, typename TQ>
-__device__ __forceinline__ float load_slice(Slice<KE>& s, uint32_t off, int i0, int n, int kmu,
-                                            float carryA, int lane,
-                                            const uint32_t* __restrict__ inc_pair,
-                                            const TL* __restrict__ inc_len,
-                                            const float* __restrict__ inc_mu,
-                                            const TQ* __restrict__ lnq) {
-  uint32_t pid[KE];
-  load_pids<KE, kPol>(pid, off, i0, kWhole ? i0 + KE : n, inc_pair);
-  return slice_from_pids<KE, kPol, kWhole, false, TL, TQ>(s, pid, off, i0, n, kmu, carryA, lane, inc_len,
-                                                          inc_mu, lnq);
-}
-
-// A at chunk-relative index idx (0 <= idx < 32 * KE), broadcast to the warp
-template <int KE>
-__device__ __forceinline__ float slice_value(const Slice<KE>& s, int idx) {
-  const int jj = idx % KE;
-  float mine = 0.0f;
-#pragma unroll
-  for (int j = 0; j < KE; ++j)
-    if (j == jj) mine = s.A[j];
-  return __shfl_sync(kFull, mine, idx / KE);
-}
-
-// pass 2 on one lane's slice: messages p*l for positions i0..i0+KE-1; the
-// vectors starting inside [k4, n_post) are written (k4 a multiple of 4).
-// cF is F at the chunk start and D = T - cF, formed in the ray's
-// accumulation type by the caller; returns the chunk's total of tau.
-template <int KE, bool kWhole>
-__device__ __forceinline__ float emit_slice(const float (&vmu)[KE], const float (&q)[KE],
-                                            const float (&len)[KE], int i0, int k4, int n_post,
-                                            float cF, float D, int lane, uint32_t off,
-                                            float* __restrict__ inc_pl) {
-  float tau[KE], eloc[KE];
-  float run = 0.0f;
-#pragma unroll
-  for (int j = 0; j < KE; ++j) {
-    tau[j] = (kWhole || i0 + j < n_post) ? vmu[j] * (1.0f - q[j]) : 0.0f;
-    eloc[j] = run;
-    run += tau[j];
-  }
-  float ex = warp_excl_scan(run, lane);
-  float out[KE];
-#pragma unroll
-  for (int j = 0; j < KE; ++j) {
-    float fin = ex + eloc[j];
-    float F = cF + fin;
-    float R = (D - fin) - tau[j];
-    float mu1 = F + vmu[j];
-    float mu0 = F + __fdividef(R, q[j]);
-    float p = clampf(__fdividef(mu1, mu1 + mu0 + 1e-7f), kFEps, 1.0f - kFEps);
-    out[j] = (kWhole || i0 + j < n_post) ? p * len[j] : 0.0f;
-  }
-  constexpr int VW = KE % 4 == 0 ? 4 : KE;
-#pragma unroll
-  for (int v = 0; v < KE / VW; ++v) {
-    const int i = i0 + VW * v;
-    if (i >= k4 && (kWhole || i < n_post)) {
-      if constexpr (VW == 4)
-        *reinterpret_cast<float4*>(inc_pl + off + i) =
-            make_float4(out[4 * v], out[4 * v + 1], out[4 * v + 2], out[4 * v + 3]);
-      else
-        *reinterpret_cast<float2*>(inc_pl + off + i) = make_float2(out[2 * v], out[2 * v + 1]);
-    }
-  }
-  return __shfl_sync(kFull, ex + run, 31);
-}
-
-// Pass-1 bookkeeping of one slice: A_{r0-1}, A_{rinf-1} and A_{k4-1} where
-// those positions fall inside it
-template <int KE>
-__device__ __forceinline__ void pre_marks(const Slice<KE>& s, int base, int r0, int rinf, int k4,
-                                          float& Ar0, float& Arinf, float& Ak) {
-  constexpr int CH = 32 * KE;
-  if (r0 - 1 >= base && r0 - 1 < base + CH) Ar0 = slice_value<KE>(s, r0 - 1 - base);
-  if (rinf - 1 >= base && rinf - 1 < base + CH) Arinf = slice_value<KE>(s, rinf - 1 - base);
-  if (k4 - 1 >= base && k4 - 1 < base + CH) Ak = slice_value<KE>(s, k4 - 1 - base);
-}
-
-// the lane's share of the Pre total from one slice that may hold non-zero
-// potentials, added to a compensated FP32 sum (ts, tc): the error of the
-// lane's sum stays at a few ulps however long the ray is
-template <int KE>
-__device__ __forceinline__ void pre_total(const Slice<KE>& s, int i0, int r0, float Ar0, float& ts,
-                                          float& tc) {
-  // exp(-A_{r0-1}) rescales Post visibility to Pre visibility unless the
-  // Post visibility may have underflowed (then exponentiate the difference)
-  const bool direct = Ar0 < kUnderflowGuard;
-  const float scale = direct ? 0.0f : __expf(-Ar0);
-  float w = 0.0f;
-#pragma unroll
-  for (int j = 0; j < KE; ++j) {
-    if (i0 + j >= r0 && s.mu[j] != 0.0f) {
-      float vp = direct ? __expf(s.A[j] - Ar0) : __expf(s.A[j]) * scale;
-      w += vp * (1.0f - __expf(s.lq[j])) * s.mu[j];
-    }
-  }
-  const float y = w - tc;
-  const float t = ts + y;
-  tc = (t - ts) - y;
-  ts = t;
-}
-
-template <typename Acc, int kPol, int kPf, typename TL, typename TQ>
-__device__ __forceinline__ void ray_bp_warp(const RayMeta& me, uint32_t rid, const QuietPrefix& qp,
-                                            const uint32_t* __restrict__ inc_pair,
-                                            const TL* __restrict__ inc_len,
-                                            const float* __restrict__ inc_mu,
-                                            const TQ* __restrict__ lnq, float* __restrict__ inc_pl,
-                                            int fix_reset, int lane) {
+// One ray per group (me.n_pre = me.n_post = 0: the group has none).
+template <int kPol, int kPf, bool kQuiet, typename TL, typename TQ>
+__device__ __forceinline__ void ray_bp_group(const RayMeta& me, uint32_t rid, const QuietPrefix& qp,
+                                             const uint32_t* __restrict__ inc_pair,
+                                             const TL* __restrict__ inc_len,
+                                             const float* __restrict__ inc_mu,
+                                             const TQ* __restrict__ lnq, float* __restrict__ inc_pl,
+                                             int fix_reset, int gl) {
   const int n_pre = me.n_pre, n_post = me.n_post;
   const int r0 = fix_reset ? 0 : me.r0;
-  const int rinf = fix_reset ? 0 : me.rinf;
-  const int kdyn = ray_kdyn(me);
-  const int k4 = kdyn & ~3;
+  const int k4 = ray_kdyn(me) & ~3;
   const uint32_t off = me.off;
-  float carryA = 0.0f, Ar0 = 0.0f, Arinf = 0.0f, Ak = 0.0f;
-  // ---- the static prefix [0, k4) from its quiet sums --------------------
-  // Its quiet incidences (pairs on voxels without a dynamic incidence in
-  // any view) keep their ln q from the third iteration of a call on, so
-  // their sums up to r0 and up to k4 were formed once (k_quiet_prefix);
-  // only the prefix's loud incidences are gathered here.  A ray in the
-  // queues has a non-zero potential, so its rinf equals r0.
-  const int start = qp.q ? k4 : 0;
   // kPf >= 1: the first chunk's pair ids are requested before the static
   // prefix's loads, so the two chains of dependent loads overlap
   uint32_t pid_next[kE];
   float len_next[kE];
-  if (kPf) load_pids<kE, kPol>(pid_next, off, start + kE * lane, n_pre, inc_pair);
-  if (kPf == 2) ld_len<kE, kPol>(len_next, inc_len + off, start + kE * lane, start + kE * lane < n_pre);
-  if (qp.q) {
-    const float2 qv = qp.q[rid];
-    const uint32_t e0 = qp.loff[rid], e1 = qp.loff[rid + 1];
-    float la = 0.0f, lk = 0.0f;
-    for (uint32_t e = e0 + lane; e < e1; e += 32) {
-      const float c = qp.llen[e] * to_f(__ldg(lnq + qp.lpid[e]));
-      lk += c;
-      if ((int)qp.lpos[e] < r0) la += c;
+  if (kPf) ld4<kPol>(pid_next, inc_pair, off + k4 + kE * gl, k4 + kE * gl < n_pre);
+  if (kPf == 2) ld4<kPol>(len_next, inc_len, off + k4 + kE * gl, k4 + kE * gl < n_pre);
+  // ---- the static prefix [0, k4): sums of l ln q before and from r0 --------
+  float la = 0.0f, lb = 0.0f;
+  if (kQuiet) {
+    // Its quiet incidences (pairs on voxels without a dynamic incidence in
+    // any view) keep their ln q from the third iteration of a call on, so
+    // their sums were formed once (k_quiet_prefix); only the prefix's loud
+    // incidences are gathered here, kLoudPer per lane at a time (the list
+    // is short and its loads depend on one another: what counts is how many
+    // are in flight).
+    QuietRay qr = {};
+    if (n_pre) {
+      const uint4 u = __ldg(reinterpret_cast<const uint4*>(qp.ray) + rid);
+      qr = *reinterpret_cast<const QuietRay*>(&u);
     }
-    lk = warp_sum(lk);
-    la = warp_sum(la);
-    carryA = qv.y + lk;
-    Ak = carryA;
-    if (!fix_reset && r0 <= k4) {
-      Ar0 = qv.x + la;
-      Arinf = Ar0;
+    const int nl = (int)qr.na + (int)qr.nb;
+    for (int i = gl; i < nl; i += kG * kLoudPer) {
+      uint2 en[kLoudPer];
+#pragma unroll
+      for (int k = 0; k < kLoudPer; ++k) {
+        en[k] = make_uint2(0u, 0u);
+        if (i + k * kG < nl) en[k] = ld_stream<kPol>(qp.loud + qr.first + i + k * kG);
+      }
+#pragma unroll
+      for (int k = 0; k < kLoudPer; ++k) {
+        const float c = i + k * kG < nl ? __uint_as_float(en[k].y) * to_f(__ldg(lnq + en[k].x)) : 0.0f;
+        if (i + k * kG < (int)qr.na) la += c;
+        else lb += c;
+      }
     }
-  }
-  // ---- pass 1: prefixes, Pre total ---------------------------------------
-  // Chunks of 128 (a chunk costs the same instructions however many of its
-  // lanes hold incidences: measured against 256-incidence chunks and against
-  // 256-incidence chunks with 64- or 128-incidence tails, this was fastest).
-  // Chunks wholly inside the ray skip the bounds checks; chunks wholly
-  // before k4 hold no potential and skip the Pre-total work.  kPf 1: the
-  // next chunk's pair ids are requested before this chunk's ln q gathers;
-  // kPf 2: its lengths as well.
-  float ts = 0.0f, tc = 0.0f;
-  Slice<kE> s;
-  {
-    float len[kE];
-    for (int base = start; base < n_pre; base += kChunk) {
-      const int i0 = base + kE * lane;
-      uint32_t pid[kE];
+    la = group_sum(la) + qr.qa;
+    lb = group_sum(lb) + qr.qb;
+    if (fix_reset) {
+      lb += la;
+      la = 0.0f;
+    }
+  } else {
+    // k4 is a multiple of 4: no vector crosses it
+    uint32_t p[kE];
+    if (kPf) ld4<kPol>(p, inc_pair, off + kE * gl, kE * gl < k4);
+    for (int i = kE * gl; i < k4; i += kChunk) {
+      uint32_t c[kE];
+      float l[kE];
       if (kPf) {
 #pragma unroll
-        for (int j = 0; j < kE; ++j) pid[j] = pid_next[j];
-        if (kPf == 2) {
-#pragma unroll
-          for (int j = 0; j < kE; ++j) len[j] = len_next[j];
-        }
-        if (base + kChunk < n_pre) {
-          load_pids<kE, kPol>(pid_next, off, i0 + kChunk, n_pre, inc_pair);
-          if (kPf == 2) ld_len<kE, kPol>(len_next, inc_len + off, i0 + kChunk, i0 + kChunk < n_pre);
-        }
+        for (int j = 0; j < kE; ++j) c[j] = p[j];
+        ld4<kPol>(p, inc_pair, off + i + kChunk, i + kChunk < k4);
       } else {
-        load_pids<kE, kPol>(pid, off, i0, n_pre, inc_pair);
+        ld4<kPol>(c, inc_pair, off + i, true);
       }
-      const float tot =
-          base + kChunk <= n_pre
-              ? slice_from_pids<kE, kPol, true, kPf == 2>(s, pid, off, i0, n_pre, k4, carryA, lane, inc_len,
-                                                          inc_mu, lnq, len)
-              : slice_from_pids<kE, kPol, false, kPf == 2>(s, pid, off, i0, n_pre, k4, carryA, lane,
-                                                           inc_len, inc_mu, lnq, len);
-      pre_marks<kE>(s, base, r0, rinf, k4, Ar0, Arinf, Ak);
-      if (base + kChunk > k4) pre_total<kE>(s, i0, r0, Ar0, ts, tc);
-      carryA += tot;
+      ld4<kPol>(l, inc_len, off + i, true);
+#pragma unroll
+      for (int j = 0; j < kE; ++j) l[j] *= to_f(__ldg(lnq + c[j]));
+      if (i + kE <= r0) {
+        la += (l[0] + l[1]) + (l[2] + l[3]);
+      } else if (i >= r0) {
+        lb += (l[0] + l[1]) + (l[2] + l[3]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < kE; ++j) {
+          if (i + j < r0) la += l[j];
+          else lb += l[j];
+        }
+      }
     }
+    la = group_sum(la);
+    lb = group_sum(lb);
   }
-  // the lanes' compensated shares, summed in Acc once per ray (FP64 on
-  // rays longer than kLongRay)
-  Acc T = warp_sum((Acc)ts - (Acc)tc);
-  // infinity term: visibility at the end of Pre (gvdbkernels.cu:1196-1208)
-  if (me.flags & 1u) T += (Acc)__expf(carryA - Arinf);
-  if (kdyn >= n_post) return;  // every message of the ray is static
-  // ---- pass 2: dynamic messages ------------------------------------------
-  // F is zero before k_dyn, so the running F starts at zero at k4; the
-  // long-range difference T - F is carried in Acc, one subtraction per chunk
-  Acc Dd = T;
-  float cF = 0.0f;
-  float carryA2 = Ak;
-  for (int base = k4; base < n_post; base += kChunk) {
-    const int i0 = base + kE * lane;
-    const bool full = base + kChunk <= n_post;
-    const float tot2 =
-        full ? load_slice<kE, kPol, true>(s, off, i0, n_post, k4, carryA2, lane, inc_pair, inc_len, inc_mu,
-                                          lnq)
-             : load_slice<kE, kPol, false>(s, off, i0, n_post, k4, carryA2, lane, inc_pair, inc_len,
-                                           inc_mu, lnq);
-    carryA2 += tot2;
-    float vmu[kE], q[kE];
+  // ---- pass 1: Pre total ---------------------------------------------------
+  // kPf 1: the next chunk's pair ids are requested before this chunk's ln q
+  // gathers; kPf 2: its lengths as well.
+  float pre = lb;  // A_{k4-1} - A_{r0-1}; la: A_{r0-1}
+  float ts = 0.0f, tc = 0.0f, carry = 0.0f;
+  const int trips = __reduce_max_sync(kFull, (n_pre - k4 + kChunk - 1) / kChunk);
+  const bool behind = __any_sync(kFull, r0 > k4);
+  Slice s;
+  float e[kE], q[kE];
+  for (int t = 0; t < trips; ++t) {
+    const int i0 = k4 + t * kChunk + kE * gl;
+    uint32_t pid[kE];
+    if (kPf) {
+#pragma unroll
+      for (int j = 0; j < kE; ++j) pid[j] = pid_next[j];
+      if (kPf == 2) {
+#pragma unroll
+        for (int j = 0; j < kE; ++j) s.len[j] = len_next[j];
+      }
+      ld4<kPol>(pid_next, inc_pair, off + i0 + kChunk, i0 + kChunk < n_pre);
+      if (kPf == 2) ld4<kPol>(len_next, inc_len, off + i0 + kChunk, i0 + kChunk < n_pre);
+    } else {
+      ld4<kPol>(pid, inc_pair, off + i0, i0 < n_pre);
+    }
+    carry += load_slice<kPol, kPf == 2>(s, pid, off, i0, n_pre, carry, gl, inc_len, inc_mu, lnq);
+    if (t == 0 && behind) {
+      // r0 behind k4: A_{r0-1} lies in the first vector
+      const int m = r0 - 1 - k4;
+      const float c = __shfl_sync(kFull, m == 0 ? s.C[0] : (m == 1 ? s.C[1] : s.C[2]), 0, kG);
+      if (r0 > k4) {
+        la += c;
+        pre = -c;
+      }
+    }
+    float w = 0.0f;
 #pragma unroll
     for (int j = 0; j < kE; ++j) {
-      vmu[j] = __expf(s.A[j]) * s.mu[j];
+      e[j] = __expf(s.C[j] + pre);
       q[j] = __expf(s.lq[j]);
+      w += e[j] * s.mu[j] * (1.0f - q[j]);
     }
-    const float D = (float)Dd;
-    const float ct = full ? emit_slice<kE, true>(vmu, q, s.len, i0, k4, n_post, cF, D, lane, off, inc_pl)
-                          : emit_slice<kE, false>(vmu, q, s.len, i0, k4, n_post, cF, D, lane, off, inc_pl);
-    Dd -= (Acc)ct;
+    // compensated: the error of the lane's sum stays at a few ulps however
+    // long the ray is
+    const float y = w - tc;
+    const float u = ts + y;
+    tc = (u - ts) - y;
+    ts = u;
+  }
+  // The lanes' shares, summed once per ray, and the infinity term: visibility
+  // at the end of Pre (gvdbkernels.cu:1196-1208).  Rays longer than kLongRay
+  // sum and carry T in FP64 (Dd), the others in FP32 (Df).
+  const bool is_long = n_pre > kLongRay;
+  const bool any_long = __any_sync(kFull, is_long);
+  const float tinf = (me.flags & 1u) ? __expf(carry + pre) : 0.0f;
+  float Df = group_sum(ts - tc) + tinf;
+  double Dd = 0.0;
+  if (any_long) Dd = group_sum((double)ts - (double)tc) + (double)tinf;
+  // ---- pass 2: dynamic messages --------------------------------------------
+  // F is zero before k_dyn, so the running F starts at zero at k4; the
+  // long-range difference T - F is carried, one subtraction per chunk
+  const float ratio = __expf(la);
+  float cF = 0.0f;
+  carry = 0.0f;
+  const int trips2 = trips <= 1 ? trips : __reduce_max_sync(kFull, (n_post - k4 + kChunk - 1) / kChunk);
+  for (int t = 0; t < trips2; ++t) {
+    const int i0 = k4 + t * kChunk + kE * gl;
+    if (trips > 1) {
+      uint32_t pid[kE];
+      ld4<kPol>(pid, inc_pair, off + i0, i0 < n_post);
+      carry += load_slice<kPol, false>(s, pid, off, i0, n_post, carry, gl, inc_len, inc_mu, lnq);
+#pragma unroll
+      for (int j = 0; j < kE; ++j) {
+        e[j] = __expf(s.C[j] + pre);
+        q[j] = __expf(s.lq[j]);
+      }
+    }
+    float eloc[kE], run = 0.0f;
+#pragma unroll
+    for (int j = 0; j < kE; ++j) {
+      e[j] *= ratio * s.mu[j];  // V mu
+      eloc[j] = run;
+      run += e[j] * (1.0f - q[j]);
+    }
+    const float incl = group_incl_scan(run, gl);
+    const float ex = incl - run;
+    const float D = is_long ? (float)Dd : Df;
+    float out[kE];
+#pragma unroll
+    for (int j = 0; j < kE; ++j) {
+      const float fin = ex + eloc[j];
+      const float F = cF + fin;
+      const float R = (D - fin) - e[j] * (1.0f - q[j]);
+      const float mu1 = F + e[j];
+      const float mu0 = F + __fdividef(R, q[j]);
+      const float p = clampf(__fdividef(mu1, mu1 + mu0 + 1e-7f), kFEps, 1.0f - kFEps);
+      out[j] = i0 + j < n_post ? p * s.len[j] : 0.0f;
+    }
+    if (i0 < n_post)
+      *reinterpret_cast<float4*>(inc_pl + off + i0) = make_float4(out[0], out[1], out[2], out[3]);
+    const float ct = __shfl_sync(kFull, incl, kG - 1, kG);
+    Df -= ct;
+    if (any_long) Dd -= (double)ct;
     cF += ct;
   }
 }
 
-// Persistent launch: each warp takes the next ray from a work counter.
-// kReg false: one queue, rays longest first (sorted once per incidence
-// build, their RayMeta records copied into queue order), so the long rays
-// start early and the short ones fill the tail.  kReg true (SM-affine):
-// the view's pixels are cut into regions of consecutive pixels holding
-// equal shares of its incidences, one region per SM (block b serves
-// regions b mod G, + G, ..., G = min(grid, regions); a persistent grid is
-// placed on the SMs in block order, so a region's blocks share an SM); a
-// warp takes the home rays of its regions, then drains the view's leftover
-// queue of short rays.  The warps of one SM trace neighbouring rays at the
-// same time -- rays that cross the same voxels, so their ln q gathers hit
-// the SM's L1.  Which warp handles a ray does not change its result.  Variants differ only in register budget (kMinBlocks
-// resident blocks per SM), load policy and schedule: their arithmetic is
-// identical, so the autotuner's choice never changes a result.
-template <int kMinBlocks, int kPol, int kPf, bool kReg, typename TL, typename TQ>
-__global__ void __launch_bounds__(kRayWarps * 32, kMinBlocks) k_ray_bp(const RayMeta* __restrict__ queue,
-                                                           uint32_t n_rays,
-                                                           const uint32_t* __restrict__ rstart,
-                                                           uint32_t nreg, uint32_t rper,
-                                                           const uint32_t* __restrict__ lprefix,
-                                                           const uint32_t* __restrict__ lbase,
-                                                           uint32_t nlv,
-                                                           uint32_t* __restrict__ lcounter,
-                                                           uint32_t* __restrict__ counter,
-                                                           const uint32_t* __restrict__ inc_pair,
-                                                           const TL* __restrict__ inc_len,
-                                                           const float* __restrict__ inc_mu,
-                                                           const TQ* __restrict__ lnq,
-                                                           float* __restrict__ inc_pl,
-                                                           const uint32_t* __restrict__ ids,
-                                                           QuietPrefix qp, int fix_reset) {
+// Persistent launch: each warp takes its next kRaysPerWarp rays from a work
+// counter.  kReg false: one queue, rays longest first (sorted once per
+// incidence build, their RayMeta records copied into queue order), so the
+// long rays start early and the short ones fill the tail, and a warp's rays
+// have nearly equal lengths.  kReg true (SM-affine): the view's pixels are
+// cut into regions of consecutive pixels holding equal shares of its
+// incidences, one region per SM (block b serves regions b mod G, + G, ...,
+// G = min(grid, regions); a persistent grid is placed on the SMs in block
+// order, so a region's blocks share an SM); a warp takes the home rays of
+// its regions, then drains the view's leftover queue of short rays.  The
+// warps of one SM trace neighbouring rays at the same time -- rays that
+// cross the same voxels, so their ln q gathers hit the SM's L1.  Which group
+// handles a ray does not change its result.  Variants differ only in
+// register budget (kMinBlocks resident blocks per SM), load policy and
+// schedule: their arithmetic is identical, so the autotuner's choice never
+// changes a result.
+template <int kMinBlocks, int kPol, int kPf, bool kReg, bool kQuiet, typename TL, typename TQ>
+__global__ void __launch_bounds__(kRayWarps * 32, kMinBlocks)
+    k_ray_bp(const RayMeta* __restrict__ queue, uint32_t n_rays, const uint32_t* __restrict__ rstart,
+             uint32_t nreg, uint32_t rper, const uint32_t* __restrict__ lprefix,
+             const uint32_t* __restrict__ lbase, uint32_t nlv, uint32_t* __restrict__ lcounter,
+             uint32_t* __restrict__ counter, const uint32_t* __restrict__ inc_pair,
+             const TL* __restrict__ inc_len, const float* __restrict__ inc_mu, const TQ* __restrict__ lnq,
+             float* __restrict__ inc_pl, const uint32_t* __restrict__ ids, QuietPrefix qp, int fix_reset) {
   const int lane = threadIdx.x & 31;
-  auto ray_at = [&](uint32_t i) {
-    const RayMeta me = queue[i];
-    const uint32_t rid = qp.q ? ids[i] : 0u;
-    if (me.n_pre <= kLongRay)
-      ray_bp_warp<float, kPol, kPf, TL, TQ>(me, rid, qp, inc_pair, inc_len, inc_mu, lnq, inc_pl, fix_reset,
-                                            lane);
-    else
-      ray_bp_warp<double, kPol, kPf, TL, TQ>(me, rid, qp, inc_pair, inc_len, inc_mu, lnq, inc_pl, fix_reset,
-                                             lane);
+  const int gl = lane % kG;
+  const uint32_t grp = lane / kG;
+  // the warp's next tickets of counter c
+  auto take = [&](uint32_t* c) {
+    uint32_t t = 0;
+    if (lane == 0) t = atomicAdd(c, (uint32_t)kRaysPerWarp);
+    return __shfl_sync(kFull, t, 0);
   };
-  if constexpr (kReg) {
-    // counter[r]: tickets of region r, whose home rays are positions
-    // rstart[q (rper + 1) + rr] .. rstart[q (rper + 1) + rr + 1] (view q =
-    // r / rper, rr = r % rper).  Block b serves regions b mod G, + G, ...
-    // (G = min(grid, regions): every region has a home block).
-    const uint32_t G = min(gridDim.x, nreg);
-    for (uint32_t r = blockIdx.x % G; r < nreg; r += G) {
+  // the queue in use: kReg false, the whole queue (counter); kReg true, the
+  // home rays of region r (counter[r]: positions rstart[q (rper + 1) + rr] ..
+  // rstart[q (rper + 1) + rr + 1], view q = r / rper, rr = r % rper; block b
+  // serves regions b mod G, + G, ..., G = min(grid, regions): every region
+  // has a home block), then the views' leftovers (lcounter: ticket t is view
+  // q's (t - lprefix[q])-th leftover for the last q with lprefix[q] <= t)
+  const uint32_t G = kReg ? min(gridDim.x, nreg) : 1u;
+  uint32_t r = kReg ? blockIdx.x % G : 0u;
+  uint32_t first = 0, n = n_rays;
+  uint32_t* c = counter;
+  bool left = !kReg;
+  auto open = [&]() {
+    if (r < nreg) {
       const uint32_t q = r / rper;
       const uint32_t* rs = rstart + (size_t)q * (rper + 1) + (r - q * rper);
-      const uint32_t a = rs[0], nr = rs[1] - a;
-      // the next ticket is taken before the current ray runs, so its
-      // atomic's latency hides behind the ray's work
-      uint32_t idx = 0;
-      if (lane == 0) idx = atomicAdd(counter + r, 1u);
-      idx = __shfl_sync(kFull, idx, 0);
-      while (idx < nr) {
-        const uint32_t cur = a + idx;
-        if (lane == 0) idx = atomicAdd(counter + r, 1u);
-        idx = __shfl_sync(kFull, idx, 0);
-        ray_at(cur);
+      first = rs[0];
+      n = rs[1] - first;
+      c = counter + r;
+    } else {
+      left = true;
+      n = lprefix[nlv];
+      c = lcounter;
+    }
+  };
+  if (kReg) open();
+  // the record of the group's ray among the warp's tickets t..
+  auto record = [&](uint32_t t, RayMeta& me, uint32_t& rid) {
+    t += grp;
+    me = RayMeta{};
+    if (t >= n) return;
+    uint32_t pos = first + t;
+    if (kReg && left) {
+      uint32_t lo = 0, hi = nlv;
+      while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (lprefix[mid] <= t) lo = mid;
+        else hi = mid;
       }
+      pos = lbase[lo] + (t - lprefix[lo]);
     }
-    // the views' leftovers, one ticket counter over all of them: ticket t
-    // is view q's (t - lprefix[q])-th leftover for the last q with
-    // lprefix[q] <= t
-    const uint32_t n_left = lprefix[nlv];
-    auto leftover = [&]() {
-      uint32_t pos = 0xFFFFFFFFu;
-      if (lane == 0) {
-        const uint32_t t = atomicAdd(lcounter, 1u);
-        if (t < n_left) {
-          uint32_t lo = 0, hi = nlv;
-          while (hi - lo > 1) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (lprefix[mid] <= t) lo = mid;
-            else hi = mid;
-          }
-          pos = lbase[lo] + (t - lprefix[lo]);
-        }
-      }
-      return __shfl_sync(kFull, pos, 0);
-    };
-    uint32_t pos = leftover();
-    while (pos != 0xFFFFFFFFu) {
-      const uint32_t cur = pos;
-      pos = leftover();
-      ray_at(cur);
+    const uint4 u = __ldg(reinterpret_cast<const uint4*>(queue) + pos);
+    me = *reinterpret_cast<const RayMeta*>(&u);
+    if (kQuiet) rid = __ldg(ids + pos);
+  };
+  uint32_t idx = take(c);
+  for (;;) {
+    if (idx >= n) {
+      if (left) return;
+      r += G;
+      open();
+      idx = take(c);
+      continue;
     }
-  } else {
-    uint32_t idx = 0;
-    if (lane == 0) idx = atomicAdd(counter, 1u);
-    idx = __shfl_sync(kFull, idx, 0);
-    while (idx < n_rays) {
-      const uint32_t cur = idx;
-      if (lane == 0) idx = atomicAdd(counter, 1u);
-      idx = __shfl_sync(kFull, idx, 0);
-      ray_at(cur);
-    }
+    RayMeta me;
+    uint32_t rid = 0u;
+    record(idx, me, rid);
+    // the next tickets are taken before the current rays run, so the atomic's
+    // latency hides behind their work
+    idx = take(c);
+    ray_bp_group<kPol, kPf, kQuiet, TL, TQ>(me, rid, qp, inc_pair, inc_len, inc_mu, lnq, inc_pl, fix_reset, gl);
   }
 }
 
@@ -607,51 +510,57 @@ __global__ void k_ray_queue(const RayMeta* __restrict__ meta, const uint32_t* __
 // The static prefix of each queued ray of one view (rays r0..r0+n of the
 // pixel arrays; a warp per ray): the loud incidences in [0, k4) -- those
 // whose pair is among the view's first n_loud, the pairs on voxels with a
-// dynamic incidence in any view -- counted (emit false) or listed at
-// loff[r] (emit true: pair id, length, position), in ray order.
+// dynamic incidence in any view -- counted to loff[r] (emit false) or listed
+// from loud[loff[r]] on (emit true: pair id and length, in ray order; ray[r]
+// gets the list's start and its entries before and from r0 on).
 template <bool kEmit>
 __global__ void k_loud_prefix(const RayMeta* __restrict__ meta, uint32_t r_first, uint32_t n,
                               const uint32_t* __restrict__ inc_pair, const float* __restrict__ inc_len,
                               uint32_t pair_base, uint32_t n_loud, uint32_t* __restrict__ loff,
-                              uint32_t* __restrict__ lpid, float* __restrict__ llen,
-                              uint16_t* __restrict__ lpos) {
+                              uint2* __restrict__ loud, QuietRay* __restrict__ ray) {
   const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (w >= n) return;
   const uint32_t r = r_first + w;
   const RayMeta me = meta[r];
-  uint32_t cnt = 0;
-  uint32_t at = kEmit ? loff[r] : 0u;
+  uint32_t cnt = 0, na = 0;
+  const uint32_t first = kEmit ? loff[r] : 0u;
   if (ray_in_bp(me)) {
     const int k4 = ray_kdyn(me) & ~3;
     for (int b = 0; b < k4; b += 32) {
       const int j = b + lane;
       const uint32_t p = j < k4 ? inc_pair[me.off + j] : 0u;
-      const bool loud = j < k4 && p - pair_base < n_loud;
-      const unsigned m = __ballot_sync(kFull, loud);
-      if (kEmit && loud) {
-        const uint32_t e = at + (uint32_t)__popc(m & ((1u << lane) - 1u));
-        lpid[e] = p;
-        llen[e] = inc_len[me.off + j];
-        lpos[e] = (uint16_t)j;
+      const bool is_loud = j < k4 && p - pair_base < n_loud;
+      const unsigned m = __ballot_sync(kFull, is_loud);
+      if (kEmit) {
+        if (is_loud)
+          loud[first + cnt + (uint32_t)__popc(m & ((1u << lane) - 1u))] =
+              make_uint2(p, __float_as_uint(inc_len[me.off + j]));
+        na += (uint32_t)__popc(__ballot_sync(kFull, is_loud && j < (int)me.r0));
       }
-      at += (uint32_t)__popc(m);
       cnt += (uint32_t)__popc(m);
     }
   }
-  if (!kEmit && lane == 0) loff[r] = cnt;
+  if (lane) return;
+  if (kEmit) {
+    ray[r].first = first;
+    ray[r].na = (uint16_t)na;
+    ray[r].nb = (uint16_t)(cnt - na);
+  } else {
+    loff[r] = cnt;
+  }
 }
 
 // The quiet sums of the static prefix of each queued ray of one view (a
 // warp per ray): sum of l ln q over the quiet incidences j < min(r0, k4)
-// and j < k4, written to q[r] -- valid while the quiet pairs' ln q stay
+// and min(r0, k4) <= j < k4, written to ray[r] -- valid while the quiet pairs' ln q stay
 // fixed, from the third iteration of a call on.  Lane-strided partial
 // sums and a butterfly warp sum: a fixed order.
 template <typename TQ>
 __global__ void k_quiet_prefix(const RayMeta* __restrict__ meta, uint32_t r_first, uint32_t n,
                                const uint32_t* __restrict__ inc_pair, const float* __restrict__ inc_len,
                                const TQ* __restrict__ lnq, uint32_t pair_base, uint32_t n_loud,
-                               float2* __restrict__ q) {
+                               QuietRay* __restrict__ ray) {
   const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (w >= n) return;
@@ -665,13 +574,13 @@ __global__ void k_quiet_prefix(const RayMeta* __restrict__ meta, uint32_t r_firs
     const uint32_t p = inc_pair[me.off + j];
     if (p - pair_base >= n_loud) {
       const float c = inc_len[me.off + j] * to_f(__ldg(lnq + p));
-      qk += c;
       if (j < ra) qa += c;
+      else qk += c;
     }
   }
   qa = warp_sum(qa);
   qk = warp_sum(qk);
-  if (lane == 0) q[r] = make_float2(qa, qk);
+  if (lane == 0) *reinterpret_cast<float2*>(&ray[r].qa) = make_float2(qa, qk);
 }
 
 // ray queue of one build: active rays sorted by decreasing length
@@ -1177,13 +1086,28 @@ cudaError_t launch_pair_prepare(const BpArrays& a, uint32_t p0, uint32_t p1, int
 // ray-kernel variants: (id, resident-block target, load policy, chunk
 // prefetch, schedule: 0 longest first, 1 SM regions)
 #define MRF_RAY_VARIANTS(X) \
-  X(0, 0, 0, 0, 0) X(1, 0, 0, 1, 0) X(2, 0, 0, 2, 0) X(3, 0, 0, 0, 1) X(4, 0, 0, 1, 1) X(5, 0, 0, 2, 1) \
-  X(6, 12, 0, 1, 1) X(7, 12, 1, 1, 1)
+  X(0, 8, 0, 0, 0) X(1, 8, 0, 1, 0) X(2, 7, 0, 2, 0) X(3, 8, 0, 0, 1) X(4, 8, 0, 1, 1) X(5, 7, 0, 2, 1) \
+  X(6, 10, 0, 1, 1) X(7, 8, 1, 1, 1)
 constexpr int kRayVariants = 8;
 
 int ray_bp_variants() { return kRayVariants; }
 
 namespace {
+using RayKernel32 = decltype(&k_ray_bp<0, 0, 0, false, false, float, float>);
+using RayKernel16 = decltype(&k_ray_bp<0, 0, 0, false, false, __half, __half>);
+
+#define X(id, mb, pol, pf, sc) \
+  {k_ray_bp<mb, pol, pf, (sc > 0), false, float, float>, k_ray_bp<mb, pol, pf, (sc > 0), true, float, float>},
+const RayKernel32 kRay32[kRayVariants][2] = {MRF_RAY_VARIANTS(X)};
+#undef X
+#define X(id, mb, pol, pf, sc) \
+  {k_ray_bp<mb, pol, pf, (sc > 0), false, __half, __half>, k_ray_bp<mb, pol, pf, (sc > 0), true, __half, __half>},
+const RayKernel16 kRay16[kRayVariants][2] = {MRF_RAY_VARIANTS(X)};
+#undef X
+#define X(id, mb, pol, pf, sc) (sc > 0),
+const bool kRayRegions[kRayVariants] = {MRF_RAY_VARIANTS(X)};
+#undef X
+
 template <typename K>
 int resident_of(K kernel) {
   int per_sm = 0;
@@ -1195,22 +1119,13 @@ int resident_of(K kernel) {
 }
 }  // namespace
 
-int ray_bp_resident_blocks(int variant, int half_streams) {
-  static int resident[2][kRayVariants] = {{0}};
+int ray_bp_resident_blocks(int variant, int half_streams, int quiet) {
+  static int resident[2][2][kRayVariants] = {{{0}}};
   if (variant < 0 || variant >= kRayVariants) return 1;
-  const int h = half_streams ? 1 : 0;
-  if (!resident[h][variant]) {
-    switch (variant) {
-#define X(id, mb, pol, pf, sc)                                                                        \
-  case id:                                                                                            \
-    resident[h][variant] = h ? resident_of(k_ray_bp<mb, pol, pf, (sc > 0), __half, __half>)          \
-                             : resident_of(k_ray_bp<mb, pol, pf, (sc > 0), float, float>);           \
-    break;
-      MRF_RAY_VARIANTS(X)
-#undef X
-    }
-  }
-  return resident[h][variant];
+  int& r = resident[half_streams ? 1 : 0][quiet ? 1 : 0][variant];
+  if (!r)
+    r = half_streams ? resident_of(kRay16[variant][quiet ? 1 : 0]) : resident_of(kRay32[variant][quiet ? 1 : 0]);
+  return r;
 }
 
 cudaError_t launch_ray_bp(const BpArrays& a, const RayWork& w, int fix_reset, int num_sms, int variant,
@@ -1218,33 +1133,26 @@ cudaError_t launch_ray_bp(const BpArrays& a, const RayWork& w, int fix_reset, in
   if (!w.n_rays) return cudaSuccess;
   QuietPrefix qp{};
   if (quiet) {
-    qp.q = a.quiet_q;
-    qp.loff = a.loud_off;
-    qp.lpid = a.loud_pid;
-    qp.llen = a.loud_len;
-    qp.lpos = a.loud_pos;
+    qp.ray = a.quiet_ray;
+    qp.loud = a.loud;
   }
   if (variant < 0 || variant >= kRayVariants) return cudaErrorInvalidValue;
-  int64_t b = std::min<int64_t>((int64_t)num_sms * ray_bp_resident_blocks(variant, a.half_streams),
-                                (w.n_rays + kRayWarps - 1) / kRayWarps);
+  constexpr int kRaysPerBlock = kRayWarps * kRaysPerWarp;
+  int64_t b = std::min<int64_t>((int64_t)num_sms * ray_bp_resident_blocks(variant, a.half_streams, quiet),
+                                (w.n_rays + kRaysPerBlock - 1) / kRaysPerBlock);
   const unsigned grid = (unsigned)std::max<int64_t>(b, 1);
-  switch (variant) {
-#define X(id, mb, pol, pf, sc)                                                                    \
-  case id:                                                                                        \
-    if (a.half_streams)                                                                           \
-      k_ray_bp<mb, pol, pf, (sc > 0), __half, __half><<<grid, kRayWarps * 32, 0, s>>>(            \
-          sc == 0 ? w.queue : w.region, w.n_rays, w.rstart, w.nreg, w.rper, w.lprefix, w.lbase,    \
-          w.nlv, w.lcounter, sc == 0 ? w.counter : w.rcounter, a.inc_pair, a.inc_len16, a.inc_mu,  \
-          a.pair_lnq16, a.inc_pl, sc == 0 ? w.queue_ids : w.region_ids, qp, fix_reset);            \
-    else                                                                                          \
-      k_ray_bp<mb, pol, pf, (sc > 0), float, float><<<grid, kRayWarps * 32, 0, s>>>(              \
-          sc == 0 ? w.queue : w.region, w.n_rays, w.rstart, w.nreg, w.rper, w.lprefix, w.lbase,    \
-          w.nlv, w.lcounter, sc == 0 ? w.counter : w.rcounter, a.inc_pair, a.inc_len, a.inc_mu,    \
-          a.pair_lnq, a.inc_pl, sc == 0 ? w.queue_ids : w.region_ids, qp, fix_reset);              \
-    break;
-    MRF_RAY_VARIANTS(X)
-#undef X
-  }
+  const bool reg = kRayRegions[variant];
+  const RayMeta* queue = reg ? w.region : w.queue;
+  uint32_t* counter = reg ? w.rcounter : w.counter;
+  const uint32_t* ids = reg ? w.region_ids : w.queue_ids;
+  if (a.half_streams)
+    kRay16[variant][quiet]<<<grid, kRayWarps * 32, 0, s>>>(
+        queue, w.n_rays, w.rstart, w.nreg, w.rper, w.lprefix, w.lbase, w.nlv, w.lcounter, counter, a.inc_pair,
+        a.inc_len16, a.inc_mu, a.pair_lnq16, a.inc_pl, ids, qp, fix_reset);
+  else
+    kRay32[variant][quiet]<<<grid, kRayWarps * 32, 0, s>>>(
+        queue, w.n_rays, w.rstart, w.nreg, w.rper, w.lprefix, w.lbase, w.nlv, w.lcounter, counter, a.inc_pair,
+        a.inc_len, a.inc_mu, a.pair_lnq, a.inc_pl, ids, qp, fix_reset);
   return cudaGetLastError();
 }
 
@@ -1264,28 +1172,27 @@ cudaError_t launch_ray_queue(const RayMeta* meta, const uint32_t* order, uint32_
 
 cudaError_t launch_loud_prefix(const RayMeta* meta, uint32_t r_first, uint32_t n, const uint32_t* inc_pair,
                                const float* inc_len, uint32_t pair_base, uint32_t n_loud, uint32_t* loff,
-                               uint32_t* lpid, float* llen, uint16_t* lpos, bool emit, cudaStream_t s) {
+                               uint2* loud, QuietRay* ray, bool emit, cudaStream_t s) {
   if (!n) return cudaSuccess;
   const unsigned g = blocks((uint64_t)n * 32, 256);
   if (emit)
-    k_loud_prefix<true><<<g, 256, 0, s>>>(meta, r_first, n, inc_pair, inc_len, pair_base, n_loud, loff, lpid,
-                                          llen, lpos);
+    k_loud_prefix<true><<<g, 256, 0, s>>>(meta, r_first, n, inc_pair, inc_len, pair_base, n_loud, loff, loud, ray);
   else
-    k_loud_prefix<false><<<g, 256, 0, s>>>(meta, r_first, n, inc_pair, inc_len, pair_base, n_loud, loff,
-                                           lpid, llen, lpos);
+    k_loud_prefix<false><<<g, 256, 0, s>>>(meta, r_first, n, inc_pair, inc_len, pair_base, n_loud, loff, loud,
+                                           ray);
   return cudaGetLastError();
 }
 
 cudaError_t launch_quiet_prefix(const BpArrays& a, uint32_t r_first, uint32_t n, uint32_t pair_base,
-                                uint32_t n_loud, float2* q, cudaStream_t s) {
+                                uint32_t n_loud, QuietRay* ray, cudaStream_t s) {
   if (!n) return cudaSuccess;
   const unsigned g = blocks((uint64_t)n * 32, 256);
   if (a.half_streams)
     k_quiet_prefix<__half><<<g, 256, 0, s>>>(a.meta, r_first, n, a.inc_pair, a.inc_len, a.pair_lnq16, pair_base,
-                                             n_loud, q);
+                                             n_loud, ray);
   else
     k_quiet_prefix<float><<<g, 256, 0, s>>>(a.meta, r_first, n, a.inc_pair, a.inc_len, a.pair_lnq, pair_base,
-                                            n_loud, q);
+                                            n_loud, ray);
   return cudaGetLastError();
 }
 

@@ -184,8 +184,14 @@ struct mrf_map {
   int64_t nb_grid = 0, n_bricks = 0;
   std::vector<int> h_coord;
   int version = 0, built_version = -1;
-  int ray_variant = 4;  // ray-kernel variant (mrf_autotune / mrf_set_ray_variant); 4: SM regions,
-                        // pair-id prefetch, the fastest on the bench workloads
+  // ray-kernel variant: the caller's (mrf_autotune / mrf_set_ray_variant) once
+  // chosen, else 4 (SM regions, pair-id prefetch), and 1 (longest first) for a
+  // launch over several views: its V x R regions are served one after the
+  // other and end unevenly (Jacobi iteration of 32 views at 2 cm: 1.43 ms
+  // with 1, 1.84 with 4; Gauss-Seidel, 8 x 640x480 at 1 cm: 2.15 and 2.07)
+  int ray_variant = 4;
+  bool ray_variant_chosen = false;
+  int variant_for(bool all_views) const { return ray_variant_chosen || !all_views ? ray_variant : 1; }
   uint32_t nreg = 1;    // SM regions per view of the region queues
   // what the last build left: views with lists, per-pixel entries, the ends
   // of the region blocks, the queues and the tiles, the bricks it saw
@@ -212,8 +218,7 @@ struct mrf_map {
   // arenas
   DBuf meta, inc_pair, inc_len, inc_mu, inc_pl, pair_vox, pair_m, pair_cum, pair_stat, pair_ndyn, pair_hit,
       pair_q, pair_dm, pair_seg, dperm, s_q0, s_q1, s_q2, s_q3, s_bf, s_loud, s_pv, s_sg, dpair, dseg, drun, carry, ray_order, ray_queue, region_q, rstart, rcounters, counters,
-      tile_first, lbase, lsingle, lprefix, queue_ids, region_ids, loud_off, loud_pid, loud_len, loud_pos,
-      quiet_q;
+      tile_first, lbase, lsingle, lprefix, queue_ids, region_ids, loud_off, loud, quiet_ray;
   uint32_t jac_tile_base = 0;
   int64_t n_inc = 0, n_pairs = 0, n_dperm = 0, n_dpairs = 0;
   // voxels with a pair past the length gate (their beliefs follow L)
@@ -270,11 +275,8 @@ struct mrf_map {
     a.belief = d_belief.as<float>();
     a.half_streams = precision == MRF_PRECISION_HALF_STREAMS ? 1 : 0;
     a.pair_variant = pair_variant;
-    a.quiet_q = quiet_q.as<float2>();
-    a.loud_off = loud_off.as<uint32_t>();
-    a.loud_pid = loud_pid.as<uint32_t>();
-    a.loud_len = loud_len.as<float>();
-    a.loud_pos = loud_pos.as<uint16_t>();
+    a.quiet_ray = quiet_ray.as<QuietRay>();
+    a.loud = loud.as<uint2>();
     a.inc_len16 = inc_len16.as<__half>();
     a.pair_lnq16 = pair_q16.as<__half>();
     return a;
@@ -882,7 +884,7 @@ void count_loud_lists(mrf_map* m) {
     if (v.retired || v.n_inc == 0) continue;
     CK(launch_loud_prefix(meta, (uint32_t)v.pix_base, (uint32_t)view_pixels(v), m->inc_pair.as<uint32_t>(),
                           m->inc_len.as<float>(), v.pair_base, v.n_loud, m->loud_off.as<uint32_t>(), nullptr,
-                          nullptr, nullptr, false, m->stream));
+                          nullptr, false, m->stream));
   }
   m->s_offs.reserve((size_t)(npix + 1) * 4, false, m->stream);
   const size_t t = scan_temp_bytes((uint32_t)(npix + 1));
@@ -898,16 +900,13 @@ void emit_loud_lists(mrf_map* m) {
   const int64_t npix = m->npix_total;
   const uint32_t total = (uint32_t)m->n_loud_prefix;
   const RayMeta* meta = m->meta.as<RayMeta>();
-  m->quiet_q.reserve((size_t)std::max<int64_t>(npix, 1) * 8, false, m->stream);
-  m->loud_pid.reserve((size_t)std::max<uint32_t>(total, 1) * 4, false, m->stream);
-  m->loud_len.reserve((size_t)std::max<uint32_t>(total, 1) * 4, false, m->stream);
-  m->loud_pos.reserve((size_t)std::max<uint32_t>(total, 1) * 2, false, m->stream);
+  m->quiet_ray.reserve((size_t)std::max<int64_t>(npix, 1) * sizeof(QuietRay), false, m->stream);
+  m->loud.reserve((size_t)std::max<uint32_t>(total, 1) * 8, false, m->stream);
   for (const View& v : m->views) {
     if (v.retired || v.n_inc == 0) continue;
     CK(launch_loud_prefix(meta, (uint32_t)v.pix_base, (uint32_t)view_pixels(v), m->inc_pair.as<uint32_t>(),
                           m->inc_len.as<float>(), v.pair_base, v.n_loud, m->loud_off.as<uint32_t>(),
-                          m->loud_pid.as<uint32_t>(), m->loud_len.as<float>(), m->loud_pos.as<uint16_t>(), true,
-                          m->stream));
+                          m->loud.as<uint2>(), m->quiet_ray.as<QuietRay>(), true, m->stream));
   }
 }
 
@@ -946,7 +945,7 @@ void quiet_prefix_all(mrf_map* m, const BpArrays& a) {
   for (const View& v : m->views) {
     if (v.retired || v.n_inc == 0) continue;
     CK(launch_quiet_prefix(a, (uint32_t)v.pix_base, (uint32_t)view_pixels(v), v.pair_base, v.n_loud,
-                           m->quiet_q.as<float2>(), m->stream));
+                           m->quiet_ray.as<QuietRay>(), m->stream));
   }
 }
 
@@ -1592,7 +1591,7 @@ void enqueue_iteration(mrf_map* m, const BpArrays& a, bool jacobi, int fix, int 
                              m->stream));
       prof.end();
       prof.begin(1);
-      CK(launch_ray_bp(a, ray_work(m, c), fix, m->num_sms, m->ray_variant, quiet && phase >= 2, m->stream));
+      CK(launch_ray_bp(a, ray_work(m, c), fix, m->num_sms, m->variant_for(false), quiet && phase >= 2, m->stream));
       prof.end();
       prof.begin(2);
       if (v.n_dperm) {
@@ -1615,7 +1614,7 @@ void enqueue_iteration(mrf_map* m, const BpArrays& a, bool jacobi, int fix, int 
     prof.end();
     prof.begin(1);
     // the queues of all views are contiguous: one launch over all rays
-    CK(launch_ray_bp(a, ray_work(m, -1), fix, m->num_sms, m->ray_variant, quiet && phase >= 2, m->stream));
+    CK(launch_ray_bp(a, ray_work(m, -1), fix, m->num_sms, m->variant_for(V > 1), quiet && phase >= 2, m->stream));
     prof.end();
     prof.begin(2);
     CK(launch_pair_update(a, 0, (uint32_t)m->n_dperm, 0, (uint32_t)m->n_dpairs,
@@ -1841,7 +1840,7 @@ void destroy_bufs(mrf_map* m) {
                  &m->pair_seg, &m->dperm, &m->dpair, &m->dseg, &m->drun,
                  &m->carry, &m->ray_order, &m->ray_queue, &m->region_q, &m->rstart, &m->rcounters, &m->counters, &m->tile_first,
                  &m->lbase, &m->lsingle, &m->lprefix, &m->queue_ids, &m->region_ids, &m->loud_off,
-                 &m->loud_pid, &m->loud_len, &m->loud_pos, &m->quiet_q,
+                 &m->loud, &m->quiet_ray,
                  &m->vseg, &m->vpairs, &m->vvox, &m->vox_active, &m->d_Lbase, &m->inc_len16, &m->pair_q16,
                  &m->s_rec, &m->s_recs, &m->s_pf, &m->s_ps,
                  &m->s_flags, &m->s_ind, &m->s_scan,
@@ -1934,8 +1933,8 @@ mrf_status mrf_create(const mrf_params* params, mrf_map** out) {
     CK(cudaGetDevice(&m->device));
     CK(cudaDeviceGetAttribute(&m->num_sms, cudaDevAttrMultiProcessorCount, m->device));
     for (int k = 0; k < ray_bp_variants(); ++k) {
-      ray_bp_resident_blocks(k, 0);
-      ray_bp_resident_blocks(k, 1);
+      for (int h = 0; h < 2; ++h)
+        for (int q = 0; q < 2; ++q) ray_bp_resident_blocks(k, h, q);
     }
     CK(cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking));
     CK(cudaEventCreate(&m->ev0));
@@ -2319,7 +2318,7 @@ static void warm_start_impl(mrf_map* m, const float* L_pred, bool device_ptr, in
   for (int k = 0; k < sweeps; ++k) {
     zero_counters(m);
     CK(launch_pair_prepare(a, 0, P, 1, m->stream));
-    CK(launch_ray_bp(a, ray_work(m, -1), 0, m->num_sms, m->ray_variant, false, m->stream));
+    CK(launch_ray_bp(a, ray_work(m, -1), 0, m->num_sms, m->variant_for(V > 1), false, m->stream));
     CK(launch_pair_update(a, 0, (uint32_t)m->n_dperm, 0, (uint32_t)m->n_dpairs,
                           m->tile_first.as<uint32_t>() + m->jac_tile_base, m->carry.as<TileCarry>(),
                           1, m->stream));
@@ -2462,6 +2461,7 @@ mrf_status mrf_set_ray_variant(mrf_map* m, int variant) {
     return MRF_ERR_INVALID;
   }
   m->ray_variant = variant;
+  m->ray_variant_chosen = true;
   drop_graphs(m);
   return MRF_OK;
 }
@@ -2601,6 +2601,8 @@ mrf_status mrf_autotune_flags(mrf_map* m, int reps, int flags, double* ms_out, i
       CK(cudaMemcpyAsync(snap + nv, m->d_belief.p, nv, cudaMemcpyDeviceToDevice, m->stream));
       CK(cudaMemcpyAsync(snap + 2 * nv, m->pair_m.p, npb, cudaMemcpyDeviceToDevice, m->stream));
       const int keep = m->ray_variant;
+      const bool keep_chosen = m->ray_variant_chosen;
+      m->ray_variant_chosen = true;
       Profiler off{m, false};
       int64_t launches = 0;
       if (quiet) quiet_prefix_all(m, a);
@@ -2620,6 +2622,7 @@ mrf_status mrf_autotune_flags(mrf_map* m, int reps, int flags, double* ms_out, i
         CK(cudaMemcpyAsync(m->pair_m.p, snap + 2 * nv, npb, cudaMemcpyDeviceToDevice, m->stream));
       }
       m->ray_variant = keep;
+      m->ray_variant_chosen = keep_chosen;
       sync(m);
     }
     int best = 0;
@@ -2627,6 +2630,7 @@ mrf_status mrf_autotune_flags(mrf_map* m, int reps, int flags, double* ms_out, i
       if (ms[k] < ms[best]) best = k;
     for (int k = 0; k < NV && k < cap; ++k) ms_out[k] = ms[k];
     m->ray_variant = best;
+    m->ray_variant_chosen = true;
     drop_graphs(m);
     // then the pair reduction's variant with that ray kernel
     if (m->n_inc > 0) {

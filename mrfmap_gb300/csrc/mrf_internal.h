@@ -182,6 +182,16 @@ cudaError_t sort_pairs_u32(void* tmp, size_t tmp_bytes, const uint32_t* kin, uin
                            const uint32_t* vin, uint32_t* vout, uint32_t n, int bits, cudaStream_t s);
 
 // BP
+// the static-prefix data of the ray kernel's fast path (iterations from the
+// third of a call on), per ray (pixel index): the quiet sums before and from
+// r0 on (up to k4), and the list of the prefix's loud incidences (na before
+// r0, then nb from r0 on)
+struct QuietRay {
+  float qa, qb;
+  uint32_t first;
+  uint16_t na, nb;
+};
+static_assert(sizeof(QuietRay) == 16, "QuietRay layout");
 struct BpArrays {
   const RayMeta* meta;
   const uint32_t* inc_pair;
@@ -206,11 +216,8 @@ struct BpArrays {
   // fp16 then
   int half_streams;
   int pair_variant;  // pair reduction: 0 one prefetched pair per thread, 1 two
-  const float2* quiet_q;     // per ray: quiet sums of the static prefix
-  const uint32_t* loud_off;  // per ray: first entry of its loud list (and the next ray's)
-  const uint32_t* loud_pid;
-  const float* loud_len;
-  const uint16_t* loud_pos;
+  const QuietRay* quiet_ray;  // per ray: the static prefix's quiet sums and loud list
+  const uint2* loud;          // the loud lists' entries: pair id, length
   const __half* inc_len16;
   __half* pair_lnq16;
 };
@@ -226,7 +233,7 @@ cudaError_t launch_pair_prepare(const BpArrays& a, uint32_t p0, uint32_t p1, int
 // ray-kernel variants (register budget x load policy; identical arithmetic)
 int ray_bp_variants();
 // resident blocks per SM of a variant of the persistent ray kernel (queried once)
-int ray_bp_resident_blocks(int variant, int half_streams);
+int ray_bp_resident_blocks(int variant, int half_streams, int quiet);
 // fp32 -> fp16, round to nearest
 cudaError_t launch_to_half(const float* in, int64_t n, __half* out, cudaStream_t s);
 // the rays of one ray-kernel launch in its schedules: queue[0..n_rays)
@@ -237,15 +244,9 @@ cudaError_t launch_to_half(const float* in, int64_t n, __half* out, cudaStream_t
 // zeroed counters), and the views' remaining short rays (longest first):
 // view q's lprefix[q + 1] - lprefix[q] leftovers from region[lbase[q]] on,
 // nlv views, one zeroed counter
-// the static-prefix data of the ray kernel's fast path (iterations from the
-// third of a call on): per ray (pixel index) the quiet sums up to r0 and up
-// to k4, and the list of the prefix's loud incidences at loff[r]..loff[r+1]
 struct QuietPrefix {
-  const float2* q;
-  const uint32_t* loff;
-  const uint32_t* lpid;
-  const float* llen;
-  const uint16_t* lpos;
+  const QuietRay* ray;
+  const uint2* loud;
 };
 
 struct RayWork {
@@ -263,7 +264,7 @@ struct RayWork {
   uint32_t nlv;
   uint32_t* lcounter;
 };
-// quiet: the static prefix from the quiet sums (a.quiet_q and the loud
+// quiet: the static prefix from the quiet sums (a.quiet_ray and the loud
 // lists must be current)
 cudaError_t launch_ray_bp(const BpArrays& a, const RayWork& w, int fix_reset, int num_sms, int variant,
                           bool quiet, cudaStream_t s);
@@ -271,10 +272,10 @@ cudaError_t launch_ray_bp(const BpArrays& a, const RayWork& w, int fix_reset, in
 // view: counts to loff[r] (emit false), or the lists at loff[r] (emit true)
 cudaError_t launch_loud_prefix(const RayMeta* meta, uint32_t r_first, uint32_t n, const uint32_t* inc_pair,
                                const float* inc_len, uint32_t pair_base, uint32_t n_loud, uint32_t* loff,
-                               uint32_t* lpid, float* llen, uint16_t* lpos, bool emit, cudaStream_t s);
+                               uint2* loud, QuietRay* ray, bool emit, cudaStream_t s);
 // quiet sums of the static prefixes of rays r_first..r_first+n of one view
 cudaError_t launch_quiet_prefix(const BpArrays& a, uint32_t r_first, uint32_t n, uint32_t pair_base,
-                                uint32_t n_loud, float2* q, cudaStream_t s);
+                                uint32_t n_loud, QuietRay* ray, cudaStream_t s);
 cudaError_t launch_ray_keys(const RayMeta* meta, uint32_t n, uint32_t* keys, uint32_t* vals,
                             cudaStream_t s);
 // queue[i] = meta[order[i]], ids[i] = id_base + order[i], i < n
