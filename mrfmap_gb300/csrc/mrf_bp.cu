@@ -1093,8 +1093,8 @@ constexpr int kRayVariants = 8;
 int ray_bp_variants() { return kRayVariants; }
 
 namespace {
-using RayKernel32 = decltype(&k_ray_bp<0, 0, 0, false, false, float, float>);
-using RayKernel16 = decltype(&k_ray_bp<0, 0, 0, false, false, __half, __half>);
+using RayKernel32 = decltype(&k_ray_bp<8, 0, 0, false, false, float, float>);
+using RayKernel16 = decltype(&k_ray_bp<8, 0, 0, false, false, __half, __half>);
 
 #define X(id, mb, pol, pf, sc) \
   {k_ray_bp<mb, pol, pf, (sc > 0), false, float, float>, k_ray_bp<mb, pol, pf, (sc > 0), true, float, float>},

@@ -148,8 +148,7 @@ struct View {
   DBuf depth;
   uint32_t inc_base = 0, n_inc = 0;
   uint32_t pair_base = 0, n_pairs = 0;
-  uint32_t perm_base = 0, n_perm = 0;     // pair-grouped positions of all incidences
-  uint32_t dperm_base = 0, n_dperm = 0;   // ... of the dynamic ones
+  uint32_t dperm_base = 0, n_dperm = 0;   // pair-grouped positions of the dynamic incidences
   uint32_t dpair_base = 0, n_dpairs = 0;  // runs of dynamic incidences (one per pair)
   uint32_t order_base = 0, n_active = 0;  // ray queue (longest first)
   uint32_t left_base = 0, n_left = 0;     // leftover queue of the SM-affine schedule
@@ -196,7 +195,7 @@ struct mrf_map {
   // what the last build left: views with lists, per-pixel entries, the ends
   // of the region blocks, the queues and the tiles, the bricks it saw
   int built_views = 0;
-  int64_t npix_total = 0, queue_end = 0, tile_end = 0, carry_tiles = 0, vox_active_n = 0, n_perm_total = 0;
+  int64_t npix_total = 0, queue_end = 0, tile_end = 0, carry_tiles = 0, vox_active_n = 0;
   int64_t n_loud_prefix = 0;  // entries of the static prefixes' loud lists
   int64_t loud_count_version = -1, loud_list_version = -1;  // builds the loud lists were counted / made for
   uint32_t region_end = 0;
@@ -208,7 +207,7 @@ struct mrf_map {
   // test hook: the next append fails with this status once its pairs are
   // built (0: none)
   int test_append_fail = 0;
-  // the build scratch s_vox / s_rec holds the incidences from this index on
+  // the build scratch s_vox holds the incidences from this index on
   // (0 in a full build; an appended build's first new incidence, so the
   // scratch holds the new views only, not the arenas' retired lists)
   uint32_t scratch_base = 0;
@@ -217,7 +216,7 @@ struct mrf_map {
   std::vector<View> views;
   // arenas
   DBuf meta, inc_pair, inc_len, inc_mu, inc_pl, pair_vox, pair_m, pair_cum, pair_stat, pair_ndyn, pair_hit,
-      pair_q, pair_dm, pair_seg, dperm, s_q0, s_q1, s_q2, s_q3, s_bf, s_loud, s_pv, s_sg, dpair, dseg, drun, carry, ray_order, ray_queue, region_q, rstart, rcounters, counters,
+      pair_q, pair_dm, dperm, s_q0, s_q1, s_q2, s_q3, s_q4, s_bf, s_first, s_len, s_loud, dpair, dseg, drun, carry, ray_order, ray_queue, region_q, rstart, rcounters, counters,
       tile_first, lbase, lsingle, lprefix, queue_ids, region_ids, loud_off, loud, quiet_ray;
   uint32_t jac_tile_base = 0;
   int64_t n_inc = 0, n_pairs = 0, n_dperm = 0, n_dpairs = 0;
@@ -239,8 +238,8 @@ struct mrf_map {
   uint32_t n_vvox = 0;
   int jacobi_version = -1;
   // scratch
-  DBuf s_rec, s_recs, s_pf, s_ps, s_flags, s_ind, s_scan, s_tmp, s_counts, s_offs, s_vox, s_k0, s_k1, s_v0, s_v1,
-      s_seg, s_dense, s_err, s_depth_in, s_depth, s_img, s_part, s_sum, s_prev, s_delta, s_snap, s_vcnt;
+  DBuf s_pf, s_ps, s_flags, s_ind, s_scan, s_tmp, s_counts, s_offs, s_vox, s_k0, s_k1, s_v0, s_v1,
+      s_dense, s_err, s_depth_in, s_depth, s_img, s_part, s_sum, s_prev, s_delta, s_snap, s_vcnt;
   mrf_stats stats{};
   // MRF_PROFILE event pool
   std::vector<cudaEvent_t> prof_ev;
@@ -435,150 +434,115 @@ void ray_records_and_counters(mrf_map* m, const std::vector<int>& views, int64_t
   }
 }
 
-// The pairs of view c: its incidences (at v.inc_base; voxel ids in s_vox and
-// build records in s_rec at the same positions) sorted by voxel (stable),
-// one pair per run, the pairs renumbered brick-major by first visit
-// (mrf_build.cu, k_pair_first; pairs on voxels flagged in s_loud first) and
-// the incidences regrouped in the new pair order; then the pair statistics
-// and the dynamic runs.  Numbered from the totals' current ends, which
-// advance.
-void view_pairs(mrf_map* m, int c, int bits, int64_t& pair_total, int64_t& perm_total, int64_t& dperm_total,
-                int64_t& dpair_total) {
+// The pairs of view c from its incidences (at v.inc_base; voxel ids in s_vox):
+// numbered brick-major by first visit (mrf_build.cu), pairs on voxels flagged
+// in s_loud first; then the dynamic incidences grouped by pair and the pair
+// statistics.  Numbered from the totals' current ends, which advance.
+void view_pairs(mrf_map* m, int c, int64_t& pair_total, int64_t& dperm_total, int64_t& dpair_total) {
   View& v = m->views[c];
-  uint32_t n = v.n_inc;
-  uint32_t nr = (uint32_t)v.c_npre;
+  const uint32_t n = v.n_inc;
+  const uint32_t nd = (uint32_t)v.c_ndyn;
+  const cudaStream_t st = m->stream;
   v.pair_base = (uint32_t)pair_total;
-  v.perm_base = (uint32_t)perm_total;
   v.dperm_base = (uint32_t)dperm_total;
   v.dpair_base = (uint32_t)dpair_total;
   v.n_pairs = 0;
-  v.n_perm = 0;
   v.n_dperm = 0;
   v.n_dpairs = 0;
   v.n_loud = 0;
-  if (nr == 0) return;
-    m->s_k0.reserve((size_t)n * 4 + 4, false, m->stream);
-    m->s_k1.reserve((size_t)n * 4 + 4, false, m->stream);
-    m->s_v0.reserve((size_t)n * 4 + 4, false, m->stream);
-    m->s_v1.reserve((size_t)n * 4 + 4, false, m->stream);
-    CK(launch_iota(m->s_v0.as<uint32_t>(), n, m->stream));
-    size_t t2 = sort_temp_bytes(n, bits);
-    m->s_tmp.reserve(t2, false, m->stream);
-    // padding incidences carry kNoVoxel, whose low bits exceed every voxel id
-    CK(sort_pairs_u32(m->s_tmp.p, t2, m->s_vox.as<uint32_t>() + (v.inc_base - m->scratch_base), m->s_k1.as<uint32_t>(),
-                      m->s_v0.as<uint32_t>(), m->s_v1.as<uint32_t>(), n, bits, m->stream));
-    size_t t1 = scan_temp_bytes(nr + 1);
-    m->s_tmp.reserve(t1, false, m->stream);
-    // voxel-order pairs: runs of the sorted voxel keys
-    CK(launch_vox_heads(m->s_k1.as<uint32_t>(), nr, m->s_k0.as<uint32_t>(), m->stream));
-    CK(cudaMemsetAsync(m->s_k0.as<uint32_t>() + nr, 0, 4, m->stream));
-    CK(exclusive_scan_u32(m->s_tmp.p, t1, m->s_k0.as<uint32_t>(), m->s_v0.as<uint32_t>(), nr + 1,
-                          m->stream));
-    const uint32_t np = read1(m, m->s_v0.as<uint32_t>() + nr);
-    u32_checked(pair_total + np + 1, "pair count");
-    size_t pb = (size_t)(pair_total + np + 1);
-    m->pair_vox.reserve(pb * 4, true, m->stream);
-    m->pair_m.reserve(pb * 4, true, m->stream);
-    m->pair_cum.reserve(pb * 4, true, m->stream);
-    m->pair_stat.reserve(pb * 4, true, m->stream);
-    m->pair_ndyn.reserve(pb * 4, true, m->stream);
-    m->pair_hit.reserve(pb * 4, true, m->stream);
-    m->pair_seg.reserve(pb * 4, true, m->stream);
-    {
-      const uint32_t np0 = np;
-      const size_t q4 = (size_t)np0 * 4 + 4;
-      m->s_pv.reserve(q4, false, m->stream);
-      m->s_sg.reserve(q4, false, m->stream);
-      uint32_t* pv = m->s_pv.as<uint32_t>();
-      uint32_t* sg = m->s_sg.as<uint32_t>();
-      CK(launch_pairs_from_sorted(m->s_k1.as<uint32_t>(), m->s_v1.as<uint32_t>(), m->s_k0.as<uint32_t>(),
-                                  m->s_v0.as<uint32_t>(), nr, 0, 0, v.inc_base, pv, sg, nullptr, m->stream));
-      CK(launch_fill_u32(sg + np0, 1, nr, m->stream));
-      // first visits: of each pair, and of each brick (min over its pairs)
-      m->s_q0.reserve(q4, false, m->stream);
-      m->s_q1.reserve(q4, false, m->stream);
-      m->s_q2.reserve(q4, false, m->stream);
-      m->s_q3.reserve(q4, false, m->stream);
-      m->s_bf.reserve((size_t)m->n_bricks * 4 + 4, false, m->stream);
-      uint32_t* q0 = m->s_q0.as<uint32_t>();
-      uint32_t* q1 = m->s_q1.as<uint32_t>();
-      uint32_t* q2 = m->s_q2.as<uint32_t>();
-      uint32_t* q3 = m->s_q3.as<uint32_t>();
-      CK(launch_pair_first(sg, np0, 0, m->s_v1.as<uint32_t>(), q0, m->stream));
-      CK(launch_fill_u32(m->s_bf.as<uint32_t>(), m->n_bricks, 0xFFFFFFFFu, m->stream));
-      CK(launch_brick_first(pv, q0, np0, m->s_bf.as<uint32_t>(), m->stream));
-      // order: by own first visit, then (stable) by (quiet voxel, the
-      // brick's first visit)
-      int ibits = 1;
-      while (ibits < 31 && ((uint64_t)1 << ibits) < (uint64_t)n) ++ibits;
-      size_t t4 = std::max(sort_temp_bytes(np0, ibits), sort_temp_bytes(np0, ibits + 1));
-      m->s_tmp.reserve(std::max(t4, t1), false, m->stream);
-      CK(launch_iota(q2, np0, m->stream));
-      CK(sort_pairs_u32(m->s_tmp.p, t4, q0, q1, q2, q3, np0, ibits, m->stream));  // q3: by own visit
-      CK(launch_brick_keys(q3, np0, pv, m->s_bf.as<uint32_t>(), m->s_loud.as<uint8_t>(), ibits, q0,
-                           m->stream));
-      CK(sort_pairs_u32(m->s_tmp.p, t4, q0, q1, q3, q2, np0, ibits + 1, m->stream));  // q2: new order
-      // new runs: lengths in the new order, their starts, the old -> new map
-      CK(launch_new_lengths(q2, np0, sg, q0, q3, m->stream));
-      CK(cudaMemsetAsync(q0 + np0, 0, 4, m->stream));
-      size_t t5 = scan_temp_bytes(np0 + 1);
-      m->s_tmp.reserve(t5, false, m->stream);
-      CK(exclusive_scan_u32(m->s_tmp.p, t5, q0, q1, np0 + 1, m->stream));
-      // the sorted positions in the new pair order (and each incidence's
-      // new pair id), the renumbered pairs' voxels and runs
-      m->s_recs.reserve((size_t)nr * 8, false, m->stream);
-      uint32_t* nidx = m->s_recs.as<uint32_t>();
-      CK(launch_move_positions(m->s_v1.as<uint32_t>(), m->s_k0.as<uint32_t>(), m->s_v0.as<uint32_t>(), sg, q3,
-                               q1, nr, v.inc_base, v.pair_base, nidx, m->inc_pair.as<uint32_t>(), m->stream));
-      CK(launch_pairs_renumbered(q2, np0, pv, q1, v.pair_base, v.perm_base, m->pair_vox.as<uint32_t>(),
-                                 m->pair_seg.as<uint32_t>(), m->stream));
-      std::swap(m->s_v1, m->s_recs);  // the moved positions become the sorted order
-      m->s_v1.reserve((size_t)n * 4 + 4, true, m->stream);
-    }
-    CK(cudaMemsetAsync(m->s_k1.p, 0, 4, m->stream));
-    CK(launch_count_loud(m->pair_vox.as<uint32_t>() + v.pair_base, np, m->s_loud.as<uint8_t>(),
-                         m->s_k1.as<uint32_t>(), m->stream));
-    v.n_loud = read1(m, m->s_k1.as<uint32_t>());
-    m->s_recs.reserve((size_t)nr * 8, false, m->stream);
-    CK(launch_gather_rec(m->s_v1.as<uint32_t>(), nr, v.inc_base - m->scratch_base, m->s_rec.as<float2>(),
-                         m->s_recs.as<float2>(), m->s_k0.as<uint32_t>(), m->stream));
-    m->s_pf.reserve((size_t)np * 4 + 4, false, m->stream);
-    CK(launch_pair_stats(m->pair_seg.as<uint32_t>(), v.pair_base, np, v.perm_base, m->s_recs.as<float2>(),
-                         m->pair_cum.as<float>(), m->pair_stat.as<float>(), m->pair_ndyn.as<uint32_t>(),
-                         m->pair_hit.as<float>(), m->s_pf.as<uint32_t>(), m->stream));
-    // dynamic incidences in pair-grouped order (a stable compaction of the
-    // sorted positions) and the run of each pair that has any
-    CK(cudaMemsetAsync(m->s_k0.as<uint32_t>() + nr, 0, 4, m->stream));
-    CK(exclusive_scan_u32(m->s_tmp.p, t1, m->s_k0.as<uint32_t>(), m->s_v0.as<uint32_t>(), nr + 1,
-                          m->stream));
-    uint32_t nd = read1(m, m->s_v0.as<uint32_t>() + nr);
-    CK(launch_dyn_scatter(m->s_v1.as<uint32_t>(), m->s_k0.as<uint32_t>(), m->s_v0.as<uint32_t>(), nr,
-                          v.inc_base, v.dperm_base, m->dperm.as<uint32_t>(), m->stream));
-    m->s_pf.reserve((size_t)np * 4 + 4, false, m->stream);
-    m->s_ps.reserve((size_t)np * 4 + 4, false, m->stream);
-    CK(launch_dpair_flags(m->pair_ndyn.as<uint32_t>(), v.pair_base, np, m->s_pf.as<uint32_t>(),
-                          m->stream));
-    CK(cudaMemsetAsync(m->s_pf.as<uint32_t>() + np, 0, 4, m->stream));
-    size_t t3 = scan_temp_bytes(np + 1);
-    m->s_tmp.reserve(t3, false, m->stream);
-    CK(exclusive_scan_u32(m->s_tmp.p, t3, m->s_pf.as<uint32_t>(), m->s_ps.as<uint32_t>(), np + 1,
-                          m->stream));
-    uint32_t ndp = read1(m, m->s_ps.as<uint32_t>() + np);
-    size_t db = (size_t)(dpair_total + ndp + 1);
-    m->dpair.reserve(db * 4, true, m->stream);
-    m->dseg.reserve(db * 4, true, m->stream);
-    CK(launch_dpairs(m->s_pf.as<uint32_t>(), m->s_ps.as<uint32_t>(), v.pair_base, np,
-                     m->pair_seg.as<uint32_t>(), v.perm_base, m->s_v0.as<uint32_t>(), v.dperm_base,
-                     v.dpair_base, m->dpair.as<uint32_t>(), m->dseg.as<uint32_t>(), m->stream));
-    CK(launch_fill_u32(m->dseg.as<uint32_t>() + v.dpair_base + ndp, 1, v.dperm_base + nd, m->stream));
-    v.n_pairs = np;
-    v.n_perm = nr;
-    v.n_dperm = nd;
-    v.n_dpairs = ndp;
-    pair_total += np;
-    perm_total += nr;
-    dperm_total += nd;
-    dpair_total += ndp;
+  if (v.c_npre == 0) return;
+  const uint32_t nb = (uint32_t)m->n_bricks;
+  const uint32_t npix = (uint32_t)view_pixels(v);
+  const uint32_t* vox = m->s_vox.as<uint32_t>() + (v.inc_base - m->scratch_base);
+  // first visits, the bricks in their order, the pairs' places
+  m->s_first.reserve((size_t)nb * kBrickVox * 4, false, st);
+  m->s_bf.reserve((size_t)nb * 4, false, st);
+  CK(cudaMemsetAsync(m->s_first.p, 0xFF, (size_t)nb * kBrickVox * 4, st));
+  CK(cudaMemsetAsync(m->s_bf.p, 0xFF, (size_t)nb * 4, st));
+  uint32_t* table = m->s_first.as<uint32_t>();
+  CK(launch_first_visit(vox, n, table, m->s_bf.as<uint32_t>(), st));
+  m->s_q0.reserve((size_t)nb * 4, false, st);
+  m->s_q1.reserve((size_t)nb * 4, false, st);
+  m->s_q2.reserve((size_t)nb * 4, false, st);
+  m->s_q3.reserve(((size_t)2 * nb + 1) * 4, false, st);
+  m->s_q4.reserve(((size_t)2 * nb + 1) * 4, false, st);
+  const size_t ts = std::max(sort_temp_bytes(nb, 32), scan_temp_bytes(2 * nb + 1));
+  m->s_tmp.reserve(ts, false, st);
+  const uint32_t* bkey = m->s_q0.as<uint32_t>();
+  const uint32_t* order = m->s_q2.as<uint32_t>();
+  uint32_t* cnt = m->s_q3.as<uint32_t>();
+  uint32_t* start = m->s_q4.as<uint32_t>();
+  CK(launch_iota(m->s_q1.as<uint32_t>(), nb, st));
+  CK(sort_pairs_u32(m->s_tmp.p, ts, m->s_bf.as<uint32_t>(), m->s_q0.as<uint32_t>(), m->s_q1.as<uint32_t>(),
+                    m->s_q2.as<uint32_t>(), nb, 32, st));
+  CK(launch_brick_count(bkey, order, nb, table, m->s_loud.as<uint8_t>(), cnt, st));
+  CK(cudaMemsetAsync(cnt + 2 * (size_t)nb, 0, 4, st));
+  CK(exclusive_scan_u32(m->s_tmp.p, ts, cnt, start, 2 * nb + 1, st));
+  uint32_t np = 0;
+  CK(cudaMemcpyAsync(&v.n_loud, start + nb, 4, cudaMemcpyDeviceToHost, st));
+  CK(cudaMemcpyAsync(&np, start + 2 * (size_t)nb, 4, cudaMemcpyDeviceToHost, st));
+  // the dynamic incidences' places, while the host waits
+  m->s_k0.reserve((size_t)std::max(nd, npix) * 4 + 4, false, st);
+  m->s_ps.reserve((size_t)npix * 4 + 4, false, st);
+  const size_t tp = scan_temp_bytes(npix);
+  m->s_pf.reserve(tp, false, st);
+  CK(launch_dyn_counts(m->meta.as<RayMeta>() + v.pix_base, npix, m->s_k0.as<uint32_t>(), st));
+  CK(exclusive_scan_u32(m->s_pf.p, tp, m->s_k0.as<uint32_t>(), m->s_ps.as<uint32_t>(), npix, st));
+  sync(m);
+  u32_checked(pair_total + np + 1, "pair count");
+  const size_t pb = (size_t)(pair_total + np + 1);
+  m->pair_vox.reserve(pb * 4, true, st);
+  m->pair_m.reserve(pb * 4, true, st);
+  m->pair_cum.reserve(pb * 4, true, st);
+  m->pair_stat.reserve(pb * 4, true, st);
+  m->pair_ndyn.reserve(pb * 4, true, st);
+  m->pair_hit.reserve(pb * 4, true, st);
+  CK(launch_brick_number(bkey, order, nb, table, m->s_loud.as<uint8_t>(), start, v.pair_base,
+                         m->pair_vox.as<uint32_t>(), st));
+  // the incidences' pairs; pair numbers and indices of the dynamic ones in
+  // s_k0, s_v0, sorted by pair (stable: increasing incidence within a pair)
+  m->s_len.reserve((size_t)np * 8, false, st);
+  m->s_v0.reserve((size_t)nd * 4 + 4, false, st);
+  m->s_k1.reserve((size_t)nd * 4 + 4, false, st);
+  CK(cudaMemsetAsync(m->s_len.p, 0, (size_t)np * 8, st));
+  unsigned long long* slen = m->s_len.as<unsigned long long>();
+  CK(launch_assign_pairs(m->meta.as<RayMeta>() + v.pix_base, npix, vox, m->inc_len.as<float>() + v.inc_base, table,
+                         v.inc_base, v.pair_base, m->s_ps.as<uint32_t>(), m->inc_pair.as<uint32_t>() + v.inc_base,
+                         slen, m->s_k0.as<uint32_t>(), m->s_v0.as<uint32_t>(), st));
+  CK(launch_static_stats(slen, np, m->pair_cum.as<float>() + v.pair_base, m->pair_stat.as<float>() + v.pair_base,
+                         m->pair_ndyn.as<uint32_t>() + v.pair_base, m->pair_hit.as<float>() + v.pair_base, st));
+  uint32_t ndp = 0;
+  if (nd) {
+    int bits = 1;
+    while (bits < 32 && ((uint64_t)1 << bits) < (uint64_t)v.n_loud) ++bits;  // dynamic pairs are loud
+    const size_t td = std::max(sort_temp_bytes(nd, bits), scan_temp_bytes(nd + 1));
+    m->s_tmp.reserve(td, false, st);
+    uint32_t* sk = m->s_k1.as<uint32_t>();
+    uint32_t* flag = m->s_k0.as<uint32_t>();
+    uint32_t* scan = m->s_v0.as<uint32_t>();
+    CK(sort_pairs_u32(m->s_tmp.p, td, m->s_k0.as<uint32_t>(), sk, m->s_v0.as<uint32_t>(),
+                      m->dperm.as<uint32_t>() + v.dperm_base, nd, bits, st));
+    CK(launch_run_heads(sk, nd, flag, st));
+    CK(cudaMemsetAsync(flag + nd, 0, 4, st));
+    CK(exclusive_scan_u32(m->s_tmp.p, td, flag, scan, nd + 1, st));
+    ndp = read1(m, scan + nd);
+    const size_t db = (size_t)(dpair_total + ndp + 1);
+    m->dpair.reserve(db * 4, true, st);
+    m->dseg.reserve(db * 4, true, st);
+    CK(launch_runs(sk, flag, scan, nd, v.pair_base, v.dperm_base, m->dpair.as<uint32_t>() + v.dpair_base,
+                   m->dseg.as<uint32_t>() + v.dpair_base, st));
+    CK(launch_fill_u32(m->dseg.as<uint32_t>() + v.dpair_base + ndp, 1, v.dperm_base + nd, st));
+    m->s_pf.reserve((size_t)ndp * 4 + 4, false, st);
+    CK(launch_run_stats(m->dpair.as<uint32_t>(), m->dseg.as<uint32_t>(), m->dperm.as<uint32_t>(), v.dpair_base, ndp,
+                        m->inc_len.as<float>(), m->inc_mu.as<float>(), slen, v.pair_base, m->pair_cum.as<float>(),
+                        m->pair_ndyn.as<uint32_t>(), m->pair_hit.as<float>(), m->s_pf.as<uint32_t>(), st));
+  }
+  v.n_pairs = np;
+  v.n_dperm = nd;
+  v.n_dpairs = ndp;
+  pair_total += np;
+  dperm_total += nd;
+  dpair_total += ndp;
 }
 
 // A view's rays in the SM-affine schedule: R regions of consecutive pixels
@@ -808,12 +772,6 @@ void stats_from_views(mrf_map* m) {
   m->stats.n_loud_prefix = m->loud_count_version == m->built_version ? m->n_loud_prefix : 0;
 }
 
-int voxel_id_bits(const mrf_map* m) {
-  int bits = 1;
-  while (bits < 32 && ((uint64_t)1 << bits) <= (uint64_t)(m->n_bricks * kBrickVox)) ++bits;
-  return bits;
-}
-
 // Incidence counts of the given views: view k's pixel counts at
 // s_counts + coff[k] (its hw entries and a sentinel) and their exclusive scan
 // at s_offs + coff[k]; each view's total is summed in 64 bits and the running
@@ -859,8 +817,8 @@ void emit_view(mrf_map* m, int c, const uint32_t* pix_off) {
   View& v = m->views[c];
   CK(launch_trace_emit(v.cam, v.pose, v.depth.as<float>(), pix_off, v.inc_base,
                        m->meta.as<RayMeta>() + v.pix_base, m->s_vox.as<uint32_t>() + (v.inc_base - m->scratch_base),
-                       m->inc_len.as<float>() + v.inc_base, m->inc_mu.as<float>() + v.inc_base,
-                       m->s_rec.as<float2>() + (v.inc_base - m->scratch_base), m->s_err.as<int>(), m->stream));
+                       m->inc_len.as<float>() + v.inc_base, m->inc_mu.as<float>() + v.inc_base, m->s_err.as<int>(),
+                       m->stream));
 }
 
 // tiles of view c's pair update, from position tb of tile_first
@@ -992,10 +950,8 @@ void rebuild_lists(mrf_map* m, OldPairs& old) {
     m->inc_pair.reserve(ib, false, m->stream);
     m->inc_len.reserve(ib, false, m->stream);
     m->inc_mu.reserve(ib, false, m->stream);
-    m->dperm.reserve(ib, false, m->stream);
     m->inc_pl.reserve(ib, false, m->stream);
     m->s_vox.reserve(ib, false, m->stream);
-    m->s_rec.reserve(ib * 2, false, m->stream);
     m->scratch_base = 0;
   }
   // 3. emit
@@ -1025,10 +981,11 @@ void rebuild_lists(mrf_map* m, OldPairs& old) {
     }
   });
   // 4. pairs per view
-  const int bits = voxel_id_bits(m);
-  int64_t pair_total = 0, perm_total = 0, dperm_total = 0, dpair_total = 0;
+  int64_t pair_total = 0, dperm_total = 0, dpair_total = 0, nd_all = 0;
+  for (int c : live) nd_all += m->views[c].c_ndyn;
   try {
-    for (int c = 0; c < V; ++c) view_pairs(m, c, bits, pair_total, perm_total, dperm_total, dpair_total);
+    m->dperm.reserve((size_t)std::max<int64_t>(nd_all, 1) * 4, false, m->stream);
+    for (int c = 0; c < V; ++c) view_pairs(m, c, pair_total, dperm_total, dpair_total);
   } catch (...) {
     lists_thread.join();
     throw;
@@ -1067,7 +1024,6 @@ void rebuild_lists(mrf_map* m, OldPairs& old) {
   }
   m->n_inc = n_inc;
   m->n_pairs = pair_total;
-  m->n_perm_total = perm_total;
   m->n_dperm = dperm_total;
   m->n_dpairs = dpair_total;
   size_t pb = (size_t)std::max<int64_t>(pair_total + 1, 1);
@@ -1077,7 +1033,6 @@ void rebuild_lists(mrf_map* m, OldPairs& old) {
   m->pair_stat.reserve(pb * 4, true, m->stream);
   m->pair_ndyn.reserve(pb * 4, true, m->stream);
   m->pair_hit.reserve(pb * 4, true, m->stream);
-  m->pair_seg.reserve(pb * 4, true, m->stream);
   m->dpair.reserve((size_t)(dpair_total + 1) * 4, true, m->stream);
   m->dseg.reserve((size_t)(dpair_total + 1) * 4, true, m->stream);
   if (dpair_total == 0) CK(launch_fill_u32(m->dseg.as<uint32_t>(), 1, 0u, m->stream));
@@ -1223,13 +1178,11 @@ bool append_lists(mrf_map* m) {
     m->inc_mu.reserve(ib, true, m->stream);
     m->inc_pair.reserve(ib, true, m->stream);
     m->inc_pl.reserve(ib, true, m->stream);
-    m->dperm.reserve((size_t)(m->n_dperm + (n_inc - m->n_inc)) * 4 + 4, true, m->stream);
     // scratch of the build: the new views' incidences only, from the first
     // new one on (the arenas' retired lists need none)
     m->scratch_base = (uint32_t)m->n_inc;
     const size_t sb = (size_t)std::max<int64_t>(n_inc - m->n_inc, 1) * 4;
     m->s_vox.reserve(sb, false, m->stream);
-    m->s_rec.reserve(sb * 2, false, m->stream);
   }
   for (size_t k = 0; k < added.size(); ++k) emit_view(m, added[k], m->s_offs.as<uint32_t>() + coff[k]);
   // the new views' ray records on the host, and their counters
@@ -1279,11 +1232,11 @@ bool append_lists(mrf_map* m) {
     if (read1(m, m->s_k1.as<uint32_t>())) v.n_loud = v.n_pairs;
   }
   // 4. pairs of the new views, numbered after the existing ones
-  const int bits = voxel_id_bits(m);
-  int64_t pair_total = m->n_pairs, perm_total = m->n_perm_total, dperm_total = m->n_dperm,
-          dpair_total = m->n_dpairs;
+  int64_t pair_total = m->n_pairs, dperm_total = m->n_dperm, dpair_total = m->n_dpairs, nd_all = m->n_dperm;
+  for (int c : added) nd_all += m->views[c].c_ndyn;
+  m->dperm.reserve((size_t)std::max<int64_t>(nd_all, 1) * 4, true, m->stream);
   const int64_t pair0 = pair_total, dpair0 = dpair_total;
-  for (int c : added) view_pairs(m, c, bits, pair_total, perm_total, dperm_total, dpair_total);
+  for (int c : added) view_pairs(m, c, pair_total, dperm_total, dpair_total);
   if (m->test_append_fail) {
     const mrf_status st = (mrf_status)m->test_append_fail;
     m->test_append_fail = 0;
@@ -1320,7 +1273,6 @@ bool append_lists(mrf_map* m) {
   }
   m->n_inc = n_inc;
   m->n_pairs = pair_total;
-  m->n_perm_total = perm_total;
   m->n_dperm = dperm_total;
   m->n_dpairs = dpair_total;
   const size_t pb = (size_t)std::max<int64_t>(pair_total + 1, 1);
@@ -1330,7 +1282,6 @@ bool append_lists(mrf_map* m) {
   m->pair_stat.reserve(pb * 4, true, m->stream);
   m->pair_ndyn.reserve(pb * 4, true, m->stream);
   m->pair_hit.reserve(pb * 4, true, m->stream);
-  m->pair_seg.reserve(pb * 4, true, m->stream);
   m->dpair.reserve((size_t)(dpair_total + 1) * 4, true, m->stream);
   m->dseg.reserve((size_t)(dpair_total + 1) * 4, true, m->stream);
   m->drun.reserve((size_t)(dpair_total + 1) * 16, true, m->stream);
@@ -1837,16 +1788,16 @@ void destroy_bufs(mrf_map* m) {
                  &m->meta, &m->inc_pair, &m->inc_len, &m->inc_mu, &m->inc_pl, &m->pair_vox,
                  &m->pair_m, &m->pair_cum, &m->pair_stat, &m->pair_ndyn, &m->pair_hit, &m->pair_q,
                  &m->pair_dm,
-                 &m->pair_seg, &m->dperm, &m->dpair, &m->dseg, &m->drun,
+                 &m->dperm, &m->dpair, &m->dseg, &m->drun,
                  &m->carry, &m->ray_order, &m->ray_queue, &m->region_q, &m->rstart, &m->rcounters, &m->counters, &m->tile_first,
                  &m->lbase, &m->lsingle, &m->lprefix, &m->queue_ids, &m->region_ids, &m->loud_off,
                  &m->loud, &m->quiet_ray,
                  &m->vseg, &m->vpairs, &m->vvox, &m->vox_active, &m->d_Lbase, &m->inc_len16, &m->pair_q16,
-                 &m->s_rec, &m->s_recs, &m->s_pf, &m->s_ps,
+                 &m->s_pf, &m->s_ps,
                  &m->s_flags, &m->s_ind, &m->s_scan,
-                 &m->s_q0, &m->s_q1, &m->s_q2, &m->s_q3, &m->s_bf, &m->s_loud, &m->s_pv, &m->s_sg,
+                 &m->s_q0, &m->s_q1, &m->s_q2, &m->s_q3, &m->s_q4, &m->s_bf, &m->s_first, &m->s_len, &m->s_loud,
                  &m->s_tmp, &m->s_counts, &m->s_offs, &m->s_vox, &m->s_k0, &m->s_k1, &m->s_v0,
-                 &m->s_v1, &m->s_seg, &m->s_dense, &m->s_err, &m->s_depth_in, &m->s_depth,
+                 &m->s_v1, &m->s_dense, &m->s_err, &m->s_depth_in, &m->s_depth,
                  &m->s_img, &m->s_part, &m->s_sum, &m->s_prev, &m->s_delta, &m->s_snap, &m->s_vcnt};
   for (DBuf* b : all) b->release();
   for (auto& v : m->views) v.depth.release();
@@ -2237,7 +2188,7 @@ mrf_status mrf_retire_view(mrf_map* m, int view_id) {
     // in the arenas is reclaimed by the next full build
     if (v.n_inc) m->holes = true;
     m->dead_inc += v.n_inc;
-    v.n_inc = v.n_pairs = v.n_perm = v.n_dperm = v.n_dpairs = v.n_active = v.n_left = v.n_loud = 0;
+    v.n_inc = v.n_pairs = v.n_dperm = v.n_dpairs = v.n_active = v.n_left = v.n_loud = 0;
     m->version++;
   });
 }

@@ -99,18 +99,34 @@ cudaError_t launch_brick_footprint(const Geom& g, const Pose& P, const int* coor
                                    uint8_t* mask, int* all, cudaStream_t s);
 cudaError_t launch_trace_emit(const Geom& g, const Pose& P, const float* depth,
                               const uint32_t* pix_off, uint32_t inc_base, RayMeta* meta,
-                              uint32_t* inc_vox, float* inc_len, float* inc_mu, float2* inc_rec,
-                              int* err, cudaStream_t s);
-// runs of the voxel-sorted incidences (the pairs before renumbering)
-cudaError_t launch_vox_heads(const uint32_t* sk, uint32_t n, uint32_t* flag, cudaStream_t s);
-// brick-major first-visit pair numbering (mrf_build.cu)
-cudaError_t launch_pair_first(const uint32_t* seg, uint32_t np, uint32_t perm_base, const uint32_t* sidx,
-                              uint32_t* key, cudaStream_t s);
-cudaError_t launch_brick_first(const uint32_t* pair_vox, const uint32_t* key, uint32_t np, uint32_t* bfirst,
+                              uint32_t* inc_vox, float* inc_len, float* inc_mu, int* err, cudaStream_t s);
+// the pairs of a view (mrf_build.cu): first incidence per voxel and brick;
+// voxel counts of the bricks in order; the pairs' numbers (table: first
+// incidences in, pair numbers out); the incidences' pairs, static lengths per
+// pair and the dynamic incidences; the pair statistics
+cudaError_t launch_first_visit(const uint32_t* vox, uint32_t n, uint32_t* first, uint32_t* bfirst,
                                cudaStream_t s);
-cudaError_t launch_brick_keys(const uint32_t* order, uint32_t np, const uint32_t* pair_vox,
-                              const uint32_t* bfirst, const uint8_t* loud, int bits, uint32_t* key,
-                              cudaStream_t s);
+cudaError_t launch_brick_count(const uint32_t* bkey, const uint32_t* order, uint32_t nb, const uint32_t* first,
+                               const uint8_t* loud, uint32_t* cnt, cudaStream_t s);
+cudaError_t launch_brick_number(const uint32_t* bkey, const uint32_t* order, uint32_t nb, uint32_t* table,
+                                const uint8_t* loud, const uint32_t* start, uint32_t pair_base, uint32_t* pair_vox,
+                                cudaStream_t s);
+cudaError_t launch_dyn_counts(const RayMeta* meta, uint32_t npix, uint32_t* cnt, cudaStream_t s);
+cudaError_t launch_assign_pairs(const RayMeta* meta, uint32_t npix, const uint32_t* vox, const float* len,
+                                const uint32_t* table, uint32_t inc_base, uint32_t pair_base, const uint32_t* doff,
+                                uint32_t* inc_pair, unsigned long long* static_len, uint32_t* dkey, uint32_t* dval,
+                                cudaStream_t s);
+cudaError_t launch_static_stats(const unsigned long long* static_len, uint32_t np, float* cum, float* stat,
+                                uint32_t* ndyn, float* hit, cudaStream_t s);
+cudaError_t launch_run_heads(const uint32_t* sk, uint32_t n, uint32_t* flag, cudaStream_t s);
+cudaError_t launch_runs(const uint32_t* sk, const uint32_t* flag, const uint32_t* scan, uint32_t n,
+                        uint32_t pair_base, uint32_t dperm_base, uint32_t* dpair, uint32_t* dseg, cudaStream_t s);
+// runs j0..j0+nrun (dpair, dseg); long_list: scratch of 1 + nrun u32 (count,
+// then the long runs)
+cudaError_t launch_run_stats(const uint32_t* dpair, const uint32_t* dseg, const uint32_t* dperm, uint32_t j0,
+                             uint32_t nrun, const float* len, const float* mu,
+                             const unsigned long long* static_len, uint32_t pair_base, float* cum, uint32_t* ndyn,
+                             float* hit, uint32_t* long_list, cudaStream_t s);
 // voxels with a dynamic incidence in any view (vox[k]: the voxel of
 // incidence vox_base + k), and the pairs on them
 cudaError_t launch_loud_voxels(const RayMeta* meta, int64_t npix, const uint32_t* vox, uint32_t vox_base,
@@ -123,31 +139,6 @@ cudaError_t launch_mark_active(const uint32_t* pair_vox, const float* cum, uint3
                                cudaStream_t s);
 cudaError_t launch_count_loud(const uint32_t* pair_vox, uint32_t np, const uint8_t* loud, uint32_t* count,
                               cudaStream_t s);
-cudaError_t launch_new_lengths(const uint32_t* order, uint32_t np, const uint32_t* seg, uint32_t* len,
-                               uint32_t* slot_of, cudaStream_t s);
-cudaError_t launch_move_positions(const uint32_t* sidx, const uint32_t* flag, const uint32_t* scan,
-                                  const uint32_t* seg, const uint32_t* slot_of, const uint32_t* start, uint32_t n,
-                                  uint32_t inc_base, uint32_t pair_base, uint32_t* out_idx, uint32_t* inc_pair,
-                                  cudaStream_t s);
-cudaError_t launch_pairs_renumbered(const uint32_t* order, uint32_t np, const uint32_t* vox_old,
-                                    const uint32_t* start, uint32_t pair_base, uint32_t perm_base,
-                                    uint32_t* pair_vox, uint32_t* seg, cudaStream_t s);
-// pairs from the pair-grouped incidences: pair_vox, seg and (when given)
-// inc_pair
-cudaError_t launch_pairs_from_sorted(const uint32_t* sk, const uint32_t* sidx, const uint32_t* flag,
-                                     const uint32_t* scan, uint32_t n, uint32_t pair_base,
-                                     uint32_t perm_base, uint32_t inc_base, uint32_t* pair_vox,
-                                     uint32_t* seg, uint32_t* inc_pair, cudaStream_t s);
-// build records (post length, -(mu l) on dynamic incidences) in sorted order
-// build records in pair-grouped order, and each position's dynamic flag
-cudaError_t launch_gather_rec(const uint32_t* sidx, uint32_t n, uint32_t inc_base, const float2* rec,
-                              float2* out, uint32_t* dflag, cudaStream_t s);
-// per pair: cumulative length, summed static messages, dynamic incidences,
-// potential mass (from the sorted records)
-// long_list: scratch of 1 + np u32 (count, then the pairs with long runs)
-cudaError_t launch_pair_stats(const uint32_t* seg, uint32_t p0, uint32_t np, uint32_t perm_base,
-                              const float2* srec, float* cum, float* stat, uint32_t* ndyn, float* hit,
-                              uint32_t* long_list, cudaStream_t s);
 // warm-start initial messages from a predicted log-odds field (voxel CSR)
 // (base: per-voxel log-odds without the live views' messages, or NULL for
 // the prior lp everywhere)
@@ -158,17 +149,6 @@ cudaError_t launch_warm_split(const uint32_t* vseg, const uint32_t* vpairs, cons
 cudaError_t launch_voxel_features(const uint32_t* vseg, const uint32_t* vpairs, const uint32_t* vvox,
                                   uint32_t nvox, const float* cum, const float* stat, const float* hit,
                                   const float* belief, int64_t n_slots_vox, float* feat, cudaStream_t s);
-// dynamic incidences of a view in pair-grouped order (dperm) and the pairs
-// that own them (dpair, with their first position dseg)
-cudaError_t launch_dyn_scatter(const uint32_t* sidx, const uint32_t* flag, const uint32_t* scan,
-                               uint32_t n, uint32_t inc_base, uint32_t dperm_base, uint32_t* dperm,
-                               cudaStream_t s);
-cudaError_t launch_dpair_flags(const uint32_t* ndyn, uint32_t p0, uint32_t np, uint32_t* flag,
-                               cudaStream_t s);
-cudaError_t launch_dpairs(const uint32_t* pflag, const uint32_t* pscan, uint32_t p0, uint32_t np,
-                          const uint32_t* seg, uint32_t perm_base, const uint32_t* dscan,
-                          uint32_t dperm_base, uint32_t dpair_base, uint32_t* dpair, uint32_t* dseg,
-                          cudaStream_t s);
 cudaError_t launch_iota(uint32_t* out, uint32_t n, cudaStream_t s);
 // CUB helpers (scratch-managed by the caller)
 size_t scan_temp_bytes(uint32_t n);
