@@ -320,106 +320,140 @@ __global__ void __launch_bounds__(kThreads, 4)
 // the incidences).  View of 104 M incidences at 1 cm: 13.5 ms with sorts of
 // all incidences by voxel and of all pairs by first visits.
 
-// first[v]: lowest index of an incidence on voxel v; bfirst[b]: the same for
-// brick b (a run of incidences in one brick reports its start).  Most
-// visits come after the first one: a look at the table saves the atomic.
-__global__ void k_first_visit(const uint32_t* __restrict__ vox, uint32_t n4, uint32_t* first, uint32_t* bfirst) {
+// first[v]: lowest index of an incidence on voxel v.  Most visits come after
+// the first one: a look at the table, stale in the SM's own cache at worst,
+// saves the atomic (0.56 ms for a view of 104 M incidences; a look in L2 takes
+// 0.92, near incidences through shared memory as below 0.56).
+__global__ void k_first_visit(const uint32_t* __restrict__ vox, uint32_t n4, uint32_t* first) {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n4) return;
   const uint4 u = reinterpret_cast<const uint4*>(vox)[t];
   const uint32_t v[4] = {u.x, u.y, u.z, u.w};
-  uint32_t last = t ? vox[4 * t - 1] : kNoVoxel;
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const uint32_t i = 4 * t + j;
-    if (v[j] != kNoVoxel) {
-      if (first[v[j]] > i) atomicMin(first + v[j], i);
-      const uint32_t b = v[j] / kBrickVox;
-      if (b != last / kBrickVox && bfirst[b] > i) atomicMin(bfirst + b, i);
-    }
-    last = v[j];
-  }
+  for (int j = 0; j < 4; ++j)
+    if (v[j] != kNoVoxel && first[v[j]] > 4 * t + j) atomicMin(first + v[j], 4 * t + j);
 }
 
-// bricks in the order of their first incidence (bkey, order; untouched ones
-// last): cnt[i] the loud voxels with an incidence of the i-th brick,
-// cnt[nb + i] the other voxels with one.  A warp per brick.
-__global__ void k_brick_count(const uint32_t* __restrict__ bkey, const uint32_t* __restrict__ order, uint32_t nb,
-                              const uint32_t* __restrict__ first, const uint8_t* __restrict__ loud,
-                              uint32_t* __restrict__ cnt) {
-  const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+// per brick: its first incidence (kNoVoxel: none), its loud voxels with an
+// incidence and its other voxels with one.  A warp per brick.
+__global__ void k_brick_count(uint32_t nb, const uint32_t* __restrict__ first, const uint8_t* __restrict__ loud,
+                              uint32_t* __restrict__ bfirst, uint32_t* __restrict__ bloud,
+                              uint32_t* __restrict__ bquiet) {
+  const uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (i >= nb) return;
-  uint32_t nl = 0, nq = 0;
-  if (bkey[i] != kNoVoxel) {
-    const size_t at = (size_t)order[i] * (kBrickVox / 4);
+  if (b >= nb) return;
+  uint32_t nl = 0, nq = 0, lo = kNoVoxel;
+  const size_t at = (size_t)b * (kBrickVox / 4);
 #pragma unroll
-    for (int k = 0; k < kBrickVox / 128; ++k) {
-      const uint4 f = reinterpret_cast<const uint4*>(first)[at + k * 32 + lane];
-      const uchar4 l = reinterpret_cast<const uchar4*>(loud)[at + k * 32 + lane];
-      auto add = [&](uint32_t fv, uint8_t lv) {
-        nl += fv != kNoVoxel && lv;
-        nq += fv != kNoVoxel && !lv;
-      };
-      add(f.x, l.x);
-      add(f.y, l.y);
-      add(f.z, l.z);
-      add(f.w, l.w);
-    }
+  for (int k = 0; k < kBrickVox / 128; ++k) {
+    const uint4 f = reinterpret_cast<const uint4*>(first)[at + k * 32 + lane];
+    const uchar4 l = reinterpret_cast<const uchar4*>(loud)[at + k * 32 + lane];
+    auto add = [&](uint32_t fv, uint8_t lv) {
+      nl += fv != kNoVoxel && lv;
+      nq += fv != kNoVoxel && !lv;
+      lo = min(lo, fv);
+    };
+    add(f.x, l.x);
+    add(f.y, l.y);
+    add(f.z, l.z);
+    add(f.w, l.w);
   }
   nl = __reduce_add_sync(0xFFFFFFFFu, nl);
   nq = __reduce_add_sync(0xFFFFFFFFu, nq);
+  lo = __reduce_min_sync(0xFFFFFFFFu, lo);
   if (lane == 0) {
-    cnt[i] = nl;
-    cnt[nb + i] = nq;
+    bfirst[b] = lo;
+    bloud[b] = nl;
+    bquiet[b] = nq;
+  }
+}
+
+// the counts in brick order: cnt[i] loud, cnt[nb + i] others, of brick order[i]
+__global__ void k_order_counts(const uint32_t* __restrict__ order, uint32_t nb, const uint32_t* __restrict__ bloud,
+                               const uint32_t* __restrict__ bquiet, uint32_t* __restrict__ cnt) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nb) return;
+  cnt[i] = bloud[order[i]];
+  cnt[nb + i] = bquiet[order[i]];
+}
+
+// Ascending bitonic sort of 512 keys of a warp, 16 per lane (element e = 16
+// lane + r): steps within a lane are register compares, the 15 others one
+// shuffle per key.
+__device__ __forceinline__ void warp_sort512(uint32_t (&x)[16], int lane) {
+#pragma unroll
+  for (int k = 2; k <= kBrickVox; k <<= 1) {
+#pragma unroll
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      if (j >= 16) {
+        const bool keep_min = ((lane & (j / 16)) == 0) == ((lane & (k / 16)) == 0);
+#pragma unroll
+        for (int r = 0; r < 16; ++r) {
+          const uint32_t y = __shfl_xor_sync(0xFFFFFFFFu, x[r], j / 16);
+          x[r] = keep_min ? min(x[r], y) : max(x[r], y);
+        }
+      } else {
+#pragma unroll
+        for (int r = 0; r < 16; ++r) {
+          if (r & j) continue;
+          const bool up = k < 16 ? (r & k) == 0 : (lane & (k / 16)) == 0;
+          const uint32_t lo = min(x[r], x[r | j]), hi = max(x[r], x[r | j]);
+          x[r] = up ? lo : hi;
+          x[r | j] = up ? hi : lo;
+        }
+      }
+    }
   }
 }
 
 // numbers of the i-th brick's pairs: its loud voxels from start[i] on, the
 // others from start[nb + i] on (start: the exclusive scan of cnt), each part
 // by first incidence.  Writes the pairs' voxels and turns the table's entries
-// into the voxels' pair numbers.  A block per brick: a bitonic sort of
-// (quiet, first incidence, voxel) keys in shared memory; a step whose pairs
-// lie within a warp's 64 keys needs no block barrier.
-constexpr int kNumberThreads = kBrickVox / 2;
-
-__global__ void __launch_bounds__(kNumberThreads)
+// into the voxels' pair numbers.  A warp per brick sorts the first incidences;
+// no two voxels share one, so vox gives each its voxel back.  (A block per
+// brick sorting 64-bit keys in shared memory: 0.61 ms for a 1 cm view of 13 M
+// pairs.)
+__global__ void __launch_bounds__(kThreads)
     k_brick_number(const uint32_t* __restrict__ bkey, const uint32_t* __restrict__ order, uint32_t nb,
-                   uint32_t* __restrict__ table, const uint8_t* __restrict__ loud,
+                   uint32_t* __restrict__ table, const uint8_t* __restrict__ loud, const uint32_t* __restrict__ vox,
                    const uint32_t* __restrict__ start, uint32_t pair_base, uint32_t* __restrict__ pair_vox) {
-  __shared__ unsigned long long key[kBrickVox];
-  const uint32_t i = blockIdx.x;
-  if (bkey[i] == kNoVoxel) return;
-  const uint32_t v0 = order[i] * kBrickVox;
-  const uint32_t t = threadIdx.x;
+  const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (i >= nb || bkey[i] == kNoVoxel) return;
+  const uint4* src = reinterpret_cast<const uint4*>(table) + (size_t)order[i] * (kBrickVox / 4);
+  uint32_t x[16];
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const uint32_t loc = t + h * kNumberThreads;
-    const uint32_t f = table[v0 + loc];
-    key[loc] = f == kNoVoxel ? ~0ull
-                             : ((unsigned long long)(loud[v0 + loc] ? 0u : 1u) << 62) | ((unsigned long long)f << 9) | loc;
+  for (int k = 0; k < 4; ++k) {
+    const uint4 f = src[k * 32 + lane];
+    x[4 * k + 0] = f.x;
+    x[4 * k + 1] = f.y;
+    x[4 * k + 2] = f.z;
+    x[4 * k + 3] = f.w;
   }
-  uint32_t prev = kBrickVox;
-  for (uint32_t k = 2; k <= kBrickVox; k <<= 1)
-    for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-      if (j > 32 || prev > 32) __syncthreads();
-      else __syncwarp();
-      prev = j;
-      const uint32_t a = 2 * t - (t & (j - 1)), b = a + j;
-      const unsigned long long x = key[a], y = key[b];
-      if ((x > y) == ((a & k) == 0)) {
-        key[a] = y;
-        key[b] = x;
-      }
-    }
-  __syncthreads();
-  const uint32_t l0 = start[i], nl = start[i + 1] - l0;
-  const uint32_t q0 = start[nb + i], n = nl + start[nb + i + 1] - q0;
-  for (uint32_t r = t; r < n; r += kNumberThreads) {
-    const uint32_t v = v0 + (uint32_t)(key[r] & (kBrickVox - 1));
-    const uint32_t q = r < nl ? l0 + r : q0 + (r - nl);
-    pair_vox[pair_base + q] = v;
-    table[v] = q;
+  warp_sort512(x, lane);  // voxels without an incidence (kNoVoxel) last
+  // loud voxels before each of the lane's, then every voxel's number
+  unsigned is_loud = 0;
+#pragma unroll
+  for (int k = 0; k < 16; ++k) {
+    if (x[k] == kNoVoxel) continue;
+    x[k] = vox[x[k]];
+    if (loud[x[k]]) is_loud |= 1u << k;
+  }
+  uint32_t nl = __popc(is_loud);
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, nl, o);
+    if (lane >= o) nl += u;
+  }
+  nl -= __popc(is_loud);
+  const uint32_t l0 = start[i], q0 = start[nb + i];
+#pragma unroll
+  for (int k = 0; k < 16; ++k) {
+    if (x[k] == kNoVoxel) continue;
+    const uint32_t before = nl + __popc(is_loud & ((1u << k) - 1u));
+    const uint32_t q = (is_loud >> k) & 1u ? l0 + before : q0 + (16 * lane + k - before);
+    pair_vox[pair_base + q] = x[k];
+    table[x[k]] = q;
   }
 }
 
@@ -434,41 +468,82 @@ __device__ __forceinline__ float len_float(long long s) { return __ll2float_rn(s
 
 // every incidence's pair id; the static incidences' lengths summed per pair;
 // the dynamic incidences (pair number, incidence index) listed in ray order
-// at doff[r].  Eight lanes per ray, four incidences each.
-constexpr int kAssignLanes = 8;
+// at doff[r].
+//
+// All rays start at the camera: its voxel gets a length from every ray of the
+// view, the ones around it from thousands, and their atomics serialise (1.9
+// ms of a 1 cm view, 0.7 without the first 64 incidences of each ray).  A
+// block takes kNearRays consecutive rays, which cross the same near voxels,
+// and adds up the lengths of a ray's first kNear incidences in a shared hash
+// table (four probes; a pair that finds no place goes straight to memory):
+// the low 21 bits and the rest apart, in 32-bit sums that kNearRays additions
+// of at most 2^41 cannot overflow.  0.67 ms; a small image (160x120) wants few
+// rays a block: 0.05 ms with 64, 0.03 with 32.
+constexpr int kRayLanes = 8;  // lanes per ray, four incidences each
+constexpr int kNearThreads = 128;
+constexpr int kNearRays = 32;
+constexpr int kNear = 64;
+constexpr uint32_t kNearSlots = 1024;
+static_assert(kNearSlots == 1u << 10, "the hash keeps ten bits");
 
-__global__ void k_assign_pairs(const RayMeta* __restrict__ meta, uint32_t npix, const uint32_t* __restrict__ vox,
-                               const float* __restrict__ len, const uint32_t* __restrict__ table,
-                               uint32_t inc_base, uint32_t pair_base, const uint32_t* __restrict__ doff,
-                               uint32_t* __restrict__ inc_pair, unsigned long long* __restrict__ static_len,
-                               uint32_t* __restrict__ dkey, uint32_t* __restrict__ dval) {
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t r = t / kAssignLanes;
-  if (r >= npix) return;
-  const RayMeta me = meta[r];
-  const int n = me.n_pre, np = me.n_post, kd = ray_kdyn(me);
-  const uint32_t off = me.off - inc_base;
-  const uint32_t d0 = doff[r] - (uint32_t)kd;
-  for (int i = 4 * (t % kAssignLanes); i < n; i += 4 * kAssignLanes) {
-    const uint4 u = *reinterpret_cast<const uint4*>(vox + off + i);
-    const float4 lv = *reinterpret_cast<const float4*>(len + off + i);
-    const uint32_t v[4] = {u.x, u.y, u.z, u.w};
-    const float l[4] = {lv.x, lv.y, lv.z, lv.w};
-    uint32_t q[4];
+__global__ void __launch_bounds__(kNearThreads)
+    k_assign_pairs(const RayMeta* __restrict__ meta, uint32_t npix, const uint32_t* __restrict__ vox,
+                   const float* __restrict__ len, const uint32_t* __restrict__ table, uint32_t inc_base,
+                   uint32_t pair_base, const uint32_t* __restrict__ doff, uint32_t* __restrict__ inc_pair,
+                   unsigned long long* __restrict__ static_len, uint32_t* __restrict__ dkey,
+                   uint32_t* __restrict__ dval) {
+  __shared__ uint32_t skey[kNearSlots], slo[kNearSlots], shi[kNearSlots];
+  for (uint32_t k = threadIdx.x; k < kNearSlots; k += kNearThreads) {
+    skey[k] = kNoVoxel;
+    slo[k] = 0u;
+    shi[k] = 0u;
+  }
+  __syncthreads();
+  const uint32_t r1 = min(npix, (blockIdx.x + 1) * kNearRays);
+  for (uint32_t r = blockIdx.x * kNearRays + threadIdx.x / kRayLanes; r < r1; r += kNearThreads / kRayLanes) {
+    const RayMeta me = meta[r];
+    const int n = me.n_pre, np = me.n_post, kd = ray_kdyn(me);
+    const uint32_t off = me.off - inc_base;
+    const uint32_t d0 = doff[r] - (uint32_t)kd;
+    for (int i = 4 * (threadIdx.x % kRayLanes); i < n; i += 4 * kRayLanes) {
+      const uint4 u = *reinterpret_cast<const uint4*>(vox + off + i);
+      const float4 lv = *reinterpret_cast<const float4*>(len + off + i);
+      const uint32_t v[4] = {u.x, u.y, u.z, u.w};
+      const float l[4] = {lv.x, lv.y, lv.z, lv.w};
+      uint32_t q[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) q[j] = i + j < n ? table[v[j]] : 0u;
-    *reinterpret_cast<uint4*>(inc_pair + off + i) =
-        make_uint4(pair_base + q[0], pair_base + q[1], pair_base + q[2], pair_base + q[3]);
+      for (int j = 0; j < 4; ++j) q[j] = i + j < n ? table[v[j]] : 0u;
+      *reinterpret_cast<uint4*>(inc_pair + off + i) =
+          make_uint4(pair_base + q[0], pair_base + q[1], pair_base + q[2], pair_base + q[3]);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      if (i + j < kd) {
-        atomicAdd(static_len + q[j], (unsigned long long)len_fixed(l[j]));
-      } else if (i + j < np) {
-        dkey[d0 + i + j] = q[j];
-        dval[d0 + i + j] = me.off + i + j;
+      for (int j = 0; j < 4; ++j) {
+        if (i + j < kd) {
+          const unsigned long long x = (unsigned long long)len_fixed(l[j]);
+          bool added = false;
+          if (i < kNear) {
+            uint32_t h = (q[j] * 2654435761u) >> 22;
+            for (int probe = 0; probe < 4 && !added; ++probe) {
+              const uint32_t old = skey[h] == q[j] ? q[j] : atomicCAS(skey + h, kNoVoxel, q[j]);
+              added = old == q[j] || old == kNoVoxel;
+              if (!added) h = (h + 1) & (kNearSlots - 1);
+            }
+            if (added) {
+              atomicAdd(slo + h, (uint32_t)x & 0x1FFFFFu);
+              atomicAdd(shi + h, (uint32_t)(x >> 21));
+            }
+          }
+          if (!added) atomicAdd(static_len + q[j], x);
+        } else if (i + j < np) {
+          dkey[d0 + i + j] = q[j];
+          dval[d0 + i + j] = me.off + i + j;
+        }
       }
     }
   }
+  __syncthreads();
+  for (uint32_t k = threadIdx.x; k < kNearSlots; k += kNearThreads)
+    if (skey[k] != kNoVoxel)
+      atomicAdd(static_len + skey[k], (unsigned long long)slo[k] + ((unsigned long long)shi[k] << 21));
 }
 
 // dynamic incidences of each ray
@@ -748,25 +823,32 @@ cudaError_t launch_trace_emit(const Geom& g, const Pose& P, const float* depth,
   return cudaGetLastError();
 }
 
-cudaError_t launch_first_visit(const uint32_t* vox, uint32_t n, uint32_t* first, uint32_t* bfirst,
-                               cudaStream_t s) {
+cudaError_t launch_first_visit(const uint32_t* vox, uint32_t n, uint32_t* first, cudaStream_t s) {
   if (!n) return cudaSuccess;
-  k_first_visit<<<grid_for(n / 4), kThreads, 0, s>>>(vox, n / 4, first, bfirst);
+  k_first_visit<<<grid_for(n / 4), kThreads, 0, s>>>(vox, n / 4, first);
   return cudaGetLastError();
 }
 
-cudaError_t launch_brick_count(const uint32_t* bkey, const uint32_t* order, uint32_t nb, const uint32_t* first,
-                               const uint8_t* loud, uint32_t* cnt, cudaStream_t s) {
+cudaError_t launch_brick_count(uint32_t nb, const uint32_t* first, const uint8_t* loud, uint32_t* bfirst,
+                               uint32_t* bloud, uint32_t* bquiet, cudaStream_t s) {
   if (!nb) return cudaSuccess;
-  k_brick_count<<<grid_for((int64_t)nb * 32), kThreads, 0, s>>>(bkey, order, nb, first, loud, cnt);
+  k_brick_count<<<grid_for((int64_t)nb * 32), kThreads, 0, s>>>(nb, first, loud, bfirst, bloud, bquiet);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_order_counts(const uint32_t* order, uint32_t nb, const uint32_t* bloud, const uint32_t* bquiet,
+                                uint32_t* cnt, cudaStream_t s) {
+  if (!nb) return cudaSuccess;
+  k_order_counts<<<grid_for(nb), kThreads, 0, s>>>(order, nb, bloud, bquiet, cnt);
   return cudaGetLastError();
 }
 
 cudaError_t launch_brick_number(const uint32_t* bkey, const uint32_t* order, uint32_t nb, uint32_t* table,
-                                const uint8_t* loud, const uint32_t* start, uint32_t pair_base, uint32_t* pair_vox,
-                                cudaStream_t s) {
+                                const uint8_t* loud, const uint32_t* vox, const uint32_t* start,
+                                uint32_t pair_base, uint32_t* pair_vox, cudaStream_t s) {
   if (!nb) return cudaSuccess;
-  k_brick_number<<<nb, kNumberThreads, 0, s>>>(bkey, order, nb, table, loud, start, pair_base, pair_vox);
+  k_brick_number<<<grid_for((int64_t)nb * 32), kThreads, 0, s>>>(bkey, order, nb, table, loud, vox, start, pair_base,
+                                                                 pair_vox);
   return cudaGetLastError();
 }
 
@@ -781,7 +863,7 @@ cudaError_t launch_assign_pairs(const RayMeta* meta, uint32_t npix, const uint32
                                 uint32_t* inc_pair, unsigned long long* static_len, uint32_t* dkey, uint32_t* dval,
                                 cudaStream_t s) {
   if (!npix) return cudaSuccess;
-  k_assign_pairs<<<grid_for((int64_t)npix * kAssignLanes, 128), 128, 0, s>>>(
+  k_assign_pairs<<<grid_for(npix, kNearRays), kNearThreads, 0, s>>>(
       meta, npix, vox, len, table, inc_base, pair_base, doff, inc_pair, static_len, dkey, dval);
   return cudaGetLastError();
 }

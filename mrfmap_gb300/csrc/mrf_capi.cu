@@ -216,7 +216,7 @@ struct mrf_map {
   std::vector<View> views;
   // arenas
   DBuf meta, inc_pair, inc_len, inc_mu, inc_pl, pair_vox, pair_m, pair_cum, pair_stat, pair_ndyn, pair_hit,
-      pair_q, pair_dm, dperm, s_q0, s_q1, s_q2, s_q3, s_q4, s_bf, s_first, s_len, s_loud, dpair, dseg, drun, carry, ray_order, ray_queue, region_q, rstart, rcounters, counters,
+      pair_q, pair_dm, dperm, s_q0, s_q1, s_q2, s_q3, s_q4, s_bf, s_bc, s_first, s_len, s_loud, dpair, dseg, drun, carry, ray_order, ray_queue, region_q, rstart, rcounters, counters,
       tile_first, lbase, lsingle, lprefix, queue_ids, region_ids, loud_off, loud, quiet_ray;
   uint32_t jac_tile_base = 0;
   int64_t n_inc = 0, n_pairs = 0, n_dperm = 0, n_dpairs = 0;
@@ -458,9 +458,10 @@ void view_pairs(mrf_map* m, int c, int64_t& pair_total, int64_t& dperm_total, in
   m->s_first.reserve((size_t)nb * kBrickVox * 4, false, st);
   m->s_bf.reserve((size_t)nb * 4, false, st);
   CK(cudaMemsetAsync(m->s_first.p, 0xFF, (size_t)nb * kBrickVox * 4, st));
-  CK(cudaMemsetAsync(m->s_bf.p, 0xFF, (size_t)nb * 4, st));
   uint32_t* table = m->s_first.as<uint32_t>();
-  CK(launch_first_visit(vox, n, table, m->s_bf.as<uint32_t>(), st));
+  const RayMeta* rays = m->meta.as<RayMeta>() + v.pix_base;
+  CK(launch_first_visit(vox, n, table, st));
+  m->s_bc.reserve((size_t)2 * nb * 4, false, st);
   m->s_q0.reserve((size_t)nb * 4, false, st);
   m->s_q1.reserve((size_t)nb * 4, false, st);
   m->s_q2.reserve((size_t)nb * 4, false, st);
@@ -472,10 +473,12 @@ void view_pairs(mrf_map* m, int c, int64_t& pair_total, int64_t& dperm_total, in
   const uint32_t* order = m->s_q2.as<uint32_t>();
   uint32_t* cnt = m->s_q3.as<uint32_t>();
   uint32_t* start = m->s_q4.as<uint32_t>();
+  uint32_t* bloud = m->s_bc.as<uint32_t>();
+  CK(launch_brick_count(nb, table, m->s_loud.as<uint8_t>(), m->s_bf.as<uint32_t>(), bloud, bloud + nb, st));
   CK(launch_iota(m->s_q1.as<uint32_t>(), nb, st));
   CK(sort_pairs_u32(m->s_tmp.p, ts, m->s_bf.as<uint32_t>(), m->s_q0.as<uint32_t>(), m->s_q1.as<uint32_t>(),
                     m->s_q2.as<uint32_t>(), nb, 32, st));
-  CK(launch_brick_count(bkey, order, nb, table, m->s_loud.as<uint8_t>(), cnt, st));
+  CK(launch_order_counts(order, nb, bloud, bloud + nb, cnt, st));
   CK(cudaMemsetAsync(cnt + 2 * (size_t)nb, 0, 4, st));
   CK(exclusive_scan_u32(m->s_tmp.p, ts, cnt, start, 2 * nb + 1, st));
   uint32_t np = 0;
@@ -486,7 +489,7 @@ void view_pairs(mrf_map* m, int c, int64_t& pair_total, int64_t& dperm_total, in
   m->s_ps.reserve((size_t)npix * 4 + 4, false, st);
   const size_t tp = scan_temp_bytes(npix);
   m->s_pf.reserve(tp, false, st);
-  CK(launch_dyn_counts(m->meta.as<RayMeta>() + v.pix_base, npix, m->s_k0.as<uint32_t>(), st));
+  CK(launch_dyn_counts(rays, npix, m->s_k0.as<uint32_t>(), st));
   CK(exclusive_scan_u32(m->s_pf.p, tp, m->s_k0.as<uint32_t>(), m->s_ps.as<uint32_t>(), npix, st));
   sync(m);
   u32_checked(pair_total + np + 1, "pair count");
@@ -497,7 +500,7 @@ void view_pairs(mrf_map* m, int c, int64_t& pair_total, int64_t& dperm_total, in
   m->pair_stat.reserve(pb * 4, true, st);
   m->pair_ndyn.reserve(pb * 4, true, st);
   m->pair_hit.reserve(pb * 4, true, st);
-  CK(launch_brick_number(bkey, order, nb, table, m->s_loud.as<uint8_t>(), start, v.pair_base,
+  CK(launch_brick_number(bkey, order, nb, table, m->s_loud.as<uint8_t>(), vox, start, v.pair_base,
                          m->pair_vox.as<uint32_t>(), st));
   // the incidences' pairs; pair numbers and indices of the dynamic ones in
   // s_k0, s_v0, sorted by pair (stable: increasing incidence within a pair)
@@ -506,8 +509,8 @@ void view_pairs(mrf_map* m, int c, int64_t& pair_total, int64_t& dperm_total, in
   m->s_k1.reserve((size_t)nd * 4 + 4, false, st);
   CK(cudaMemsetAsync(m->s_len.p, 0, (size_t)np * 8, st));
   unsigned long long* slen = m->s_len.as<unsigned long long>();
-  CK(launch_assign_pairs(m->meta.as<RayMeta>() + v.pix_base, npix, vox, m->inc_len.as<float>() + v.inc_base, table,
-                         v.inc_base, v.pair_base, m->s_ps.as<uint32_t>(), m->inc_pair.as<uint32_t>() + v.inc_base,
+  CK(launch_assign_pairs(rays, npix, vox, m->inc_len.as<float>() + v.inc_base, table, v.inc_base, v.pair_base,
+                         m->s_ps.as<uint32_t>(), m->inc_pair.as<uint32_t>() + v.inc_base,
                          slen, m->s_k0.as<uint32_t>(), m->s_v0.as<uint32_t>(), st));
   CK(launch_static_stats(slen, np, m->pair_cum.as<float>() + v.pair_base, m->pair_stat.as<float>() + v.pair_base,
                          m->pair_ndyn.as<uint32_t>() + v.pair_base, m->pair_hit.as<float>() + v.pair_base, st));
@@ -1795,7 +1798,7 @@ void destroy_bufs(mrf_map* m) {
                  &m->vseg, &m->vpairs, &m->vvox, &m->vox_active, &m->d_Lbase, &m->inc_len16, &m->pair_q16,
                  &m->s_pf, &m->s_ps,
                  &m->s_flags, &m->s_ind, &m->s_scan,
-                 &m->s_q0, &m->s_q1, &m->s_q2, &m->s_q3, &m->s_q4, &m->s_bf, &m->s_first, &m->s_len, &m->s_loud,
+                 &m->s_q0, &m->s_q1, &m->s_q2, &m->s_q3, &m->s_q4, &m->s_bf, &m->s_bc, &m->s_first, &m->s_len, &m->s_loud,
                  &m->s_tmp, &m->s_counts, &m->s_offs, &m->s_vox, &m->s_k0, &m->s_k1, &m->s_v0,
                  &m->s_v1, &m->s_dense, &m->s_err, &m->s_depth_in, &m->s_depth,
                  &m->s_img, &m->s_part, &m->s_sum, &m->s_prev, &m->s_delta, &m->s_snap, &m->s_vcnt};

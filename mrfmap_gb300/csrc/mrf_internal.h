@@ -104,13 +104,14 @@ cudaError_t launch_trace_emit(const Geom& g, const Pose& P, const float* depth,
 // voxel counts of the bricks in order; the pairs' numbers (table: first
 // incidences in, pair numbers out); the incidences' pairs, static lengths per
 // pair and the dynamic incidences; the pair statistics
-cudaError_t launch_first_visit(const uint32_t* vox, uint32_t n, uint32_t* first, uint32_t* bfirst,
-                               cudaStream_t s);
-cudaError_t launch_brick_count(const uint32_t* bkey, const uint32_t* order, uint32_t nb, const uint32_t* first,
-                               const uint8_t* loud, uint32_t* cnt, cudaStream_t s);
+cudaError_t launch_first_visit(const uint32_t* vox, uint32_t n, uint32_t* first, cudaStream_t s);
+cudaError_t launch_brick_count(uint32_t nb, const uint32_t* first, const uint8_t* loud, uint32_t* bfirst,
+                               uint32_t* bloud, uint32_t* bquiet, cudaStream_t s);
+cudaError_t launch_order_counts(const uint32_t* order, uint32_t nb, const uint32_t* bloud, const uint32_t* bquiet,
+                                uint32_t* cnt, cudaStream_t s);
 cudaError_t launch_brick_number(const uint32_t* bkey, const uint32_t* order, uint32_t nb, uint32_t* table,
-                                const uint8_t* loud, const uint32_t* start, uint32_t pair_base, uint32_t* pair_vox,
-                                cudaStream_t s);
+                                const uint8_t* loud, const uint32_t* vox, const uint32_t* start,
+                                uint32_t pair_base, uint32_t* pair_vox, cudaStream_t s);
 cudaError_t launch_dyn_counts(const RayMeta* meta, uint32_t npix, uint32_t* cnt, cudaStream_t s);
 cudaError_t launch_assign_pairs(const RayMeta* meta, uint32_t npix, const uint32_t* vox, const float* len,
                                 const uint32_t* table, uint32_t inc_base, uint32_t pair_base, const uint32_t* doff,
