@@ -168,12 +168,9 @@ __global__ void __launch_bounds__(kThreads, 4)
     k_trace(Geom g, Pose P, const float* __restrict__ depth, uint32_t* __restrict__ counts,
             const uint32_t* __restrict__ pix_off, uint32_t inc_base, RayMeta* __restrict__ meta,
             uint32_t* __restrict__ inc_vox, float* __restrict__ inc_len,
-            float* __restrict__ inc_mu, int* __restrict__ err, const uint8_t* __restrict__ only, const int* __restrict__ only_all) {
+            float* __restrict__ inc_mu, int* __restrict__ err) {
   int pix = blockIdx.x * blockDim.x + threadIdx.x;
   if (pix >= g.rows * g.cols) return;
-  // a checking count pass may be limited to the pixels marked in `only`
-  // (unless *only_all is set)
-  if (only && !*only_all && !only[pix]) return;
   float d = depth[pix];
   int count = 0, n_pre = -1, n_post = -1, r0 = -1, run_start = 0, kmu = -1;
   bool gate = false;
@@ -235,13 +232,6 @@ __global__ void __launch_bounds__(kThreads, 4)
         }
         float s = fm(te, ray.mult);
         if (!run_open) run_start = count;
-        if (!EMIT && meta && (r0 < 0 || kmu < 0)) {
-          // a checking count pass: the visibility-reset and dynamic starts
-          // of the record it compares against
-          const bool z = potential_is_zero(sg, bs, n, s, d);
-          if (r0 < 0 && !z) r0 = run_start;
-          if (kmu < 0 && !z) kmu = count;
-        }
         if (EMIT) {
           const bool z = potential_is_zero(sg, bs, n, s, d);
           const float mu = z ? 0.0f : potential(sg, bs, n, s, d);
@@ -273,16 +263,6 @@ __global__ void __launch_bounds__(kThreads, 4)
   const int padded = (n_pre + 3) & ~3;
   if (!EMIT) {
     counts[pix] = (uint32_t)padded;
-    if (meta) {
-      // the view's stored records: does this trace still give the same list?
-      const int kdyn = (kmu >= 0 && kmu < n_post) ? kmu : n_post;
-      const RayMeta o = meta[pix];
-      const uint32_t flags = (gate ? 1u : 0u) | ((uint32_t)kdyn << 16);
-      if (o.n_pre != (uint16_t)n_pre || o.n_post != (uint16_t)n_post ||
-          o.r0 != (uint16_t)(r0 >= 0 ? r0 : n_pre) || o.rinf != (uint16_t)(r0 >= 0 ? r0 : run_start) ||
-          o.flags != flags)
-        err[1] = 1;
-    }
   } else {
     // the last group, completed with padding (invalid voxel, zeros)
     if (count & 3) {
@@ -563,15 +543,6 @@ __global__ void k_loud_voxels(const RayMeta* __restrict__ meta, int64_t npix, co
   for (int i = ray_kdyn(me); i < me.n_post; ++i) loud[vox[me.off - vox_base + i]] = 1;
 }
 
-__global__ void k_loud_voxels_from_pairs(const RayMeta* __restrict__ meta, int64_t npix,
-                                         const uint32_t* __restrict__ inc_pair,
-                                         const uint32_t* __restrict__ pair_vox, uint8_t* __restrict__ loud) {
-  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= npix) return;
-  const RayMeta me = meta[r];
-  for (int i = ray_kdyn(me); i < me.n_post; ++i) loud[pair_vox[inc_pair[me.off + i]]] = 1;
-}
-
 // *count += number of pairs on loud voxels
 __global__ void k_count_loud(const uint32_t* __restrict__ pair_vox, uint32_t np,
                              const uint8_t* __restrict__ loud, uint32_t* __restrict__ count) {
@@ -754,10 +725,9 @@ cudaError_t launch_set_points(const Geom& g, const float* pts, const float* occ,
 }
 
 cudaError_t launch_trace_count(const Geom& g, const Pose& P, const float* depth, uint32_t* counts,
-                               int* err, cudaStream_t s, const RayMeta* check, const uint8_t* only,
-                               const int* only_all) {
+                               int* err, cudaStream_t s) {
   k_trace<false><<<grid_for((int64_t)g.rows * g.cols), kThreads, 0, s>>>(
-      g, P, depth, counts, nullptr, 0, const_cast<RayMeta*>(check), nullptr, nullptr, nullptr, err, only, only_all);
+      g, P, depth, counts, nullptr, 0, nullptr, nullptr, nullptr, nullptr, err);
   return cudaGetLastError();
 }
 
@@ -819,7 +789,7 @@ cudaError_t launch_trace_emit(const Geom& g, const Pose& P, const float* depth,
                               const uint32_t* pix_off, uint32_t inc_base, RayMeta* meta,
                               uint32_t* inc_vox, float* inc_len, float* inc_mu, int* err, cudaStream_t s) {
   k_trace<true><<<grid_for((int64_t)g.rows * g.cols), kThreads, 0, s>>>(
-      g, P, depth, nullptr, pix_off, inc_base, meta, inc_vox, inc_len, inc_mu, err, nullptr, nullptr);
+      g, P, depth, nullptr, pix_off, inc_base, meta, inc_vox, inc_len, inc_mu, err);
   return cudaGetLastError();
 }
 
@@ -907,13 +877,6 @@ cudaError_t launch_loud_voxels(const RayMeta* meta, int64_t npix, const uint32_t
                                uint8_t* loud, cudaStream_t s) {
   if (npix <= 0) return cudaSuccess;
   k_loud_voxels<<<grid_for(npix), kThreads, 0, s>>>(meta, npix, vox, vox_base, loud);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_loud_voxels_from_pairs(const RayMeta* meta, int64_t npix, const uint32_t* inc_pair,
-                                          const uint32_t* pair_vox, uint8_t* loud, cudaStream_t s) {
-  if (npix <= 0) return cudaSuccess;
-  k_loud_voxels_from_pairs<<<grid_for(npix), kThreads, 0, s>>>(meta, npix, inc_pair, pair_vox, loud);
   return cudaGetLastError();
 }
 

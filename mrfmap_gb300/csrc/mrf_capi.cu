@@ -193,13 +193,13 @@ struct mrf_map {
   int variant_for(bool all_views) const { return ray_variant_chosen || !all_views ? ray_variant : 1; }
   uint32_t nreg = 1;    // SM regions per view of the region queues
   // what the last build left: views with lists, per-pixel entries, the ends
-  // of the region blocks, the queues and the tiles, the bricks it saw
+  // of the region blocks, the queues and the tiles
   int built_views = 0;
   int64_t npix_total = 0, queue_end = 0, tile_end = 0, carry_tiles = 0, vox_active_n = 0;
   int64_t n_loud_prefix = 0;  // entries of the static prefixes' loud lists
   int64_t loud_count_version = -1, loud_list_version = -1;  // builds the loud lists were counted / made for
   uint32_t region_end = 0;
-  int64_t bricks_at_build = -1;
+  int64_t loud_n = 0;  // voxels s_loud holds a flag for
   // holes: retired views' lists still in the arenas; appended: lists added
   // without a full build (the all-view structures of Jacobi are stale);
   // needs_full: the next build must rebuild every view
@@ -970,6 +970,7 @@ void rebuild_lists(mrf_map* m, OldPairs& old) {
   // quiet, see enqueue_iteration)
   m->s_loud.reserve((size_t)std::max<int64_t>(m->n_bricks * kBrickVox, 1), false, m->stream);
   CK(cudaMemsetAsync(m->s_loud.p, 0, (size_t)std::max<int64_t>(m->n_bricks * kBrickVox, 1), m->stream));
+  m->loud_n = m->n_bricks * kBrickVox;
   CK(launch_loud_voxels(m->meta.as<RayMeta>(), npix, m->s_vox.as<uint32_t>(), 0u, m->s_loud.as<uint8_t>(),
                         m->stream));
   // the region lists of the SM-affine schedule are host work on the ray
@@ -1101,7 +1102,6 @@ void rebuild_lists(mrf_map* m, OldPairs& old) {
   m->jacobi_version = -1;
   m->built_views = V;
   m->npix_total = npix;
-  m->bricks_at_build = m->n_bricks;
   m->holes = false;
   m->needs_full = false;
   m->dead_inc = 0;
@@ -1110,47 +1110,17 @@ void rebuild_lists(mrf_map* m, OldPairs& old) {
 
 // Appends the lists of the views added since the last build (a full-ray
 // map only; see ensure_built), leaving the other views' lists, pairs and
-// messages as they are: every brick a full-ray view's rays cross before
-// their stop was activated by the view itself, so bricks activated later
-// change no old list -- which a count pass over the old views, compared
-// with their stored ray records, confirms whenever the brick set grew.
-// Returns false (nothing changed) when a full build is needed instead.
-bool append_lists(mrf_map* m) {
+// messages as they are.  That is exact: a view's activation walks the same
+// rays with the same arithmetic as its trace and activates every brick up to
+// the run that stops the trace, so the trace meets active bricks only until
+// it stops, whatever bricks other views activate later.  (Tracing the old
+// views' pixels around new bricks again, to compare them with their records,
+// took 37 of a 16-frame walk's 178 ms and could find nothing.)
+void append_lists(mrf_map* m) {
   const int V = (int)m->views.size();
   CK(cudaEventRecord(m->ev0, m->stream));
   m->g.brick_slot = m->d_slot.as<int>();
   for (View& v : m->views) v.cam.brick_slot = m->g.brick_slot;
-  if (m->n_bricks != m->bricks_at_build) {
-    // err[1]: the count pass's mismatch flag (err[0], the kernels' error
-    // flag, is left as it is and checked below).  Only the pixels whose
-    // rays may cross a brick activated since the last build are traced
-    // again (their footprint through each view's camera); err[2] tells the
-    // pass to check every pixel of the view.
-    CK(cudaMemsetAsync(m->s_err.as<int>() + 1, 0, 4, m->stream));
-    const uint32_t b0 = (uint32_t)std::max<int64_t>(m->bricks_at_build, 0), b1 = (uint32_t)m->n_bricks;
-    for (int c = 0; c < m->built_views; ++c) {
-      const View& v = m->views[c];
-      const int64_t hw = view_pixels(v);
-      if (!hw) continue;
-      m->s_counts.reserve((size_t)hw * 4 + 4, false, m->stream);
-      m->s_dense.reserve((size_t)hw + 16, false, m->stream);
-      CK(cudaMemsetAsync(m->s_dense.p, 0, (size_t)hw, m->stream));
-      CK(cudaMemsetAsync(m->s_err.as<int>() + 2, 0, 4, m->stream));
-      CK(launch_brick_footprint(v.cam, v.pose, m->d_coord.as<int>(), b0, b1, m->s_dense.as<uint8_t>(),
-                                m->s_err.as<int>() + 2, m->stream));
-      CK(launch_trace_count(v.cam, v.pose, v.depth.as<float>(), m->s_counts.as<uint32_t>(), m->s_err.as<int>(),
-                            m->stream, m->meta.as<RayMeta>() + v.pix_base, m->s_dense.as<uint8_t>(),
-                            m->s_err.as<int>() + 2));
-    }
-    int flags[2] = {0, 0};
-    CK(cudaMemcpyAsync(flags, m->s_err.p, 8, cudaMemcpyDeviceToHost, m->stream));
-    sync(m);
-    check_device_err(m);
-    if (flags[1]) {
-      CK(cudaMemsetAsync(m->s_err.as<int>() + 1, 0, 4, m->stream));
-      return false;
-    }
-  }
   std::vector<int> added;
   for (int c = m->built_views; c < V; ++c)
     if (!m->views[c].retired) added.push_back(c);
@@ -1209,17 +1179,14 @@ bool append_lists(mrf_map* m) {
       if (t.joinable()) t.join();
     }
   } joiner{lists_thread};
-  // loud voxels of every live view: the old views' from their pairs, the
-  // new ones' from the voxel ids of the emit pass
+  // loud voxels: the old views' stay flagged (those of views retired since the
+  // last full build too: a quiet voxel taken for a loud one only costs its
+  // pairs' preparation), the new views add theirs from the emit pass's ids
   const int64_t nvox = m->n_bricks * kBrickVox;
-  m->s_loud.reserve((size_t)std::max<int64_t>(nvox, 1), false, m->stream);
-  CK(cudaMemsetAsync(m->s_loud.p, 0, (size_t)std::max<int64_t>(nvox, 1), m->stream));
-  for (int c = 0; c < m->built_views; ++c) {
-    const View& v = m->views[c];
-    if (v.retired || !v.n_inc) continue;
-    CK(launch_loud_voxels_from_pairs(m->meta.as<RayMeta>() + v.pix_base, view_pixels(v), m->inc_pair.as<uint32_t>(),
-                                     m->pair_vox.as<uint32_t>(), m->s_loud.as<uint8_t>(), m->stream));
-  }
+  m->s_loud.reserve((size_t)std::max<int64_t>(nvox, 1), true, m->stream);
+  if (nvox > m->loud_n)
+    CK(cudaMemsetAsync(m->s_loud.as<uint8_t>() + m->loud_n, 0, (size_t)(nvox - m->loud_n), m->stream));
+  m->loud_n = nvox;
   for (int c : added)
     CK(launch_loud_voxels(m->meta.as<RayMeta>() + m->views[c].pix_base, view_pixels(m->views[c]),
                           m->s_vox.as<uint32_t>(), m->scratch_base, m->s_loud.as<uint8_t>(), m->stream));
@@ -1327,9 +1294,7 @@ bool append_lists(mrf_map* m) {
   m->jacobi_version = -1;
   m->built_views = V;
   m->npix_total = npix;
-  m->bricks_at_build = m->n_bricks;
   stats_from_views(m);
-  return true;
 }
 
 void build_jacobi_csr(mrf_map* m) {
@@ -1407,7 +1372,8 @@ void ensure_built(mrf_map* m) {
         }
       };
       try {
-        done = append_lists(m);
+        append_lists(m);
+        done = true;
       } catch (const Fail& e) {
         abandon();
         // out of memory: the retired views' lists fill it, and the full
@@ -2972,10 +2938,10 @@ mrf_status mrf_stats_get(mrf_map* m, mrf_stats* out) {
     ensure_built(m);
     // pairs past the length gate and the distinct voxels they reach
     const int64_t nvox = m->n_bricks * kBrickVox;
-    m->s_loud.reserve((size_t)std::max<int64_t>(nvox, 1), false, m->stream);
+    m->s_dense.reserve((size_t)std::max<int64_t>(nvox, 1), false, m->stream);
     m->s_delta.reserve(64, false, m->stream);
     CK(launch_touch_counts(m->pair_vox.as<uint32_t>(), m->pair_cum.as<float>(), (uint32_t)m->n_pairs,
-                           m->s_loud.as<uint8_t>(), nvox, m->s_delta.as<unsigned long long>(), m->stream));
+                           m->s_dense.as<uint8_t>(), nvox, m->s_delta.as<unsigned long long>(), m->stream));
     unsigned long long cnt[2] = {0, 0};
     CK(cudaMemcpyAsync(cnt, m->s_delta.p, 16, cudaMemcpyDeviceToHost, m->stream));
     sync(m);

@@ -87,12 +87,9 @@ cudaError_t launch_fill_new_voxels(float* L, float* belief, int64_t v0, int64_t 
 cudaError_t launch_set_points(const Geom& g, const float* pts, const float* occ, int64_t n,
                               float* belief, cudaStream_t s);
 
-// traversal: count pass then emit pass.  With check (the view's stored ray
-// records) the count pass also sets err[1] when any ray's record would
-// differ from the stored one (err holds two ints).
+// traversal: count pass then emit pass
 cudaError_t launch_trace_count(const Geom& g, const Pose& P, const float* depth, uint32_t* counts,
-                               int* err, cudaStream_t s, const RayMeta* check = nullptr,
-                               const uint8_t* only = nullptr, const int* only_all = nullptr);
+                               int* err, cudaStream_t s);
 // pixels of a view whose rays may cross one of the bricks in slots b0..b1
 // (mask[pix] = 1; *all = 1 when every pixel must be checked)
 cudaError_t launch_brick_footprint(const Geom& g, const Pose& P, const int* coord, uint32_t b0, uint32_t b1,
@@ -132,9 +129,6 @@ cudaError_t launch_run_stats(const uint32_t* dpair, const uint32_t* dseg, const 
 // incidence vox_base + k), and the pairs on them
 cudaError_t launch_loud_voxels(const RayMeta* meta, int64_t npix, const uint32_t* vox, uint32_t vox_base,
                                uint8_t* loud, cudaStream_t s);
-// the same with each incidence's voxel from its pair (vox = pair_vox[inc_pair])
-cudaError_t launch_loud_voxels_from_pairs(const RayMeta* meta, int64_t npix, const uint32_t* inc_pair,
-                                          const uint32_t* pair_vox, uint8_t* loud, cudaStream_t s);
 // flag[v] = 1 for the voxels of the given pairs past the length gate (no reset)
 cudaError_t launch_mark_active(const uint32_t* pair_vox, const float* cum, uint32_t np, uint8_t* flag,
                                cudaStream_t s);
