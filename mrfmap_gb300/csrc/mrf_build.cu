@@ -52,8 +52,8 @@ __device__ __forceinline__ void mark_point(const Geom& g, float px, float py, fl
 
 __global__ void k_activate(Geom g, Pose P, const float* __restrict__ depth, int policy,
                            uint8_t* __restrict__ flags) {
-  int pix = blockIdx.x * blockDim.x + threadIdx.x;
-  if (pix >= g.rows * g.cols) return;
+  const int pix = tile_pixel(g.rows, g.cols, (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5, threadIdx.x & 31);
+  if (pix < 0) return;
   float d = depth[pix];
   if (!(d > 0.0f)) return;
   int x = pix % g.cols, y = pix / g.cols;
@@ -77,24 +77,17 @@ __global__ void k_activate(Geom g, Pose P, const float* __restrict__ depth, int 
     // s + bias(s) > d + 3 sigma(s)).  The trace then meets only bricks its
     // own view activated before its stop, so bricks other views activate
     // later never change this view's lists.
-    const float* sg = lut_at(g, g.sigma, x, y);
-    const float* bs = lut_at(g, g.bias, x, y);
-    const int n = g.lookup_n;
+    const Sensor c = sensor_at(g, x, y);
     Ray ray;
     ray_setup(g, P, x, y, ray);
     Dda r;
     if (dda_init(r, g, ray)) {
-      int vx, vy, vz;
-      float l, tin, te, s_last = 0.0f;
-      int64_t cur = -1;
-      while (dda_next(r, g, vx, vy, vz, l, tin, te)) {
-        int64_t lin = brick_lin(g, vx, vy, vz);
-        if (lin != cur) {
-          if (cur >= 0 && fa(s_last, poly_f(bs, n, s_last)) > fa(d, fm(3.0f, poly_f(sg, n, s_last)))) break;
-          flags[lin] = 1;
-          cur = lin;
-        }
-        s_last = fm(te, ray.mult);
+      float s_last = 0.0f;
+      for (bool first = true; r.alive && r.guard > 0; first = false) {
+        if (!first && fa(s_last, c.bias(s_last)) > fa(d, fm(3.0f, c.sigma(s_last)))) break;
+        flags[r.lin] = 1;
+        int steps;
+        s_last = fm(dda_cross(r, g, ray, steps), ray.mult);
       }
     }
   }
@@ -156,130 +149,169 @@ __global__ void k_set_points(Geom g, const float* __restrict__ pts, const float*
   belief[(int64_t)s * kBrickVox + voxel_local(vx, vy, vz)] = occ[i];
 }
 
-// One thread per pixel walks the DDA through the active bricks.  Runs of
-// voxels in one brick end with the reference's per-brick stop tests; the
-// count pass and the emit pass execute the identical loop.  The emit pass
-// keeps the last four incidences in registers (a shift register) and
-// stores each aligned group of four as 16-byte vectors: ray offsets are
-// multiples of four, so a ray's lists start on a group boundary, and the
-// last group is completed with padding.
-template <bool EMIT>
-__global__ void __launch_bounds__(kThreads, 4)
-    k_trace(Geom g, Pose P, const float* __restrict__ depth, uint32_t* __restrict__ counts,
-            const uint32_t* __restrict__ pix_off, uint32_t inc_base, RayMeta* __restrict__ meta,
-            uint32_t* __restrict__ inc_vox, float* __restrict__ inc_len,
-            float* __restrict__ inc_mu, int* __restrict__ err) {
-  int pix = blockIdx.x * blockDim.x + threadIdx.x;
-  if (pix >= g.rows * g.cols) return;
-  float d = depth[pix];
-  int count = 0, n_pre = -1, n_post = -1, r0 = -1, run_start = 0, kmu = -1;
-  bool gate = false;
-  uint32_t base = EMIT ? pix_off[pix] : 0;
-  uint32_t bv[4] = {kNoVoxel, kNoVoxel, kNoVoxel, kNoVoxel};
-  float bl[4] = {0.0f, 0.0f, 0.0f, 0.0f}, bm[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-  // shift one incidence into the group; store the group when it is whole
-  auto push = [&](uint32_t v, float len, float mu) {
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      bv[j] = bv[j + 1];
-      bl[j] = bl[j + 1];
-      bm[j] = bm[j + 1];
-    }
-    bv[3] = v;
-    bl[3] = len;
-    bm[3] = mu;
-  };
-  auto store = [&](uint32_t k0) {
-    *reinterpret_cast<uint4*>(inc_vox + k0) = make_uint4(bv[0], bv[1], bv[2], bv[3]);
-    *reinterpret_cast<float4*>(inc_len + k0) = make_float4(bl[0], bl[1], bl[2], bl[3]);
-    *reinterpret_cast<float4*>(inc_mu + k0) = make_float4(bm[0], bm[1], bm[2], bm[3]);
-  };
+// Incidences of each pixel's Pre pass, padded to a multiple of 4 (the emit
+// pass's offsets): the voxels the ray crosses in active bricks up to the
+// brick run whose end is past the return, counted brick by brick.
+__global__ void __launch_bounds__(128)
+    k_trace_count(Geom g, Pose P, const float* __restrict__ depth, uint32_t* __restrict__ counts,
+                  int* __restrict__ err) {
+  const int pix = tile_pixel(g.rows, g.cols, (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5, threadIdx.x & 31);
+  if (pix < 0) return;
+  const float d = depth[pix];
+  int count = 0;
   if (d > 0.0f) {
-    int x = pix % g.cols, y = pix / g.cols;
-    const float* sg = lut_at(g, g.sigma, x, y);
-    const float* bs = lut_at(g, g.bias, x, y);
-    const int n = g.lookup_n;
+    const int x = pix % g.cols, y = pix / g.cols;
+    const Sensor c = sensor_at(g, x, y);
     Ray ray;
     ray_setup(g, P, x, y, ray);
     Dda r;
     if (dda_init(r, g, ray)) {
-      int64_t cur = -1;
-      int slot = -1;
-      bool run_open = false;
-      float s_last = 0.0f;
-      int vx, vy, vz;
-      float l, tin, te;
-      while (dda_next(r, g, vx, vy, vz, l, tin, te)) {
-        int64_t lin = brick_lin(g, vx, vy, vz);
-        if (lin != cur) {
-          if (run_open) {
-            run_open = false;
-            float lhs = fa(s_last, poly_f(bs, n, s_last));
-            float rhs = fa(d, fm(3.0f, poly_f(sg, n, s_last)));
-            if (n_post < 0 && lhs >= rhs) n_post = count;
-            if (lhs > rhs) {
-              n_pre = count;
-              break;
-            }
-          }
-          cur = lin;
-          slot = g.brick_slot[lin];
-        }
+      while (r.alive && r.guard > 0) {
+        const int slot = g.brick_slot[r.lin];
+        int steps;
+        const float s = fm(dda_cross(r, g, ray, steps), ray.mult);
         if (slot < 0) continue;
-        if (count >= kMaxRayLen) {
+        if (count + steps > kMaxRayLen) {
           atomicOr(err, 1);
+          count = kMaxRayLen;
           break;
         }
-        float s = fm(te, ray.mult);
-        if (!run_open) run_start = count;
-        if (EMIT) {
-          const bool z = potential_is_zero(sg, bs, n, s, d);
-          const float mu = z ? 0.0f : potential(sg, bs, n, s, d);
-          if (r0 < 0 && !z) r0 = run_start;
-          if (kmu < 0 && !z) kmu = count;
-          push((uint32_t)slot * kBrickVox + voxel_local(vx, vy, vz), l, mu);
-          if ((count & 3) == 3) store(base + (uint32_t)(count - 3));
-        }
-        run_open = true;
-        s_last = s;
-        ++count;
+        count += steps;
+        if (fa(s, c.bias(s)) > fa(d, fm(3.0f, c.sigma(s)))) break;
       }
-      if (n_pre < 0 && run_open) {
-        float lhs = fa(s_last, poly_f(bs, n, s_last));
-        float rhs = fa(d, fm(3.0f, poly_f(sg, n, s_last)));
+    }
+  }
+  counts[pix] = (uint32_t)((count + 3) & ~3);
+}
+
+// One thread per pixel walks the DDA through the active bricks.  Runs of
+// voxels in one brick end with the reference's per-brick stop tests.  A
+// thread's last incidences wait in shared memory (its own column) and go out
+// eight at a time, as two 16-byte stores per list: single incidences, or
+// groups of four in registers, leave half-written sectors behind that L2
+// reads and writes twice.  A ray's lists start on a multiple of four; the last
+// group is completed with padding.  A list that does not fill the room its
+// count gave it raises the error flag.
+constexpr int kEmitThreads = 128;
+constexpr int kEmitStride = 12;  // words of a thread's eight in each list: 16-byte loads, four ways to a bank
+
+__global__ void __launch_bounds__(kEmitThreads, 6)
+    k_trace_emit(Geom g, Pose P, const float* __restrict__ depth, const uint32_t* __restrict__ pix_off,
+                 uint32_t inc_base, RayMeta* __restrict__ meta, uint32_t* __restrict__ inc_vox,
+                 float* __restrict__ inc_len, float* __restrict__ inc_mu, int* __restrict__ err) {
+  const int pix = tile_pixel(g.rows, g.cols, (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5, threadIdx.x & 31);
+  __shared__ __align__(16) uint32_t pending[3][kEmitThreads * kEmitStride];
+  if (pix < 0) return;
+  const float d = depth[pix];
+  int count = 0, n_pre = -1, n_post = -1, r0 = -1, run_start = 0, kmu = -1;
+  bool gate = false;
+  const uint32_t base = pix_off[pix];
+  const int room = (int)(pix_off[pix + 1] - base);
+  // the group of eight incidence k belongs to, counted in the arena so that
+  // whole groups are whole sectors; the ray's first may be a half
+  const uint32_t mine = threadIdx.x * kEmitStride;
+  const uint32_t phase = (inc_base + base) & 7u;
+  auto push = [&](uint32_t k, uint32_t v, float len, float mu) {
+    const uint32_t a = mine + ((phase + k) & 7u);
+    pending[0][a] = v;
+    pending[1][a] = __float_as_uint(len);
+    pending[2][a] = __float_as_uint(mu);
+  };
+  // half h of the group goes to incidences first .. first + 3
+  auto store = [&](uint32_t first, uint32_t h) {
+    const uint32_t a = mine + 4 * h;
+    *reinterpret_cast<uint4*>(inc_vox + first) = *reinterpret_cast<const uint4*>(pending[0] + a);
+    *reinterpret_cast<uint4*>(inc_len + first) = *reinterpret_cast<const uint4*>(pending[1] + a);
+    *reinterpret_cast<uint4*>(inc_mu + first) = *reinterpret_cast<const uint4*>(pending[2] + a);
+  };
+  auto flush = [&](uint32_t k) {
+    // k completes its group of eight: both halves, unless the ray began in
+    // the second one
+    const uint32_t end = base + k + 1;
+    if (k + 1 >= 8) store(end - 8, 0);
+    store(end - 4, 1);
+  };
+  if (d > 0.0f) {
+    const int x = pix % g.cols, y = pix / g.cols;
+    const Sensor c = sensor_at(g, x, y);
+    Ray ray;
+    ray_setup(g, P, x, y, ray);
+    Dda r;
+    if (dda_init(r, g, ray)) {
+      bool run_open = false;
+      float s_last = 0.0f;
+      // no potential before it: 13.3 sigma' with room for rounding
+      const float s_first = window_start(c, d, 40.0f, 0.999f);
+      // the run that ends here: the stop tests
+      auto stop = [&]() {
+        const float lhs = fa(s_last, c.bias(s_last));
+        const float rhs = fa(d, fm(3.0f, c.sigma(s_last)));
         if (n_post < 0 && lhs >= rhs) n_post = count;
         if (lhs > rhs) n_pre = count;
+        return lhs > rhs;
+      };
+      while (r.alive && r.guard > 0) {
+        if (run_open && stop()) break;
+        run_open = false;
+        const int slot = g.brick_slot[r.lin];
+        if (slot < 0) {
+          int steps;
+          dda_cross(r, g, ray, steps);
+          continue;
+        }
+        run_start = count;
+        run_open = true;
+        // the brick's voxels: neighbouring rays enter and leave it nearly
+        // together, so the lanes that are done wait a step or two here
+        // rather than entering their next brick on their own
+        bool left;
+        do {
+          if (count >= room) {
+            atomicOr(err, 2);
+            r.alive = false;
+            break;
+          }
+          const uint32_t v = (uint32_t)slot * kBrickVox + dda_local(r);
+          float l, tin, te;
+          left = dda_step(r, g, l, tin, te);
+          s_last = fm(te, ray.mult);
+          float mu = 0.0f;
+          if (s_last >= s_first && !potential_is_zero(c, s_last, d)) {
+            mu = potential(c, s_last, d);
+            if (r0 < 0) r0 = run_start;
+            if (kmu < 0) kmu = count;
+          }
+          push((uint32_t)count, v, l, mu);
+          if (((phase + count) & 7) == 7) flush((uint32_t)count);
+          ++count;
+        } while (!left && r.guard > 0);
       }
+      if (n_pre < 0 && run_open) stop();
       if (n_pre < 0) {
         n_pre = count;
-        if (count > 0) gate = d > fa(s_last, poly_f(bs, n, s_last));
+        if (count > 0) gate = d > fa(s_last, c.bias(s_last));
       }
     }
   }
   if (n_pre < 0) n_pre = count;
   if (n_post < 0) n_post = count;
-  // each ray's list is padded to a multiple of 4 incidences (16-byte vector
-  // loads in the BP kernels); padding carries an invalid voxel id
+  // the last group, completed with padding (invalid voxel, zeros; 16-byte
+  // vector loads in the BP kernels)
   const int padded = (n_pre + 3) & ~3;
-  if (!EMIT) {
-    counts[pix] = (uint32_t)padded;
-  } else {
-    // the last group, completed with padding (invalid voxel, zeros)
-    if (count & 3) {
-      const int k0 = count & ~3;
-      for (int k = count; k < padded; ++k) push(kNoVoxel, 0.0f, 0.0f);
-      store(base + (uint32_t)k0);
-    }
-    const int kdyn = (kmu >= 0 && kmu < n_post) ? kmu : n_post;
-    RayMeta m;
-    m.off = inc_base + base;
-    m.n_pre = (uint16_t)n_pre;
-    m.n_post = (uint16_t)n_post;
-    m.r0 = (uint16_t)(r0 >= 0 ? r0 : n_pre);
-    m.rinf = (uint16_t)(r0 >= 0 ? r0 : run_start);
-    m.flags = (gate ? 1u : 0u) | ((uint32_t)kdyn << 16);
-    meta[pix] = m;
-  }
+  for (int k = count; k < padded; ++k) push((uint32_t)k, kNoVoxel, 0.0f, 0.0f);
+  const uint32_t left = padded ? (phase + (uint32_t)padded) & 7u : 0u;  // in the last, unfinished group of eight
+  if (count < padded && left == 0) flush((uint32_t)padded - 1u);
+  if (left == 4) store(base + (uint32_t)padded - 4u, 0);
+  if (padded != room) atomicOr(err, 2);
+  const int kdyn = (kmu >= 0 && kmu < n_post) ? kmu : n_post;
+  RayMeta m;
+  m.off = inc_base + base;
+  m.n_pre = (uint16_t)n_pre;
+  m.n_post = (uint16_t)n_post;
+  m.r0 = (uint16_t)(r0 >= 0 ? r0 : n_pre);
+  m.rinf = (uint16_t)(r0 >= 0 ? r0 : run_start);
+  m.flags = (gate ? 1u : 0u) | ((uint32_t)kdyn << 16);
+  meta[pix] = m;
 }
 
 // Pairs.  A pair is a (camera, voxel) with at least one incidence.  The pairs
@@ -687,7 +719,7 @@ cudaError_t launch_clean_depth(const float* in, float* out, int rows, int cols, 
 
 cudaError_t launch_activate(const Geom& g, const Pose& P, const float* depth, int policy,
                             uint8_t* flags, cudaStream_t s) {
-  k_activate<<<grid_for((int64_t)g.rows * g.cols, 128), 128, 0, s>>>(g, P, depth, policy, flags);
+  k_activate<<<grid_for(pixel_tiles(g.rows, g.cols) * 32, 128), 128, 0, s>>>(g, P, depth, policy, flags);
   return cudaGetLastError();
 }
 
@@ -724,10 +756,9 @@ cudaError_t launch_set_points(const Geom& g, const float* pts, const float* occ,
   return cudaGetLastError();
 }
 
-cudaError_t launch_trace_count(const Geom& g, const Pose& P, const float* depth, uint32_t* counts,
-                               int* err, cudaStream_t s) {
-  k_trace<false><<<grid_for((int64_t)g.rows * g.cols), kThreads, 0, s>>>(
-      g, P, depth, counts, nullptr, 0, nullptr, nullptr, nullptr, nullptr, err);
+cudaError_t launch_trace_count(const Geom& g, const Pose& P, const float* depth, uint32_t* counts, int* err,
+                               cudaStream_t s) {
+  k_trace_count<<<grid_for(pixel_tiles(g.rows, g.cols) * 32, 128), 128, 0, s>>>(g, P, depth, counts, err);
   return cudaGetLastError();
 }
 
@@ -788,8 +819,8 @@ cudaError_t launch_brick_footprint(const Geom& g, const Pose& P, const int* coor
 cudaError_t launch_trace_emit(const Geom& g, const Pose& P, const float* depth,
                               const uint32_t* pix_off, uint32_t inc_base, RayMeta* meta,
                               uint32_t* inc_vox, float* inc_len, float* inc_mu, int* err, cudaStream_t s) {
-  k_trace<true><<<grid_for((int64_t)g.rows * g.cols), kThreads, 0, s>>>(
-      g, P, depth, nullptr, pix_off, inc_base, meta, inc_vox, inc_len, inc_mu, err);
+  k_trace_emit<<<grid_for(pixel_tiles(g.rows, g.cols) * 32, kEmitThreads), kEmitThreads, 0, s>>>(
+      g, P, depth, pix_off, inc_base, meta, inc_vox, inc_len, inc_mu, err);
   return cudaGetLastError();
 }
 

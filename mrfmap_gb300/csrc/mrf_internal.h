@@ -72,6 +72,9 @@ __host__ __device__ __forceinline__ bool ray_in_bp(const RayMeta& m) {
 constexpr int kMaxRayLen = 65532;        // n_pre fits uint16 after padding to 4
 constexpr uint32_t kNoVoxel = 0xFFFFFFFFu;  // padding incidences
 
+// tiles of a rows x cols image in the traversal kernels (a warp each)
+__host__ __device__ inline int64_t pixel_tiles(int rows, int cols) { return (int64_t)((cols + 7) / 8) * ((rows + 3) / 4); }
+
 // ---- launchers (stream-ordered; return cudaError_t of the launch) --------
 cudaError_t launch_clean_depth(const float* in, float* out, int rows, int cols, cudaStream_t s);
 cudaError_t launch_activate(const Geom& g, const Pose& P, const float* depth, int policy,
@@ -87,9 +90,10 @@ cudaError_t launch_fill_new_voxels(float* L, float* belief, int64_t v0, int64_t 
 cudaError_t launch_set_points(const Geom& g, const float* pts, const float* occ, int64_t n,
                               float* belief, cudaStream_t s);
 
-// traversal: count pass then emit pass
-cudaError_t launch_trace_count(const Geom& g, const Pose& P, const float* depth, uint32_t* counts,
-                               int* err, cudaStream_t s);
+// traversal: count pass (counts padded to multiples of 4), then emit pass
+// (pix_off: their exclusive scan and total)
+cudaError_t launch_trace_count(const Geom& g, const Pose& P, const float* depth, uint32_t* counts, int* err,
+                               cudaStream_t s);
 // pixels of a view whose rays may cross one of the bricks in slots b0..b1
 // (mask[pix] = 1; *all = 1 when every pixel must be checked)
 cudaError_t launch_brick_footprint(const Geom& g, const Pose& P, const int* coord, uint32_t b0, uint32_t b1,

@@ -11,13 +11,13 @@ namespace {
 
 constexpr int kLikeThreads = 128;
 
-// One thread per pixel (per-pixel body in mrf_like_pixel.cuh).
+// A warp per tile of pixels (per-pixel body in mrf_like_pixel.cuh).
 __global__ void __launch_bounds__(kLikeThreads)
     k_likelihood(Geom g, Pose P, const float* __restrict__ depth, const float* __restrict__ belief,
                  float* __restrict__ out_img, double* __restrict__ partials) {
-  int pix = blockIdx.x * blockDim.x + threadIdx.x;
+  const int pix = tile_pixel(g.rows, g.cols, (blockIdx.x * (int64_t)kLikeThreads + threadIdx.x) >> 5, threadIdx.x & 31);
   float val = 0.0f;
-  if (pix < g.rows * g.cols) {
+  if (pix >= 0) {
     float d = depth[pix];
     if (d > 0.0f) val = likelihood_pixel(g, P, belief, pix, d);
     if (out_img) out_img[pix] = val;
@@ -43,7 +43,8 @@ __global__ void k_reduce_partials(const double* __restrict__ partials, int n, fl
 }  // namespace
 
 int likelihood_blocks(const Geom& g) {
-  return (g.rows * g.cols + kLikeThreads - 1) / kLikeThreads;
+  constexpr int kTiles = kLikeThreads / 32;
+  return (int)((pixel_tiles(g.rows, g.cols) + kTiles - 1) / kTiles);
 }
 
 cudaError_t launch_likelihood(const Geom& g, const Pose& P, const float* depth, const float* belief,

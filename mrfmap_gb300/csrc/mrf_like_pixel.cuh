@@ -2,74 +2,90 @@
 // belief field (src/cuda/gvdbkernels.cu:183-293, 1246-1274).  Visibility
 // V = exp(-sum alpha l) with alpha = -ln(1 - p); each voxel adds
 // (V_prev - V) * P(z | first return in the voxel); the tail adds
-// V_end * P(z | no return).  No early stop: every active brick to the volume
-// exit is visited.
+// V_end * P(z | no return).  Every active brick to the volume exit counts.
+//
+// P is LIKE_EPS at every voxel outside the return's window, so their sum is
+// LIKE_EPS times the visibility lost there: V at the near limit, minus V at
+// the end, minus what the window took.  Outside the window a voxel then
+// costs its exponent only -- ln(1 - p) by its series for the small p of free
+// space -- and two exponentials inside it.  Inactive bricks are left in one
+// go.  A ray whose visibility is below 1e-30 while the sum is above 1e-18
+// ends: the rest cannot change the FP32 result.
 #pragma once
 #include "mrf_geometry.cuh"
 #include "mrf_internal.h"
 
 namespace mrf {
 
+// ln(1 - p): the Taylor series to p^5 below 1/64 (next term p^6/6: relative
+// 1.6e-10), CUDA's log1pf above
+__device__ __forceinline__ float log_free(float p) {
+  if (!(fabsf(p) <= 0.015625f)) return log1pf(-p);
+  return -p * (1.0f + p * (0.5f + p * (1.0f / 3.0f + p * (0.25f + p * 0.2f))));
+}
+
 __device__ __forceinline__ float likelihood_pixel(const Geom& g, const Pose& P,
                                                   const float* __restrict__ belief, int pix, float d) {
-  int x = pix % g.cols, y = pix / g.cols;
-  const float* sg = lut_at(g, g.sigma, x, y);
-  const float* bs = lut_at(g, g.bias, x, y);
-  const int n = g.lookup_n;
+  const int x = pix % g.cols, y = pix / g.cols;
+  const Sensor c = sensor_at(g, x, y);
   Ray ray;
   ray_setup(g, P, x, y, ray);
-  float A = 0.0f, Vprev = 1.0f, sum = 0.0f, prev_s = 0.0f, s_last = 0.0f;
-  bool first_run = true, run_open = false;
+  // A: exponent of the visibility; Vz: visibility at the near limit; inside
+  // the window: sum of w and of w P
+  float A = 0.0f, Vz = 1.0f, win_w = 0.0f, win = 0.0f, prev_s = 0.0f, s_last = 0.0f;
+  bool first_run = true, run_open = false, near = true;
+  const float s_win = window_start(c, d, 3.0f, 0.9999f);  // the window begins behind it
   Dda r;
   if (dda_init(r, g, ray)) {
-    int64_t cur = -1;
-    int slot = -1;
-    int vx, vy, vz;
-    float l, tin, te;
-    while (dda_next(r, g, vx, vy, vz, l, tin, te)) {
-      int64_t lin = brick_lin(g, vx, vy, vz);
-      if (lin != cur) {
-        if (run_open) {
-          run_open = false;
-          // a brick hands s + bias(s) to the next as its previous s
-          // (gvdbkernels.cu:209, 292)
-          prev_s = s_last + poly_f(bs, n, s_last);
-        }
-        cur = lin;
-        slot = g.brick_slot[lin];
-      }
-      if (slot < 0) continue;
-      if (!run_open) {
-        run_open = true;
-        if (first_run) {
-          prev_s = fm(tin, ray.mult);
-          first_run = false;
+    while (r.alive && r.guard > 0) {
+      // a brick hands s + bias(s) to the next as its previous s
+      // (gvdbkernels.cu:209, 292)
+      if (run_open) {
+        prev_s = s_last + c.bias(s_last);
+        run_open = false;
+        if (A < -69.0f && !near) {
+          const float V = expf(A);
+          if (kLikeEps * (Vz - V - win_w) + win > 1e-18f) break;
         }
       }
-      float p = belief[(int64_t)slot * kBrickVox + voxel_local(vx, vy, vz)];
-      float alpha = -log1pf(-p);
-      float dA = -alpha * l;
-      A += dA;
-      float V = expf(A);
-      float w = Vprev * -expm1f(dA);
-      float s = fm(te, ray.mult);
-      float Pz;
-      if (s < kZMin) {
-        Pz = 0.0f;
-      } else {
-        float pd = fs(fa(s, poly_f(bs, n, s)), d);
-        if (fabsf(pd) <= fm(3.0f, poly_f(sg, n, s)))
-          Pz = (1.0f - kLikeEps) * 0.5f * (potential(sg, bs, n, s, d) + potential(sg, bs, n, prev_s, d));
-        else
-          Pz = kLikeEps;
+      const int slot = g.brick_slot[r.lin];
+      if (slot < 0) {
+        int steps;
+        dda_cross(r, g, ray, steps);
+        continue;
       }
-      sum += w * Pz;
-      Vprev = V;
-      prev_s = s;
-      s_last = s;
+      if (first_run) {
+        prev_s = fm(r.tprev, ray.mult);
+        first_run = false;
+      }
+      run_open = true;
+      const float* __restrict__ bel = belief + (int64_t)slot * kBrickVox;
+      // the brick's voxels, the lanes of a warp together
+      bool left;
+      do {
+        const float p = bel[dda_local(r)];
+        float l, tin, te;
+        left = dda_step(r, g, l, tin, te);
+        const float dA = log_free(p) * l;
+        const float s = fm(te, ray.mult);
+        if (near && !(s < kZMin)) {
+          Vz = expf(A);
+          near = false;
+        }
+        if (s >= s_win && !near && fabsf(fs(fa(s, c.bias(s)), d)) <= fm(3.0f, c.sigma(s))) {
+          const float w = expf(A) * -expm1f(dA);
+          win_w += w;
+          win += w * ((1.0f - kLikeEps) * 0.5f * (potential(c, s, d) + potential(c, prev_s, d)));
+        }
+        A += dA;
+        prev_s = s;
+      } while (!left && r.guard > 0);
+      s_last = prev_s;
     }
   }
-  sum += Vprev * (d >= kZMax ? 1.0f - kLikeEps : kLikeEps);
+  const float V = expf(A);
+  if (near) Vz = V;
+  const float sum = kLikeEps * (Vz - V - win_w) + win + V * (d >= kZMax ? 1.0f - kLikeEps : kLikeEps);
   return logf(sum);
 }
 

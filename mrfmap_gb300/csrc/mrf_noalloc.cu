@@ -12,9 +12,10 @@
 //
 // Limits and sharing:
 //  * scratch: kNoAllocMaxBlocks FP64 partials (32 KiB, held by every GPU
-//    that loads the library until the process exits), one per 128 pixels:
-//    images up to kNoAllocMaxBlocks * 128 = 524,288 pixels (640x480 and
-//    848x480 fit).  Larger images are rejected with MRF_ERR_INVALID.
+//    that loads the library until the process exits), one per block; images up
+//    to kNoAllocMaxBlocks * 128 = 524,288 pixels (640x480 and 848x480 fit),
+//    larger ones are rejected with MRF_ERR_INVALID.  (Narrow images have tiles
+//    of fewer pixels than a warp has lanes; a block then takes several.)
 //  * every call shares the array; each call overwrites the partials it uses
 //    before reading them, so nothing has to start at zero.  Calls that
 //    overlap on the GPU (two streams, or two maps on one device) race on the
@@ -29,6 +30,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <mutex>
 #include <string>
 
@@ -90,14 +92,18 @@ __global__ void __launch_bounds__(kNoAllocThreads)
     k_likelihood_noalloc(Geom g, Pose P, const float* __restrict__ depth,
                          const float* __restrict__ belief, float* __restrict__ out_img,
                          double* __restrict__ partials) {
-  int pix = blockIdx.x * blockDim.x + threadIdx.x;
-  float val = 0.0f;
-  if (pix < g.rows * g.cols) {
+  const int64_t tiles = pixel_tiles(g.rows, g.cols);
+  double sum = 0.0;
+  for (int64_t tile = (blockIdx.x * (int64_t)kNoAllocThreads + threadIdx.x) >> 5; tile < tiles;
+       tile += gridDim.x * (int64_t)(kNoAllocThreads / 32)) {
+    const int pix = tile_pixel(g.rows, g.cols, tile, threadIdx.x & 31);
+    if (pix < 0) continue;
     const float d = clean_depth_value(depth[pix], pix, g.rows, g.cols);
-    if (d > 0.0f) val = likelihood_pixel(g, P, belief, pix, d);
+    const float val = d > 0.0f ? likelihood_pixel(g, P, belief, pix, d) : 0.0f;
     if (out_img) out_img[pix] = val;
+    sum += (double)val;
   }
-  double t = like_block_sum<kNoAllocThreads>((double)val);
+  double t = like_block_sum<kNoAllocThreads>(sum);
   if (threadIdx.x == 0) partials[blockIdx.x] = t;
 }
 
@@ -119,9 +125,11 @@ extern "C" MRF_API mrf_status mrf_likelihood_device_noalloc(mrf_map* map, const 
   }
   mrf_status st = mrf_internal_like_inputs(map, &g, &belief, &stream, &device);
   if (st != MRF_OK) return st;
-  int64_t npix = (int64_t)g.rows * g.cols;
-  int64_t nblocks = (npix + kNoAllocThreads - 1) / kNoAllocThreads;
-  if (nblocks > kNoAllocMaxBlocks) {
+  const int64_t npix = (int64_t)g.rows * g.cols;
+  constexpr int kTiles = kNoAllocThreads / 32;
+  const int64_t nblocks =
+      std::min<int64_t>((pixel_tiles(g.rows, g.cols) + kTiles - 1) / kTiles, kNoAllocMaxBlocks);
+  if (npix > (int64_t)kNoAllocMaxBlocks * kNoAllocThreads) {
     mrf_internal_set_error(
         "mrf_likelihood_device_noalloc: image larger than 524288 pixels (fixed scratch limit)");
     return MRF_ERR_INVALID;

@@ -11,6 +11,7 @@
 // src/cuda/gvdbhelper.cu:16-62 (integer counts: order-independent).
 #include "mrf_geometry.cuh"
 #include "mrf_internal.h"
+#include "mrf_like_pixel.cuh"
 
 namespace mrf {
 
@@ -21,10 +22,8 @@ constexpr int kRenderThreads = 128;
 template <int kMode>
 __device__ float render_pixel(const Geom& g, const Pose& P, const float* __restrict__ belief, int pix,
                               float d, float thresh) {
-  int x = pix % g.cols, y = pix / g.cols;
-  const float* sg = lut_at(g, g.sigma, x, y);
-  const float* bs = lut_at(g, g.bias, x, y);
-  const int n = g.lookup_n;
+  const int x = pix % g.cols, y = pix / g.cols;
+  const Sensor c = sensor_at(g, x, y);
   Ray ray;
   ray_setup(g, P, x, y, ray);
   float A = 0.0f, Vprev = 1.0f, sum = 0.0f, peak = 0.0f, s_last = 0.0f;
@@ -32,54 +31,69 @@ __device__ float render_pixel(const Geom& g, const Pose& P, const float* __restr
   bool run_open = false;
   Dda r;
   if (dda_init(r, g, ray)) {
-    int64_t cur = -1;
-    int slot = -1;
-    int vx, vy, vz;
-    float l, tin, te;
-    while (dda_next(r, g, vx, vy, vz, l, tin, te)) {
-      int64_t lin = brick_lin(g, vx, vy, vz);
-      if (lin != cur) {
-        // simple accuracy: a brick that ends past the return is a miss
-        if (kMode == 2 && run_open && s_last >= d) return 0.0f;
-        run_open = false;
-        cur = lin;
-        slot = g.brick_slot[lin];
-      }
-      if (slot < 0) continue;
-      run_open = true;
-      float p = belief[(int64_t)slot * kBrickVox + voxel_local(vx, vy, vz)];
-      float s = fm(te, ray.mult);
-      s_last = s;
-      if (kMode == 2) {
-        if (p >= thresh) return fabsf(s - d) <= g.res ? 1.0f : 2.0f;
+    while (r.alive && r.guard > 0) {
+      // simple accuracy: a brick that ends past the return is a miss
+      if (kMode == 2 && run_open && s_last >= d) return 0.0f;
+      // expected depth: nothing visible is left, the rest cannot change the
+      // FP32 sum
+      if (kMode == 0 && Vprev < 1e-30f && sum > 1e-18f) break;
+      // the label is known
+      if (kMode == 3 && occ != -1) break;
+      run_open = false;
+      const int slot = g.brick_slot[r.lin];
+      if (slot < 0) {
+        int steps;
+        dda_cross(r, g, ray, steps);
         continue;
       }
-      float dA = log1pf(-p) * l;
-      A += dA;
-      float V = expf(A);
-      float dv = Vprev * -expm1f(dA);
-      if (kMode == 0) {
-        // z-depth of the voxel's corner (the GVDB atlas-to-world position)
-        float zc = fabsf(P.m[2] * ((float)vx - ray.o[0]) + P.m[6] * ((float)vy - ray.o[1]) +
-                         P.m[10] * ((float)vz - ray.o[2])) * g.res;
-        sum += dv * zc;
-      } else {
-        float pd = fs(fa(s, poly_f(bs, n, s)), d);
+      run_open = true;
+      const float* __restrict__ bel = belief + (int64_t)slot * kBrickVox;
+      // the brick's voxels, the lanes of a warp together
+      bool left;
+      do {
+        const uint32_t xyz = r.loc;
+        const float p = bel[dda_local(r)];
+        float l, tin, te;
+        const int kx = r.kx, ky = r.ky, kz = r.kz;
+        left = dda_step(r, g, l, tin, te);
+        const float s = fm(te, ray.mult);
+        s_last = s;
+        if (kMode == 2) {
+          if (p >= thresh) return fabsf(s - d) <= g.res ? 1.0f : 2.0f;
+        }
+        if (kMode == 3) {
+          if (fs(fa(s, c.bias(s)), d) > 0.0f && occ == -1) occ = p >= thresh ? 1 : 0;
+        }
+        if (kMode == 0 && p != 0.0f) {
+          const float dA = log_free(p) * l;
+          const float dv = Vprev * -expm1f(dA);
+          A += dA;
+          Vprev = expf(A);
+          // z-depth of the voxel's corner (the GVDB atlas-to-world position)
+          const float vx = (float)(8 * kx + (int)(xyz >> 8)), vy = (float)(8 * ky + (int)(xyz >> 4 & 7)),
+                      vz = (float)(8 * kz + (int)(xyz & 7));
+          const float zc = fabsf(P.m[2] * (vx - ray.o[0]) + P.m[6] * (vy - ray.o[1]) + P.m[10] * (vz - ray.o[2])) *
+                           g.res;
+          sum += dv * zc;
+        }
         if (kMode == 1) {
-          float w = dv / l;
+          const float dA = log1pf(-p) * l;
+          A += dA;
+          const float V = expf(A);
+          const float dv = Vprev * -expm1f(dA);
+          const float w = dv / l;
           if (w > peak) {
             peak = w;
-            peak_ok = fabsf(pd) <= poly_f(sg, n, s);
+            peak_ok = fabsf(fs(fa(s, c.bias(s)), d)) <= c.sigma(s);
           }
+          Vprev = V;
         }
-        if (kMode == 3 && pd > 0.0f && occ == -1) occ = p >= thresh ? 1 : 0;
-      }
-      Vprev = V;
+      } while (!left && r.guard > 0);
     }
   }
   if (kMode == 0) return sum / (1.0f - Vprev + kFEps);
   if (kMode == 1) {
-    if (peak > 0.0f && Vprev >= 0.9f) return fa(s_last, poly_f(bs, n, s_last)) <= d ? -1.0f : 0.0f;
+    if (peak > 0.0f && Vprev >= 0.9f) return fa(s_last, c.bias(s_last)) <= d ? -1.0f : 0.0f;
     if (peak > 0.0f) return (float)peak_ok;
     return -1.0f;
   }
@@ -94,8 +108,9 @@ __global__ void __launch_bounds__(kRenderThreads)
   __shared__ unsigned int hist[4];
   if (threadIdx.x < 4) hist[threadIdx.x] = 0;
   __syncthreads();
-  int pix = blockIdx.x * blockDim.x + threadIdx.x;
-  if (pix < g.rows * g.cols) {
+  const int pix =
+      tile_pixel(g.rows, g.cols, (blockIdx.x * (int64_t)kRenderThreads + threadIdx.x) >> 5, threadIdx.x & 31);
+  if (pix >= 0) {
     float d = depth[pix];
     float v;
     if (kMode != 0 && !(d > 0.0f)) v = -1.0f;
@@ -128,19 +143,22 @@ __global__ void k_pixel_diag(Geom g, Pose P, const float* __restrict__ belief, i
   float A = 0.0f, Vprev = 1.0f;
   Dda r;
   if (dda_init(r, g, ray)) {
-    int64_t cur = -1;
+    bool enter = true;
     int slot = -1;
-    int vx, vy, vz;
-    float l, tin, te;
-    while (dda_next(r, g, vx, vy, vz, l, tin, te)) {
-      int64_t lin = brick_lin(g, vx, vy, vz);
-      if (lin != cur) {
-        cur = lin;
-        slot = g.brick_slot[lin];
+    while (r.alive && r.guard > 0) {
+      if (enter) {
+        slot = g.brick_slot[r.lin];
+        if (slot < 0) {
+          int steps;
+          dda_cross(r, g, ray, steps);
+          continue;
+        }
       }
-      if (slot < 0) continue;
       if (count >= cap) break;
-      const int loc = voxel_local(vx, vy, vz);
+      const int loc = (int)dda_local(r);
+      const uint32_t xyz = r.loc;
+      float l, tin, te;
+      enter = dda_step(r, g, l, tin, te);
       const float p = belief[(int64_t)slot * kBrickVox + loc];
       A += log1pf(-p) * l;
       const float V = expf(A);
@@ -153,9 +171,9 @@ __global__ void k_pixel_diag(Geom g, Pose P, const float* __restrict__ belief, i
       rec[5] = V;
       reinterpret_cast<unsigned long long*>(out)[count * (kStride / 2) + 3] = (unsigned long long)slot;
       unsigned char* b = reinterpret_cast<unsigned char*>(rec + 8);
-      b[0] = (unsigned char)(vx & 7);
-      b[1] = (unsigned char)(vy & 7);
-      b[2] = (unsigned char)(vz & 7);
+      b[0] = (unsigned char)(xyz >> 8 & 7);
+      b[1] = (unsigned char)(xyz >> 4 & 7);
+      b[2] = (unsigned char)(xyz & 7);
       Vprev = V;
       ++count;
     }
@@ -174,7 +192,8 @@ cudaError_t launch_pixel_diag(const Geom& g, const Pose& P, const float* belief,
 cudaError_t launch_render(int mode, const Geom& g, const Pose& P, const float* depth,
                           const float* belief, float thresh, float* out, unsigned long long* counts,
                           cudaStream_t s) {
-  int nb = (g.rows * g.cols + kRenderThreads - 1) / kRenderThreads;
+  constexpr int kTiles = kRenderThreads / 32;
+  const int nb = (int)((pixel_tiles(g.rows, g.cols) + kTiles - 1) / kTiles);
   switch (mode) {
     case 0: k_render<0><<<nb, kRenderThreads, 0, s>>>(g, P, depth, belief, thresh, out, counts); break;
     case 1: k_render<1><<<nb, kRenderThreads, 0, s>>>(g, P, depth, belief, thresh, out, counts); break;
