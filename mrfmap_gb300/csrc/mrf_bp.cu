@@ -599,13 +599,14 @@ __global__ void k_ray_keys(const RayMeta* __restrict__ meta, uint32_t n, uint32_
 // into shared memory (coalesced permutation reads, kTile independent gathers
 // in flight) together with the segment bounds of the pairs the tile
 // touches; each thread then sums whole pairs sequentially from shared memory
-// (a fixed order) and updates the pairs that lie inside the tile.  Segments
-// that cross tile edges leave partial sums that k_pair_fixup adds in tile
-// order.  Any segment length balances: voxels next to the camera are crossed
-// by thousands of rays.
+// (a fixed order) and updates them.  A block owns the pairs that start in its
+// tile: the rest of the one that crosses into the next tile is summed by the
+// whole block (lane-strided, then a fixed tree), so no tile waits for another
+// and no second kernel adds carries (4.5 us per view and iteration, 14 % of
+// an iteration on 160x120 views).  A pair of thousands of messages takes its
+// block a few more rounds.
 constexpr int kTileThreads = 256;
 constexpr int kTile = 4 * kTileThreads;
-constexpr uint32_t kOpenStart = 1u, kOpenEnd = 2u, kSingle = 4u;
 
 // a dynamic run's update with its old message mo and the voxel's old total
 // Lo already loaded (the gate c > kCumLenGate already checked)
@@ -661,11 +662,12 @@ template <bool kTwo>
 __global__ void __launch_bounds__(kTileThreads, kTwo ? 5 : 8)
     k_pair_reduce(const uint32_t* __restrict__ perm, const float* __restrict__ pl,
                   const uint32_t* __restrict__ seg, const uint32_t* __restrict__ tile_first,
-                  uint32_t k0, uint32_t k1, uint32_t p_end, TileCarry* __restrict__ carry,
-                  const uint4* __restrict__ drun, float* __restrict__ m, float* __restrict__ L,
+                  uint32_t k0, uint32_t k1, uint32_t p_end, const uint4* __restrict__ drun, float* __restrict__ m, float* __restrict__ L,
                   float* __restrict__ dm, int jacobi) {
   __shared__ float sv[kTile];
   __shared__ uint32_t sseg[kTile + 2];
+  __shared__ float open_sum, open_m, open_L, part[kTileThreads / 32];
+  __shared__ uint4 open_run;
   const int t = threadIdx.x;
   const uint32_t base = k0 + blockIdx.x * kTile;
   const uint32_t n = min((uint32_t)kTile, k1 - base);
@@ -701,49 +703,45 @@ __global__ void __launch_bounds__(kTileThreads, kTwo ? 5 : 8)
     mo1 = m[r1.x];
     if (!jacobi) Lo1 = L[r1.y];
   }
+  if (t == kTileThreads - 1) {
+    // the pair at the next tile's first position, which this block may own
+    const uint4 r = drun[last];
+    open_run = r;
+    open_m = m[r.x];
+    open_L = jacobi ? 0.0f : L[r.y];
+  }
   __syncthreads();
   for (uint32_t q = t; q < n && pf + q < p_end && sseg[q] < end; q += kTileThreads) {
     const uint32_t s0 = sseg[q], s1 = sseg[q + 1];
-    const uint32_t a = max(s0, base) - base, b = min(s1, end) - base;
+    if (s0 < base) continue;  // an earlier tile's
+    const uint32_t a = s0 - base, b = min(s1, end) - base;
     float acc = 0.0f;
     for (uint32_t i = a; i < b; ++i) acc += sv[i];
-    const bool open_start = s0 < base, open_end = s1 > end;
-    if (!open_start && !open_end) {
-      if (q == t) {
-        if (gate0) apply_run_loaded(r0, mo0, Lo0, acc, m, L, dm, jacobi);
-      } else if (q == t + kTileThreads && pre1) {
-        if (gate1) apply_run_loaded(r1, mo1, Lo1, acc, m, L, dm, jacobi);
-      } else {
-        apply_run(drun[pf + q], acc, m, L, dm, jacobi);
-      }
+    if (s1 > end) {  // the last one
+      open_sum = acc;
       continue;
     }
-    TileCarry& c = carry[blockIdx.x];
-    if (open_start) {
-      c.first_key = pf + q;
-      c.first_sum = acc;
-    }
-    if (open_end) {
-      c.last_key = pf + q;
-      c.last_sum = acc;
+    if (q == t) {
+      if (gate0) apply_run_loaded(r0, mo0, Lo0, acc, m, L, dm, jacobi);
+    } else if (q == t + kTileThreads && pre1) {
+      if (gate1) apply_run_loaded(r1, mo1, Lo1, acc, m, L, dm, jacobi);
+    } else {
+      apply_run(drun[pf + q], acc, m, L, dm, jacobi);
     }
   }
+  // the pair that goes on behind the tile, if it starts in it
+  const uint32_t ql = last - pf;
+  if (sseg[ql] < base || sseg[ql] >= end || sseg[ql + 1] <= end) return;
+  const uint32_t s1 = sseg[ql + 1];
+  float x = 0.0f;
+  for (uint32_t i = end + t; i < s1; i += kTileThreads) x += pl[perm[i]];
+  x = warp_sum(x);
+  if ((t & 31) == 0) part[t >> 5] = x;
+  __syncthreads();  // open_sum and the warps' parts
   if (t == 0) {
-    // the first pair is open at the start iff it began before the tile; the
-    // last pair (the one holding position end-1) is open iff it goes on
-    // ql = last q with sseg[q] < end (binary search over the loaded starts)
-    uint32_t lo = 0, hi = min(n, p_end - pf);
-    while (hi - lo > 1) {
-      uint32_t mid = (lo + hi) >> 1;
-      if (sseg[mid] < end) lo = mid;
-      else hi = mid;
-    }
-    const uint32_t ql = lo;
-    uint32_t f = 0;
-    if (sseg[0] < base) f |= kOpenStart;
-    if (sseg[ql + 1] > end) f |= kOpenEnd;
-    if (ql == 0) f |= kSingle;
-    carry[blockIdx.x].flags = f;
+    for (int w = 1; w < kTileThreads / 32; ++w) x += part[w];
+    if (__uint_as_float(open_run.z) > kCumLenGate)
+      apply_run_loaded(open_run, open_m, open_L, open_sum + x, m, L, dm, jacobi);
   }
 }
 
@@ -761,27 +759,6 @@ __global__ void k_tile_first(const uint32_t* __restrict__ seg, uint32_t p0, uint
     else hi = mid;
   }
   out[t] = lo;
-}
-
-// segments crossing tile edges: the tile where such a segment starts walks
-// forward adding each following tile's partial, in tile order
-__global__ void k_pair_fixup(const TileCarry* __restrict__ carry, uint32_t ntiles,
-                             const uint4* __restrict__ drun, float* __restrict__ m,
-                             float* __restrict__ L, float* __restrict__ dm, int jacobi) {
-  uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= ntiles) return;
-  TileCarry c = carry[t];
-  if (!(c.flags & kOpenEnd)) return;
-  if ((c.flags & kSingle) && (c.flags & kOpenStart)) return;  // not where the segment starts
-  float sum = c.last_sum;
-  uint32_t key = c.last_key;
-  for (uint32_t u = t + 1; u < ntiles; ++u) {
-    TileCarry d = carry[u];
-    sum += d.first_sum;
-    if ((d.flags & kSingle) && (d.flags & kOpenEnd)) continue;
-    break;
-  }
-  apply_run(drun[key], sum, m, L, dm, jacobi);
 }
 
 // per dynamic run: {pair id, voxel, cumulative length, static-message sum}
@@ -1197,21 +1174,16 @@ cudaError_t launch_quiet_prefix(const BpArrays& a, uint32_t r_first, uint32_t n,
 }
 
 cudaError_t launch_pair_update(const BpArrays& a, uint32_t k0, uint32_t k1, uint32_t j0, uint32_t j1,
-                               const uint32_t* tile_first, TileCarry* carry, int jacobi,
-                               cudaStream_t s) {
+                               const uint32_t* tile_first, int jacobi, cudaStream_t s) {
   (void)j0;
   if (k1 <= k0) return cudaSuccess;
   uint32_t ntiles = (k1 - k0 + kTile - 1) / kTile;
   if (a.pair_variant)
     k_pair_reduce<true><<<ntiles, kTileThreads, 0, s>>>(a.dperm, a.inc_pl, a.dseg, tile_first, k0, k1, j1,
-                                                        carry, a.drun, a.pair_m, a.L, a.pair_dm, jacobi);
+                                                        a.drun, a.pair_m, a.L, a.pair_dm, jacobi);
   else
     k_pair_reduce<false><<<ntiles, kTileThreads, 0, s>>>(a.dperm, a.inc_pl, a.dseg, tile_first, k0, k1, j1,
-                                                         carry, a.drun, a.pair_m, a.L, a.pair_dm, jacobi);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  k_pair_fixup<<<blocks(ntiles, 256), 256, 0, s>>>(carry, ntiles, a.drun, a.pair_m, a.L, a.pair_dm,
-                                                   jacobi);
+                                                         a.drun, a.pair_m, a.L, a.pair_dm, jacobi);
   return cudaGetLastError();
 }
 

@@ -195,7 +195,7 @@ struct mrf_map {
   // what the last build left: views with lists, per-pixel entries, the ends
   // of the region blocks, the queues and the tiles
   int built_views = 0;
-  int64_t npix_total = 0, queue_end = 0, tile_end = 0, carry_tiles = 0, vox_active_n = 0;
+  int64_t npix_total = 0, queue_end = 0, tile_end = 0, vox_active_n = 0;
   int64_t n_loud_prefix = 0;  // entries of the static prefixes' loud lists
   int64_t loud_count_version = -1, loud_list_version = -1;  // builds the loud lists were counted / made for
   uint32_t region_end = 0;
@@ -216,7 +216,7 @@ struct mrf_map {
   std::vector<View> views;
   // arenas
   DBuf meta, inc_pair, inc_len, inc_mu, inc_pl, pair_vox, pair_m, pair_cum, pair_stat, pair_ndyn, pair_hit,
-      pair_q, pair_dm, dperm, s_q0, s_q1, s_q2, s_q3, s_q4, s_bf, s_bc, s_first, s_len, s_loud, dpair, dseg, drun, carry, ray_order, ray_queue, region_q, rstart, rcounters, counters,
+      pair_q, pair_dm, dperm, s_q0, s_q1, s_q2, s_q3, s_q4, s_bf, s_bc, s_first, s_len, s_loud, dpair, dseg, drun, ray_order, ray_queue, region_q, rstart, rcounters, counters,
       tile_first, lbase, lsingle, lprefix, queue_ids, region_ids, loud_off, loud, quiet_ray;
   uint32_t jac_tile_base = 0;
   int64_t n_inc = 0, n_pairs = 0, n_dperm = 0, n_dpairs = 0;
@@ -872,17 +872,20 @@ void emit_loud_lists(mrf_map* m) {
 }
 
 // Whether a call of `iters` iterations takes the static prefixes from
-// their quiet sums from its third iteration on: only when at least two
-// iterations use them (the quiet sums cost about one pass over the static
-// prefixes), the quiet incidences are at least half of the Pre incidences
-// and they average at least two 128-incidence chunks per ray (else the
-// per-ray overhead outweighs the saved gathers: maps of short rays, or of
-// rays near many surfaces).  Counts the loud lists of the current build
-// when needed and makes them when the answer is yes.
-constexpr int64_t kQuietPerRay = 256;
+// their quiet sums from its third iteration on.  Per iteration that saves the
+// gathers of the quiet incidences; it costs a pass over the static prefixes
+// per call (the quiet sums), and two more when the current build has no loud
+// lists yet: the call must be long enough for either (8 x 640x480 at 1 cm:
+// 0.10 ms a view and iteration saved, 0.17 and 0.36 spent), the quiet
+// incidences at least half of the Pre incidences, and on average enough per
+// ray to outweigh the records (5 x 160x120 at 4 cm, 70 a ray: iteration 0.19
+// -> 0.16 ms; 32 views of 8 scenes at 2 cm, 100 a ray: 1.43 -> 1.24).
+constexpr int64_t kQuietPerRay = 48;
+constexpr int64_t kQuietIters = 4, kQuietItersNew = 8;
 bool quiet_path(mrf_map* m, int64_t iters, int flags) {
   const bool force = (flags & MRF_QUIET_PREFIX) != 0;
-  if (iters < (force ? 3 : 4) || (flags & MRF_FULL_RAYS) || m->n_inc <= 0 || m->npix_total <= 0) return false;
+  if ((flags & MRF_FULL_RAYS) || m->n_inc <= 0 || m->npix_total <= 0) return false;
+  if (iters < (force ? 3 : (m->loud_list_version == m->built_version ? kQuietIters : kQuietItersNew))) return false;
   const int64_t pre = m->stats.n_inc_pre_bp, k4 = m->stats.n_inc_from_k4, rays = m->stats.n_rays_bp;
   if (!force && (rays <= 0 || pre - k4 < kQuietPerRay * rays)) return false;  // no count needed
   if (m->loud_count_version != m->built_version) {
@@ -1051,8 +1054,6 @@ void rebuild_lists(mrf_map* m, OldPairs& old) {
     // first pair of every tile, per view (Gauss-Seidel) and over all views
     // (Jacobi)
     int64_t tiles = (int64_t)pair_update_tiles((uint32_t)std::min<int64_t>(dperm_total, 0xFFFFFFF0ll)) + V + 1;
-    m->carry_tiles = tiles;
-    m->carry.reserve((size_t)tiles * sizeof(TileCarry), false, m->stream);
     m->tile_first.reserve((size_t)(2 * tiles + 2) * 4, false, m->stream);
     uint32_t tb = 0;
     for (int c = 0; c < V; ++c) {
@@ -1267,15 +1268,11 @@ void append_lists(mrf_map* m) {
     for (int c = m->built_views; c < V; ++c) need += pair_update_tiles(m->views[c].n_dperm) + 1;
     m->tile_first.reserve((size_t)(need + 2) * 4, true, m->stream);
     uint32_t tb = (uint32_t)m->tile_end;
-    int64_t most = m->carry_tiles;
     for (int c = m->built_views; c < V; ++c) {
       view_tiles(m, c, tb);
       tb += pair_update_tiles(m->views[c].n_dperm) + 1;
-      most = std::max<int64_t>(most, (int64_t)pair_update_tiles(m->views[c].n_dperm) + 1);
     }
     m->tile_end = tb;
-    m->carry_tiles = most;
-    m->carry.reserve((size_t)most * sizeof(TileCarry), false, m->stream);
   }
   // active voxels: the new bricks' voxels start at 0, the new pairs add theirs
   m->vox_active.reserve((size_t)std::max<int64_t>(nvox, 1), true, m->stream);
@@ -1517,8 +1514,8 @@ void enqueue_iteration(mrf_map* m, const BpArrays& a, bool jacobi, int fix, int 
       if (v.n_dperm) {
         CK(launch_pair_update(a, v.dperm_base, v.dperm_base + v.n_dperm, v.dpair_base,
                               v.dpair_base + v.n_dpairs, m->tile_first.as<uint32_t>() + v.tile_base,
-                              m->carry.as<TileCarry>(), 0, m->stream));
-        launches += 2;
+                              0, m->stream));
+        ++launches;
       }
       if (first) {
         CK(launch_static_pairs(a, v.pair_base, v.pair_base + v.n_pairs, 0, m->stream));
@@ -1538,15 +1535,14 @@ void enqueue_iteration(mrf_map* m, const BpArrays& a, bool jacobi, int fix, int 
     prof.end();
     prof.begin(2);
     CK(launch_pair_update(a, 0, (uint32_t)m->n_dperm, 0, (uint32_t)m->n_dpairs,
-                          m->tile_first.as<uint32_t>() + m->jac_tile_base, m->carry.as<TileCarry>(),
-                          1, m->stream));
+                          m->tile_first.as<uint32_t>() + m->jac_tile_base, 1, m->stream));
     if (first) CK(launch_static_pairs(a, 0, P, 1, m->stream));
     prof.end();
     prof.begin(3);
     CK(launch_voxel_apply(m->vseg.as<uint32_t>(), m->vpairs.as<uint32_t>(), m->vvox.as<uint32_t>(),
                           m->n_vvox, m->pair_dm.as<float>(), m->d_L.as<float>(), m->stream));
     prof.end();
-    launches += 5 + (first ? 1 : 0);
+    launches += 4 + (first ? 1 : 0);
   }
 }
 
@@ -1758,7 +1754,7 @@ void destroy_bufs(mrf_map* m) {
                  &m->pair_m, &m->pair_cum, &m->pair_stat, &m->pair_ndyn, &m->pair_hit, &m->pair_q,
                  &m->pair_dm,
                  &m->dperm, &m->dpair, &m->dseg, &m->drun,
-                 &m->carry, &m->ray_order, &m->ray_queue, &m->region_q, &m->rstart, &m->rcounters, &m->counters, &m->tile_first,
+                 &m->ray_order, &m->ray_queue, &m->region_q, &m->rstart, &m->rcounters, &m->counters, &m->tile_first,
                  &m->lbase, &m->lsingle, &m->lprefix, &m->queue_ids, &m->region_ids, &m->loud_off,
                  &m->loud, &m->quiet_ray,
                  &m->vseg, &m->vpairs, &m->vvox, &m->vox_active, &m->d_Lbase, &m->inc_len16, &m->pair_q16,
@@ -2240,8 +2236,7 @@ static void warm_start_impl(mrf_map* m, const float* L_pred, bool device_ptr, in
     CK(launch_pair_prepare(a, 0, P, 1, m->stream));
     CK(launch_ray_bp(a, ray_work(m, -1), 0, m->num_sms, m->variant_for(V > 1), false, m->stream));
     CK(launch_pair_update(a, 0, (uint32_t)m->n_dperm, 0, (uint32_t)m->n_dpairs,
-                          m->tile_first.as<uint32_t>() + m->jac_tile_base, m->carry.as<TileCarry>(),
-                          1, m->stream));
+                          m->tile_first.as<uint32_t>() + m->jac_tile_base, 1, m->stream));
   }
   start_logodds(m, lp);
   CK(launch_voxel_rebuild(m->vseg.as<uint32_t>(), m->vpairs.as<uint32_t>(), m->vvox.as<uint32_t>(),

@@ -200,12 +200,6 @@ struct BpArrays {
   const __half* inc_len16;
   __half* pair_lnq16;
 };
-// per-tile partial sums of the pair-update segmented reduction
-struct TileCarry {
-  uint32_t first_key, last_key;
-  float first_sum, last_sum;
-  uint32_t flags;
-};
 uint32_t pair_update_tiles(uint32_t n);
 cudaError_t launch_pair_prepare(const BpArrays& a, uint32_t p0, uint32_t p1, int jacobi,
                                 cudaStream_t s);
@@ -263,8 +257,7 @@ cudaError_t launch_ray_queue(const RayMeta* meta, const uint32_t* order, uint32_
 // dynamic positions k0..k1 hold the runs j0..j1 (dpair/dseg indices);
 // tile_first from launch_tile_first over dseg
 cudaError_t launch_pair_update(const BpArrays& a, uint32_t k0, uint32_t k1, uint32_t j0, uint32_t j1,
-                               const uint32_t* tile_first, TileCarry* carry, int jacobi,
-                               cudaStream_t s);
+                               const uint32_t* tile_first, int jacobi, cudaStream_t s);
 // per-run records of the pair update (from dpair and the pair arrays)
 cudaError_t launch_drun(const uint32_t* dpair, uint32_t n, const uint32_t* pair_vox, const float* cum,
                         const float* stat, uint4* drun, cudaStream_t s);
