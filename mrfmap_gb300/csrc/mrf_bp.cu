@@ -997,46 +997,6 @@ __global__ void k_touch_pairs(const uint32_t* __restrict__ pair_vox, const float
   if (n_active && (threadIdx.x & 31) == 0 && b) atomicAdd(n_active, (unsigned long long)__popc(b));
 }
 
-// 64-bit total of n u32 counts (the incidence total of a build, checked
-// against the 32-bit index range before any offset is formed from it)
-__global__ void k_sum_u32(const uint32_t* __restrict__ v, int64_t n, unsigned long long* __restrict__ out) {
-  unsigned long long c = 0;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    c += v[i];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(kFull, c, o);
-  if ((threadIdx.x & 31) == 0 && c) atomicAdd(out, c);
-}
-
-// the per-view counters of a view's ray records, kRayCounters 64-bit totals:
-// Pre incidences, rays with any, Post incidences, dynamic Post incidences
-// (those from k_dyn on), rays in BP, their Pre incidences, and their Pre
-// incidences from the quiet-prefix boundary (k_dyn rounded down to 4) on.
-// Integer sums: the totals do not depend on the order of the atomics.
-__global__ void k_ray_counters(const RayMeta* __restrict__ meta, int64_t n, unsigned long long* __restrict__ out) {
-  unsigned long long c[kRayCounters] = {};
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const RayMeta r = meta[i];
-    const int kd = ray_kdyn(r);
-    c[0] += r.n_pre;
-    c[1] += r.n_pre > 0;
-    c[2] += r.n_post;
-    c[3] += (unsigned)(r.n_post - min(kd, (int)r.n_post));
-    if (ray_in_bp(r)) {
-      c[4] += 1;
-      c[5] += r.n_pre;
-      c[6] += (unsigned long long)(long long)((int)r.n_pre - (kd & ~3));  // two's complement: a signed total
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < kRayCounters; ++k) {
-    unsigned long long v = c[k];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
-    if ((threadIdx.x & 31) == 0 && v) atomicAdd(out + k, v);
-  }
-}
-
 __global__ void k_count_flags(const uint8_t* __restrict__ flag, int64_t n, unsigned long long* __restrict__ out) {
   unsigned c = 0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -1347,20 +1307,6 @@ cudaError_t launch_touch_counts(const uint32_t* pair_vox, const float* cum, uint
   if (np) k_touch_pairs<<<blocks(np, 256), 256, 0, s>>>(pair_vox, cum, np, flag, out2);
   if (nvox > 0)
     k_count_flags<<<(unsigned)std::min<int64_t>(blocks(nvox, 256), 4096), 256, 0, s>>>(flag, nvox, out2 + 1);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_sum_u32(const uint32_t* v, int64_t n, unsigned long long* out, cudaStream_t s) {
-  cudaError_t e = cudaMemsetAsync(out, 0, 8, s);
-  if (e != cudaSuccess || n <= 0) return e;
-  k_sum_u32<<<(unsigned)std::min<int64_t>(blocks(n, 256), 4096), 256, 0, s>>>(v, n, out);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_ray_counters(const RayMeta* meta, int64_t n, unsigned long long* out, cudaStream_t s) {
-  cudaError_t e = cudaMemsetAsync(out, 0, kRayCounters * sizeof(unsigned long long), s);
-  if (e != cudaSuccess || n <= 0) return e;
-  k_ray_counters<<<(unsigned)std::min<int64_t>(blocks(n, 256), 1024), 256, 0, s>>>(meta, n, out);
   return cudaGetLastError();
 }
 

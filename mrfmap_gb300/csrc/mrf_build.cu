@@ -9,6 +9,7 @@
 //   per-brick stop rules      src/cuda/gvdbkernels.cu:568, 816, 1035
 //   infinity-term gate        src/cuda/gvdbkernels.cu:1196-1208
 //   Pre-pass visibility reset src/cuda/gvdbkernels.cu:708-715
+#include <algorithm>
 #include <cub/cub.cuh>
 
 #include "mrf_geometry.cuh"
@@ -149,21 +150,30 @@ __global__ void k_set_points(Geom g, const float* __restrict__ pts, const float*
   belief[(int64_t)s * kBrickVox + voxel_local(vx, vy, vz)] = occ[i];
 }
 
+// the view of a block of a batch
+__device__ __forceinline__ int batch_view(const TraceBatch& b) {
+  int k = 0;
+  while (k + 1 < b.n && blockIdx.x >= b.first[k + 1]) ++k;
+  return k;
+}
+constexpr int kTraceThreads = 128;
+
 // Incidences of each pixel's Pre pass, padded to a multiple of 4 (the emit
 // pass's offsets): the voxels the ray crosses in active bricks up to the
 // brick run whose end is past the return, counted brick by brick.
-__global__ void __launch_bounds__(128)
-    k_trace_count(Geom g, Pose P, const float* __restrict__ depth, uint32_t* __restrict__ counts,
-                  int* __restrict__ err) {
-  const int pix = tile_pixel(g.rows, g.cols, (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5, threadIdx.x & 31);
-  if (pix < 0) return;
-  const float d = depth[pix];
+__global__ void __launch_bounds__(kTraceThreads)
+    k_trace_count(const __grid_constant__ TraceBatch batch, int* __restrict__ err) {
+  const TraceView& w = batch.v[batch_view(batch)];
+  const Geom& g = w.g;
+  const int64_t block = blockIdx.x - batch.first[batch_view(batch)];
+  const int pix = tile_pixel(g.rows, g.cols, (block * kTraceThreads + threadIdx.x) >> 5, threadIdx.x & 31);
   int count = 0;
+  const float d = pix < 0 ? 0.0f : w.depth[pix];
   if (d > 0.0f) {
     const int x = pix % g.cols, y = pix / g.cols;
     const Sensor c = sensor_at(g, x, y);
     Ray ray;
-    ray_setup(g, P, x, y, ray);
+    ray_setup(g, w.P, x, y, ray);
     Dda r;
     if (dda_init(r, g, ray)) {
       while (r.alive && r.guard > 0) {
@@ -181,7 +191,11 @@ __global__ void __launch_bounds__(128)
       }
     }
   }
-  counts[pix] = (uint32_t)((count + 3) & ~3);
+  const uint32_t padded = (uint32_t)((count + 3) & ~3);
+  if (pix >= 0) w.counts[pix] = padded;
+  if (pix == 0) w.counts[g.rows * g.cols] = 0u;
+  const uint32_t sum = __reduce_add_sync(0xFFFFFFFFu, padded);
+  if ((threadIdx.x & 31) == 0 && sum) atomicAdd(w.total, (unsigned long long)sum);
 }
 
 // One thread per pixel walks the DDA through the active bricks.  Runs of
@@ -192,25 +206,24 @@ __global__ void __launch_bounds__(128)
 // reads and writes twice.  A ray's lists start on a multiple of four; the last
 // group is completed with padding.  A list that does not fill the room its
 // count gave it raises the error flag.
-constexpr int kEmitThreads = 128;
 constexpr int kEmitStride = 12;  // words of a thread's eight in each list: 16-byte loads, four ways to a bank
 
-__global__ void __launch_bounds__(kEmitThreads, 6)
-    k_trace_emit(Geom g, Pose P, const float* __restrict__ depth, const uint32_t* __restrict__ pix_off,
-                 uint32_t inc_base, RayMeta* __restrict__ meta, uint32_t* __restrict__ inc_vox,
-                 float* __restrict__ inc_len, float* __restrict__ inc_mu, int* __restrict__ err) {
-  const int pix = tile_pixel(g.rows, g.cols, (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5, threadIdx.x & 31);
-  __shared__ __align__(16) uint32_t pending[3][kEmitThreads * kEmitStride];
-  if (pix < 0) return;
-  const float d = depth[pix];
+__device__ __forceinline__ RayMeta emit_ray(const TraceView& w, int pix,
+                                            uint32_t (&pending)[3][kTraceThreads * kEmitStride],
+                                            uint8_t* __restrict__ loud, int* __restrict__ err) {
+  const Geom& g = w.g;
+  uint32_t* __restrict__ inc_vox = w.vox;
+  float* __restrict__ inc_len = w.len;
+  float* __restrict__ inc_mu = w.mu;
+  const float d = w.depth[pix];
   int count = 0, n_pre = -1, n_post = -1, r0 = -1, run_start = 0, kmu = -1;
   bool gate = false;
-  const uint32_t base = pix_off[pix];
-  const int room = (int)(pix_off[pix + 1] - base);
+  const uint32_t base = w.pix_off[pix] - w.pix_off[0];
+  const int room = (int)(w.pix_off[pix + 1] - w.pix_off[0] - base);
   // the group of eight incidence k belongs to, counted in the arena so that
   // whole groups are whole sectors; the ray's first may be a half
   const uint32_t mine = threadIdx.x * kEmitStride;
-  const uint32_t phase = (inc_base + base) & 7u;
+  const uint32_t phase = (w.inc_base + base) & 7u;
   auto push = [&](uint32_t k, uint32_t v, float len, float mu) {
     const uint32_t a = mine + ((phase + k) & 7u);
     pending[0][a] = v;
@@ -235,7 +248,7 @@ __global__ void __launch_bounds__(kEmitThreads, 6)
     const int x = pix % g.cols, y = pix / g.cols;
     const Sensor c = sensor_at(g, x, y);
     Ray ray;
-    ray_setup(g, P, x, y, ray);
+    ray_setup(g, w.P, x, y, ray);
     Dda r;
     if (dda_init(r, g, ray)) {
       bool run_open = false;
@@ -283,6 +296,8 @@ __global__ void __launch_bounds__(kEmitThreads, 6)
           }
           push((uint32_t)count, v, l, mu);
           if (((phase + count) & 7) == 7) flush((uint32_t)count);
+          // dynamic: in the Post range, from the first non-zero potential on
+          if (kmu >= 0 && n_post < 0) loud[v] = 1;
           ++count;
         } while (!left && r.guard > 0);
       }
@@ -305,13 +320,40 @@ __global__ void __launch_bounds__(kEmitThreads, 6)
   if (padded != room) atomicOr(err, 2);
   const int kdyn = (kmu >= 0 && kmu < n_post) ? kmu : n_post;
   RayMeta m;
-  m.off = inc_base + base;
+  m.off = w.inc_base + base;
   m.n_pre = (uint16_t)n_pre;
   m.n_post = (uint16_t)n_post;
   m.r0 = (uint16_t)(r0 >= 0 ? r0 : n_pre);
   m.rinf = (uint16_t)(r0 >= 0 ? r0 : run_start);
   m.flags = (gate ? 1u : 0u) | ((uint32_t)kdyn << 16);
-  meta[pix] = m;
+  w.meta[pix] = m;
+  return m;
+}
+
+__global__ void __launch_bounds__(kTraceThreads, 6)
+    k_trace_emit(const __grid_constant__ TraceBatch batch, uint8_t* __restrict__ loud, int* __restrict__ err) {
+  __shared__ __align__(16) uint32_t pending[3][kTraceThreads * kEmitStride];
+  const int vi = batch_view(batch);
+  const TraceView& w = batch.v[vi];
+  const Geom& g = w.g;
+  const int64_t block = blockIdx.x - batch.first[vi];
+  const int pix = tile_pixel(g.rows, g.cols, (block * kTraceThreads + threadIdx.x) >> 5, threadIdx.x & 31);
+  RayMeta m = {};
+  if (pix >= 0) m = emit_ray(w, pix, pending, loud, err);
+  // the view's totals: a warp's in 32 bits (rays are shorter than 2^16)
+  const bool bp = ray_in_bp(m);
+  const uint32_t c[kRayCounters] = {m.n_pre,
+                                    m.n_pre > 0 ? 1u : 0u,
+                                    m.n_post,
+                                    (uint32_t)(m.n_post - ray_kdyn(m)),
+                                    bp ? 1u : 0u,
+                                    bp ? m.n_pre : 0u,
+                                    bp ? (uint32_t)(m.n_pre - (ray_kdyn(m) & ~3)) : 0u};
+#pragma unroll
+  for (int k = 0; k < kRayCounters; ++k) {
+    const uint32_t sum = __reduce_add_sync(0xFFFFFFFFu, c[k]);
+    if ((threadIdx.x & 31) == 0 && sum) atomicAdd(w.counters + k, (unsigned long long)sum);
+  }
 }
 
 // Pairs.  A pair is a (camera, voxel) with at least one incidence.  The pairs
@@ -564,17 +606,6 @@ __global__ void k_dyn_counts(const RayMeta* __restrict__ meta, uint32_t npix, ui
   if (r < npix) cnt[r] = (uint32_t)(meta[r].n_post - ray_kdyn(meta[r]));
 }
 
-// loud[v] = 1 for every voxel with a dynamic incidence (any view): one
-// thread per ray walks its dynamic range [k_dyn, n_post); vox[k] holds the
-// voxel of incidence vox_base + k
-__global__ void k_loud_voxels(const RayMeta* __restrict__ meta, int64_t npix, const uint32_t* __restrict__ vox,
-                              uint32_t vox_base, uint8_t* __restrict__ loud) {
-  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= npix) return;
-  const RayMeta me = meta[r];
-  for (int i = ray_kdyn(me); i < me.n_post; ++i) loud[vox[me.off - vox_base + i]] = 1;
-}
-
 // *count += number of pairs on loud voxels
 __global__ void k_count_loud(const uint32_t* __restrict__ pair_vox, uint32_t np,
                              const uint8_t* __restrict__ loud, uint32_t* __restrict__ count) {
@@ -756,10 +787,36 @@ cudaError_t launch_set_points(const Geom& g, const float* pts, const float* occ,
   return cudaGetLastError();
 }
 
-cudaError_t launch_trace_count(const Geom& g, const Pose& P, const float* depth, uint32_t* counts, int* err,
-                               cudaStream_t s) {
-  k_trace_count<<<grid_for(pixel_tiles(g.rows, g.cols) * 32, 128), 128, 0, s>>>(g, P, depth, counts, err);
-  return cudaGetLastError();
+// batches of up to kTraceBatch views, the blocks of one view after another's
+template <typename F>
+cudaError_t trace_batches(const TraceView* views, int n, F launch) {
+  for (int k0 = 0; k0 < n; k0 += kTraceBatch) {
+    TraceBatch b;
+    b.n = std::min(kTraceBatch, n - k0);
+    uint32_t blocks = 0;
+    for (int k = 0; k < b.n; ++k) {
+      b.v[k] = views[k0 + k];
+      b.first[k] = blocks;
+      blocks += grid_for(pixel_tiles(b.v[k].g.rows, b.v[k].g.cols) * 32, kTraceThreads);
+    }
+    b.first[b.n] = blocks;
+    launch(b, blocks);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
+cudaError_t launch_trace_count(const TraceView* views, int n, int* err, cudaStream_t s) {
+  return trace_batches(views, n, [&](const TraceBatch& b, uint32_t blocks) {
+    k_trace_count<<<blocks, kTraceThreads, 0, s>>>(b, err);
+  });
+}
+
+cudaError_t launch_trace_emit(const TraceView* views, int n, uint8_t* loud, int* err, cudaStream_t s) {
+  return trace_batches(views, n, [&](const TraceBatch& b, uint32_t blocks) {
+    k_trace_emit<<<blocks, kTraceThreads, 0, s>>>(b, loud, err);
+  });
 }
 
 // The pixels of a view whose rays may cross one of the bricks in slots
@@ -813,14 +870,6 @@ cudaError_t launch_brick_footprint(const Geom& g, const Pose& P, const int* coor
                                    uint8_t* mask, int* all, cudaStream_t s) {
   if (b1 <= b0) return cudaSuccess;
   k_brick_footprint<<<grid_for(b1 - b0), kThreads, 0, s>>>(g, P, coord, b0, b1, mask, all);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_trace_emit(const Geom& g, const Pose& P, const float* depth,
-                              const uint32_t* pix_off, uint32_t inc_base, RayMeta* meta,
-                              uint32_t* inc_vox, float* inc_len, float* inc_mu, int* err, cudaStream_t s) {
-  k_trace_emit<<<grid_for(pixel_tiles(g.rows, g.cols) * 32, kEmitThreads), kEmitThreads, 0, s>>>(
-      g, P, depth, pix_off, inc_base, meta, inc_vox, inc_len, inc_mu, err);
   return cudaGetLastError();
 }
 
@@ -901,13 +950,6 @@ cudaError_t launch_run_stats(const uint32_t* dpair, const uint32_t* dseg, const 
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   k_run_stats_long<<<1024, kStatThreads, 0, s>>>(a, long_list);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_loud_voxels(const RayMeta* meta, int64_t npix, const uint32_t* vox, uint32_t vox_base,
-                               uint8_t* loud, cudaStream_t s) {
-  if (npix <= 0) return cudaSuccess;
-  k_loud_voxels<<<grid_for(npix), kThreads, 0, s>>>(meta, npix, vox, vox_base, loud);
   return cudaGetLastError();
 }
 

@@ -401,21 +401,15 @@ void rebuild(mrf_map* m) {
 
 // ---- per-view pieces of a build ------------------------------------------
 
-// The counters of the given views' rays, summed on the device from their ray
-// records (k_ray_counters), and the records of pixels [hm_base, hm_base +
-// hm.size()) copied to the host for the region lists: one synchronisation.
+// The counters of the given views' rays (s_vcnt, from the emit pass), and the
+// records of pixels [hm_base, hm_base + hm.size()) copied to the host for the
+// region lists: one synchronisation.
 void ray_records_and_counters(mrf_map* m, const std::vector<int>& views, int64_t hm_base,
                               std::vector<RayMeta>& hm) {
   const size_t K = (size_t)kRayCounters;
-  m->s_vcnt.reserve(std::max<size_t>(views.size(), 1) * K * 8, false, m->stream);
-  unsigned long long* dc = m->s_vcnt.as<unsigned long long>();
-  for (size_t k = 0; k < views.size(); ++k) {
-    const View& v = m->views[(size_t)views[k]];
-    CK(launch_ray_counters(m->meta.as<RayMeta>() + v.pix_base, view_pixels(v), dc + k * K, m->stream));
-  }
   std::vector<unsigned long long> hc(views.size() * K, 0ull);
   if (!hc.empty())
-    CK(cudaMemcpyAsync(hc.data(), dc, hc.size() * 8, cudaMemcpyDeviceToHost, m->stream));
+    CK(cudaMemcpyAsync(hc.data(), m->s_vcnt.p, hc.size() * 8, cudaMemcpyDeviceToHost, m->stream));
   if (!hm.empty())
     CK(cudaMemcpyAsync(hm.data(), m->meta.as<RayMeta>() + hm_base, hm.size() * sizeof(RayMeta),
                        cudaMemcpyDeviceToHost, m->stream));
@@ -776,10 +770,11 @@ void stats_from_views(mrf_map* m) {
 }
 
 // Incidence counts of the given views: view k's pixel counts at
-// s_counts + coff[k] (its hw entries and a sentinel) and their exclusive scan
-// at s_offs + coff[k]; each view's total is summed in 64 bits and the running
-// total (from `before` incidences already in the arenas) checked against the
-// 32-bit index range before any offset is used.  Returns the views' counts.
+// s_counts + coff[k] (its hw entries and a zero) and the exclusive scan of
+// all of them at s_offs; the views' totals are summed in 64 bits and the
+// running total (from `before` incidences already in the arenas) checked
+// against the 32-bit index range before any offset is used.  Returns the
+// views' counts.
 std::vector<uint32_t> count_views(mrf_map* m, const std::vector<int>& views, int64_t before,
                                   std::vector<int64_t>& coff) {
   int64_t tot_px = 0;
@@ -788,40 +783,67 @@ std::vector<uint32_t> count_views(mrf_map* m, const std::vector<int>& views, int
     coff[k] = tot_px;
     tot_px += view_pixels(m->views[views[k]]) + 1;
   }
-  m->s_counts.reserve((size_t)std::max<int64_t>(tot_px, 1) * 4, false, m->stream);
-  m->s_offs.reserve((size_t)std::max<int64_t>(tot_px, 1) * 4, false, m->stream);
-  m->s_delta.reserve(64, false, m->stream);
   std::vector<uint32_t> n(views.size(), 0u);
-  unsigned long long run = (unsigned long long)before;
+  if (views.empty()) return n;
+  u32_checked(tot_px, "pixel count");
+  m->s_counts.reserve((size_t)tot_px * 4, false, m->stream);
+  m->s_offs.reserve((size_t)tot_px * 4, false, m->stream);
+  m->s_delta.reserve(std::max<size_t>(views.size() * 8, 64), false, m->stream);
+  CK(cudaMemsetAsync(m->s_delta.p, 0, views.size() * 8, m->stream));
+  std::vector<TraceView> tv(views.size());
   for (size_t k = 0; k < views.size(); ++k) {
     const View& v = m->views[views[k]];
-    const int64_t hw = view_pixels(v);
-    uint32_t* cnt = m->s_counts.as<uint32_t>() + coff[k];
-    if (hw) CK(launch_trace_count(v.cam, v.pose, v.depth.as<float>(), cnt, m->s_err.as<int>(), m->stream));
-    CK(launch_sum_u32(cnt, hw, m->s_delta.as<unsigned long long>(), m->stream));
-    const unsigned long long total = read1(m, m->s_delta.as<unsigned long long>());
-    run += total;
+    TraceView& t = tv[k];
+    t = TraceView{};
+    t.g = v.cam;
+    t.P = v.pose;
+    t.depth = v.depth.as<float>();
+    t.counts = m->s_counts.as<uint32_t>() + coff[k];
+    t.total = m->s_delta.as<unsigned long long>() + k;
+  }
+  CK(launch_trace_count(tv.data(), (int)tv.size(), m->s_err.as<int>(), m->stream));
+  const size_t tb = scan_temp_bytes((uint32_t)tot_px);
+  m->s_tmp.reserve(tb, false, m->stream);
+  CK(exclusive_scan_u32(m->s_tmp.p, tb, m->s_counts.as<uint32_t>(), m->s_offs.as<uint32_t>(), (uint32_t)tot_px,
+                        m->stream));
+  std::vector<unsigned long long> total(views.size(), 0ull);
+  CK(cudaMemcpyAsync(total.data(), m->s_delta.p, total.size() * 8, cudaMemcpyDeviceToHost, m->stream));
+  sync(m);
+  unsigned long long run = (unsigned long long)before;
+  for (size_t k = 0; k < views.size(); ++k) {
+    run += total[k];
     if (run > 0xFFFFFFF0ull)
       fail(MRF_ERR_CAPACITY, "incidence count " + std::to_string(run) +
                                  " exceeds the 32-bit incidence index range (fewer or smaller views per map)");
-    CK(cudaMemsetAsync(cnt + hw, 0, 4, m->stream));
-    size_t tb = scan_temp_bytes((uint32_t)(hw + 1));
-    m->s_tmp.reserve(tb, false, m->stream);
-    CK(exclusive_scan_u32(m->s_tmp.p, tb, cnt, m->s_offs.as<uint32_t>() + coff[k], (uint32_t)(hw + 1),
-                          m->stream));
-    n[k] = (uint32_t)total;
+    n[k] = (uint32_t)total[k];
   }
   check_device_err(m);
   return n;
 }
 
-// the emit pass of view c at v.inc_base (pix_off: its scanned counts)
-void emit_view(mrf_map* m, int c, const uint32_t* pix_off) {
-  View& v = m->views[c];
-  CK(launch_trace_emit(v.cam, v.pose, v.depth.as<float>(), pix_off, v.inc_base,
-                       m->meta.as<RayMeta>() + v.pix_base, m->s_vox.as<uint32_t>() + (v.inc_base - m->scratch_base),
-                       m->inc_len.as<float>() + v.inc_base, m->inc_mu.as<float>() + v.inc_base, m->s_err.as<int>(),
-                       m->stream));
+// the emit pass of the given views, each at its inc_base (coff: their places
+// in the scanned counts): lists, ray records, counters (s_vcnt), loud flags
+void emit_views(mrf_map* m, const std::vector<int>& views, const std::vector<int64_t>& coff) {
+  const size_t cb = views.size() * (size_t)kRayCounters * 8;
+  m->s_vcnt.reserve(std::max<size_t>(cb, 8), false, m->stream);
+  CK(cudaMemsetAsync(m->s_vcnt.p, 0, std::max<size_t>(cb, 8), m->stream));
+  std::vector<TraceView> tv(views.size());
+  for (size_t k = 0; k < views.size(); ++k) {
+    const View& v = m->views[views[k]];
+    TraceView& t = tv[k];
+    t = TraceView{};
+    t.g = v.cam;
+    t.P = v.pose;
+    t.depth = v.depth.as<float>();
+    t.pix_off = m->s_offs.as<uint32_t>() + coff[k];
+    t.inc_base = v.inc_base;
+    t.meta = m->meta.as<RayMeta>() + v.pix_base;
+    t.vox = m->s_vox.as<uint32_t>() + (v.inc_base - m->scratch_base);
+    t.len = m->inc_len.as<float>() + v.inc_base;
+    t.mu = m->inc_mu.as<float>() + v.inc_base;
+    t.counters = m->s_vcnt.as<unsigned long long>() + k * kRayCounters;
+  }
+  CK(launch_trace_emit(tv.data(), (int)tv.size(), m->s_loud.as<uint8_t>(), m->s_err.as<int>(), m->stream));
 }
 
 // tiles of view c's pair update, from position tb of tile_first
@@ -960,22 +982,16 @@ void rebuild_lists(mrf_map* m, OldPairs& old) {
     m->s_vox.reserve(ib, false, m->stream);
     m->scratch_base = 0;
   }
-  // 3. emit
-  for (size_t k = 0; k < live.size(); ++k) emit_view(m, live[k], m->s_offs.as<uint32_t>() + coff[k]);
-  // per-view counters from the ray records
-  std::vector<RayMeta> hm((size_t)npix);
-  {
-    std::vector<int> all_views((size_t)V);
-    for (int c = 0; c < V; ++c) all_views[(size_t)c] = c;
-    ray_records_and_counters(m, all_views, 0, hm);
-  }
-  // voxels with a dynamic incidence in any view ("loud"; the others are
-  // quiet, see enqueue_iteration)
+  // 3. emit; voxels with a dynamic incidence in any view are "loud" (the
+  // others are quiet, see enqueue_iteration)
   m->s_loud.reserve((size_t)std::max<int64_t>(m->n_bricks * kBrickVox, 1), false, m->stream);
   CK(cudaMemsetAsync(m->s_loud.p, 0, (size_t)std::max<int64_t>(m->n_bricks * kBrickVox, 1), m->stream));
   m->loud_n = m->n_bricks * kBrickVox;
-  CK(launch_loud_voxels(m->meta.as<RayMeta>(), npix, m->s_vox.as<uint32_t>(), 0u, m->s_loud.as<uint8_t>(),
-                        m->stream));
+  emit_views(m, live, coff);
+  std::vector<RayMeta> hm((size_t)npix);
+  ray_records_and_counters(m, live, 0, hm);
+  for (View& v : m->views)
+    if (v.retired) v.c_npre = v.c_nrays = v.c_npost = v.c_ndyn = v.c_nrays_bp = v.c_npre_bp = v.c_nfast_bp = 0;
   // the region lists of the SM-affine schedule are host work on the ray
   // records alone: built on host threads while the GPU builds the pairs
   std::vector<RegionLists> lists((size_t)V);
@@ -1158,7 +1174,15 @@ void append_lists(mrf_map* m) {
     const size_t sb = (size_t)std::max<int64_t>(n_inc - m->n_inc, 1) * 4;
     m->s_vox.reserve(sb, false, m->stream);
   }
-  for (size_t k = 0; k < added.size(); ++k) emit_view(m, added[k], m->s_offs.as<uint32_t>() + coff[k]);
+  // loud voxels: the old views' stay flagged (those of views retired since the
+  // last full build too: a quiet voxel taken for a loud one only costs its
+  // pairs' preparation), the emit pass adds the new views'
+  const int64_t nvox = m->n_bricks * kBrickVox;
+  m->s_loud.reserve((size_t)std::max<int64_t>(nvox, 1), true, m->stream);
+  if (nvox > m->loud_n)
+    CK(cudaMemsetAsync(m->s_loud.as<uint8_t>() + m->loud_n, 0, (size_t)(nvox - m->loud_n), m->stream));
+  m->loud_n = nvox;
+  emit_views(m, added, coff);
   // the new views' ray records on the host, and their counters
   const int64_t hw_new = npix - m->npix_total;
   std::vector<RayMeta> hm((size_t)std::max<int64_t>(hw_new, 0));
@@ -1180,17 +1204,6 @@ void append_lists(mrf_map* m) {
       if (t.joinable()) t.join();
     }
   } joiner{lists_thread};
-  // loud voxels: the old views' stay flagged (those of views retired since the
-  // last full build too: a quiet voxel taken for a loud one only costs its
-  // pairs' preparation), the new views add theirs from the emit pass's ids
-  const int64_t nvox = m->n_bricks * kBrickVox;
-  m->s_loud.reserve((size_t)std::max<int64_t>(nvox, 1), true, m->stream);
-  if (nvox > m->loud_n)
-    CK(cudaMemsetAsync(m->s_loud.as<uint8_t>() + m->loud_n, 0, (size_t)(nvox - m->loud_n), m->stream));
-  m->loud_n = nvox;
-  for (int c : added)
-    CK(launch_loud_voxels(m->meta.as<RayMeta>() + m->views[c].pix_base, view_pixels(m->views[c]),
-                          m->s_vox.as<uint32_t>(), m->scratch_base, m->s_loud.as<uint8_t>(), m->stream));
   // an old view's quiet pairs (numbered after its loud ones) must all stay
   // quiet: where one became loud, the view prepares every pair
   m->s_k1.reserve(64, false, m->stream);

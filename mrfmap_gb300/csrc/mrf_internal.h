@@ -90,17 +90,36 @@ cudaError_t launch_fill_new_voxels(float* L, float* belief, int64_t v0, int64_t 
 cudaError_t launch_set_points(const Geom& g, const float* pts, const float* occ, int64_t n,
                               float* belief, cudaStream_t s);
 
-// traversal: count pass (counts padded to multiples of 4), then emit pass
-// (pix_off: their exclusive scan and total)
-cudaError_t launch_trace_count(const Geom& g, const Pose& P, const float* depth, uint32_t* counts, int* err,
-                               cudaStream_t s);
+// Traversal of several views in one launch (a small view fills a fraction of
+// the SMs with rays that take as long as a large view's): count pass (counts
+// padded to multiples of 4, a zero behind each view's, the totals added to
+// *total), then emit pass (pix_off: the scan of all counts; loud: voxels with
+// a dynamic incidence flagged; counters: kRayCounters totals added).
+constexpr int kTraceBatch = 16;
+struct TraceView {
+  Geom g;
+  Pose P;
+  const float* depth;
+  uint32_t* counts;                // rows * cols + 1
+  unsigned long long* total;
+  const uint32_t* pix_off;         // rows * cols + 1, relative to pix_off[0]
+  uint32_t inc_base;
+  RayMeta* meta;
+  uint32_t* vox;                   // the view's lists
+  float *len, *mu;
+  unsigned long long* counters;
+};
+struct TraceBatch {
+  TraceView v[kTraceBatch];
+  uint32_t first[kTraceBatch + 1];  // first block of each view
+  int n;
+};
+cudaError_t launch_trace_count(const TraceView* views, int n, int* err, cudaStream_t s);
+cudaError_t launch_trace_emit(const TraceView* views, int n, uint8_t* loud, int* err, cudaStream_t s);
 // pixels of a view whose rays may cross one of the bricks in slots b0..b1
 // (mask[pix] = 1; *all = 1 when every pixel must be checked)
 cudaError_t launch_brick_footprint(const Geom& g, const Pose& P, const int* coord, uint32_t b0, uint32_t b1,
                                    uint8_t* mask, int* all, cudaStream_t s);
-cudaError_t launch_trace_emit(const Geom& g, const Pose& P, const float* depth,
-                              const uint32_t* pix_off, uint32_t inc_base, RayMeta* meta,
-                              uint32_t* inc_vox, float* inc_len, float* inc_mu, int* err, cudaStream_t s);
 // the pairs of a view (mrf_build.cu): first incidence per voxel and brick;
 // voxel counts of the bricks in order; the pairs' numbers (table: first
 // incidences in, pair numbers out); the incidences' pairs, static lengths per
@@ -129,10 +148,6 @@ cudaError_t launch_run_stats(const uint32_t* dpair, const uint32_t* dseg, const 
                              uint32_t nrun, const float* len, const float* mu,
                              const unsigned long long* static_len, uint32_t pair_base, float* cum, uint32_t* ndyn,
                              float* hit, uint32_t* long_list, cudaStream_t s);
-// voxels with a dynamic incidence in any view (vox[k]: the voxel of
-// incidence vox_base + k), and the pairs on them
-cudaError_t launch_loud_voxels(const RayMeta* meta, int64_t npix, const uint32_t* vox, uint32_t vox_base,
-                               uint8_t* loud, cudaStream_t s);
 // flag[v] = 1 for the voxels of the given pairs past the length gate (no reset)
 cudaError_t launch_mark_active(const uint32_t* pair_vox, const float* cum, uint32_t np, uint8_t* flag,
                                cudaStream_t s);
@@ -293,12 +308,11 @@ cudaError_t launch_fill_f32(float* p, int64_t n, float v, cudaStream_t s);
 cudaError_t launch_max_abs_diff(const float* a, const float* b, int64_t n, uint32_t* out,
                                 cudaStream_t s);
 cudaError_t launch_fill_u32(uint32_t* p, int64_t n, uint32_t v, cudaStream_t s);
-// *out = sum of n u32 values, in 64 bits
-cudaError_t launch_sum_u32(const uint32_t* v, int64_t n, unsigned long long* out, cudaStream_t s);
-// per-view ray-record counters (k_ray_counters): out[0..kRayCounters) zeroed
-// on the stream, then summed over meta[0..n)
+// per-view totals of the ray records: Pre incidences, rays with any, Post
+// incidences, dynamic Post incidences (those from k_dyn on), rays in BP, their
+// Pre incidences, and their Pre incidences from the quiet-prefix boundary
+// (k_dyn rounded down to 4) on
 constexpr int kRayCounters = 7;
-cudaError_t launch_ray_counters(const RayMeta* meta, int64_t n, unsigned long long* out, cudaStream_t s);
 // out2[0] = pairs past the length gate, out2[1] = distinct voxels they
 // reach (flag: nvox bytes of scratch)
 cudaError_t launch_touch_counts(const uint32_t* pair_vox, const float* cum, uint32_t np, uint8_t* flag,
