@@ -1786,7 +1786,7 @@ void likelihood_dev(mrf_map* m, const Pose& P, const float* depth_clean, float* 
                     float* sum_dev, const Geom* cam = nullptr) {
   Geom g = cam ? *cam : m->g;
   g.brick_slot = m->d_slot.as<int>();
-  int nb = likelihood_blocks(g);
+  const int nb = likelihood_blocks(g, m->num_sms);
   m->s_part.reserve((size_t)nb * 8, false, m->stream);
   const float* bel = m->d_belief.as<float>();
   if (m->n_bricks == 0) {
@@ -1794,7 +1794,7 @@ void likelihood_dev(mrf_map* m, const Pose& P, const float* depth_clean, float* 
     m->s_dense.reserve(4, false, m->stream);
     bel = m->s_dense.as<float>();
   }
-  CK(launch_likelihood(g, P, depth_clean, bel, img_dev, m->s_part.as<double>(), nb, m->stream));
+  CK(launch_likelihood(g, P, depth_clean, bel, img_dev, m->s_part.as<double>(), m->num_sms, m->stream));
   CK(launch_reduce_partials(m->s_part.as<double>(), nb, sum_dev, m->stream));
 }
 
@@ -2678,7 +2678,7 @@ static mrf_status render_impl(mrf_map* m, int mode, const Pose& P, const float* 
       bel = m->s_dense.as<float>();
     }
     CK(launch_render(mode, g, P, depth_clean_dev, bel, threshold, m->s_img.as<float>(),
-                     reinterpret_cast<unsigned long long*>(m->s_part.p), m->stream));
+                     reinterpret_cast<unsigned long long*>(m->s_part.p), m->num_sms, m->stream));
     unsigned long long h[4] = {0, 0, 0, 0};
     CK(cudaMemcpyAsync(h, m->s_part.p, 32, cudaMemcpyDeviceToHost, m->stream));
     if (out_img)

@@ -23,7 +23,7 @@ __device__ __forceinline__ float fd(float a, float b) { return __fdiv_rn(a, b); 
 // several bricks a few metres out, and lanes that enter and leave their bricks
 // at different steps wait for one another (15 of 32 active); the tile's rays
 // mostly share a brick.
-constexpr int kTileX = 8, kTileY = 4;
+template <int kTileX = 8, int kTileY = 4>
 __device__ __forceinline__ int tile_pixel(int rows, int cols, int64_t tile, int lane) {
   const int tx = (cols + kTileX - 1) / kTileX;
   const int x = (int)(tile % tx) * kTileX + lane % kTileX;
@@ -337,6 +337,35 @@ __device__ __forceinline__ float dda_cross(Dda& r, const Geom& g, const Ray& ray
   dda_next_brick(r, g, px, py);
   steps = n;
   return te;
+}
+
+// The current voxel's coordinates as floats, from the boundaries: behind the
+// next one on an axis that counts up, at it on one that counts down, and fixed
+// (the boundary is INFINITY) on an axis the ray does not move along.
+struct Corner {
+  float ux, uy, uz, fx, fy, fz;
+  __device__ __forceinline__ explicit Corner(const Dda& r) {
+    ux = r.sx > 0.0f ? -1.0f : 0.0f;
+    uy = r.sy > 0.0f ? -1.0f : 0.0f;
+    uz = r.sz > 0.0f ? -1.0f : 0.0f;
+    fx = r.sx == 0.0f ? (float)(8 * r.kx + (int)(r.loc >> 8 & 7)) : INFINITY;
+    fy = r.sy == 0.0f ? (float)(8 * r.ky + (int)(r.loc >> 4 & 7)) : INFINITY;
+    fz = r.sz == 0.0f ? (float)(8 * r.kz + (int)(r.loc & 7)) : INFINITY;
+  }
+  __device__ __forceinline__ float x(const Dda& r) const { return fminf(r.bx + ux, fx); }
+  __device__ __forceinline__ float y(const Dda& r) const { return fminf(r.by + uy, fy); }
+  __device__ __forceinline__ float z(const Dda& r) const { return fminf(r.bz + uz, fz); }
+};
+
+// Walks on to the next active brick: its slot, -1 at the end of the ray.
+__device__ __forceinline__ int dda_next_active(Dda& r, const Geom& g, const Ray& ray) {
+  while (r.alive && r.guard > 0) {
+    const int slot = g.brick_slot[r.lin];
+    if (slot >= 0) return slot;
+    int steps;
+    dda_cross(r, g, ray, steps);
+  }
+  return -1;
 }
 
 __device__ __forceinline__ int64_t brick_lin(const Geom& g, int vx, int vy, int vz) {

@@ -75,6 +75,16 @@ constexpr uint32_t kNoVoxel = 0xFFFFFFFFu;  // padding incidences
 // tiles of a rows x cols image in the traversal kernels (a warp each)
 __host__ __device__ inline int64_t pixel_tiles(int rows, int cols) { return (int64_t)((cols + 7) / 8) * ((rows + 3) / 4); }
 
+// A ray's bricks are dealt to kSplit lanes where an image alone leaves the SMs
+// short of warps: a ray takes as long as its voxels' dependent steps.  Every
+// lane walks all bricks, whole bricks at a time, and the lanes' parts are put
+// together in brick order; the walks cost more than they hide once there are
+// about ten warps per SM.  Likelihood, us with 1 and 4 lanes on loaded maps at
+// 2 to 4 cm: 160x120 134 and 86, 240x180 179 and 145, 320x240 270 and 320;
+// expected depth 180 and 142, 232 and 215, 363 and 422 (host calls).
+constexpr int kSplit = 4;
+inline bool split_rays(int rows, int cols, int num_sms) { return pixel_tiles(rows, cols) <= (int64_t)10 * num_sms; }
+
 // ---- launchers (stream-ordered; return cudaError_t of the launch) --------
 cudaError_t launch_clean_depth(const float* in, float* out, int rows, int cols, cudaStream_t s);
 cudaError_t launch_activate(const Geom& g, const Pose& P, const float* depth, int policy,
@@ -325,8 +335,8 @@ cudaError_t launch_scatter_const(const uint32_t* idx, uint32_t n, float v, float
 
 // likelihood and readback
 cudaError_t launch_likelihood(const Geom& g, const Pose& P, const float* depth, const float* belief,
-                              float* out_img, double* partials, int nblocks, cudaStream_t s);
-int likelihood_blocks(const Geom& g);
+                              float* out_img, double* partials, int num_sms, cudaStream_t s);
+int likelihood_blocks(const Geom& g, int num_sms);
 cudaError_t launch_reduce_partials(const double* partials, int n, float* out_sum, cudaStream_t s);
 
 // per-voxel records of one pixel's ray (debug probe; out zeroed by the caller,
@@ -336,7 +346,7 @@ cudaError_t launch_pixel_diag(const Geom& g, const Pose& P, const float* belief,
 // evaluation renders (mode 0-3, see mrf_render.cu); counts: 4 zeroed u64
 cudaError_t launch_render(int mode, const Geom& g, const Pose& P, const float* depth,
                           const float* belief, float thresh, float* out, unsigned long long* counts,
-                          cudaStream_t s);
+                          int num_sms, cudaStream_t s);
 
 // Map state the likelihood needs, for entry points outside mrf_capi.cu: the
 // map's geometry (device brick table and sensor tables), its belief field

@@ -26,6 +26,24 @@ __global__ void __launch_bounds__(kLikeThreads)
   if (threadIdx.x == 0) partials[blockIdx.x] = t;
 }
 
+// the same with kSplit lanes per pixel: a warp's tile is 4 x 2
+__global__ void __launch_bounds__(kLikeThreads)
+    k_likelihood_split(Geom g, Pose P, const float* __restrict__ depth, const float* __restrict__ belief,
+                       float* __restrict__ out_img, double* __restrict__ partials) {
+  const int lane = threadIdx.x & 31, sub = lane % kSplit;
+  const int pix = tile_pixel<4, 2>(g.rows, g.cols, (blockIdx.x * (int64_t)kLikeThreads + threadIdx.x) >> 5, lane / kSplit);
+  float val = 0.0f;
+  if (pix >= 0) {
+    const float d = depth[pix];
+    const unsigned mask = ((1u << kSplit) - 1u) << (lane - sub);
+    if (d > 0.0f) val = likelihood_pixel_split(g, P, belief, pix, d, mask, sub);
+    if (out_img && sub == 0) out_img[pix] = val;
+  }
+  double t = like_block_sum<kLikeThreads>(sub == 0 ? (double)val : 0.0);
+  if (threadIdx.x == 0) partials[blockIdx.x] = t;
+}
+static_assert(kSplit * 4 * 2 == 32, "a warp per tile");
+
 __global__ void k_reduce_partials(const double* __restrict__ partials, int n, float* out) {
   __shared__ double sh[256];
   double v = 0.0;
@@ -42,14 +60,20 @@ __global__ void k_reduce_partials(const double* __restrict__ partials, int n, fl
 
 }  // namespace
 
-int likelihood_blocks(const Geom& g) {
+int likelihood_blocks(const Geom& g, int num_sms) {
   constexpr int kTiles = kLikeThreads / 32;
-  return (int)((pixel_tiles(g.rows, g.cols) + kTiles - 1) / kTiles);
+  const int64_t tiles = split_rays(g.rows, g.cols, num_sms) ? (int64_t)((g.cols + 3) / 4) * ((g.rows + 1) / 2)
+                                                            : pixel_tiles(g.rows, g.cols);
+  return (int)((tiles + kTiles - 1) / kTiles);
 }
 
 cudaError_t launch_likelihood(const Geom& g, const Pose& P, const float* depth, const float* belief,
-                              float* out_img, double* partials, int nblocks, cudaStream_t s) {
-  k_likelihood<<<nblocks, kLikeThreads, 0, s>>>(g, P, depth, belief, out_img, partials);
+                              float* out_img, double* partials, int num_sms, cudaStream_t s) {
+  const int nblocks = likelihood_blocks(g, num_sms);
+  if (split_rays(g.rows, g.cols, num_sms))
+    k_likelihood_split<<<nblocks, kLikeThreads, 0, s>>>(g, P, depth, belief, out_img, partials);
+  else
+    k_likelihood<<<nblocks, kLikeThreads, 0, s>>>(g, P, depth, belief, out_img, partials);
   return cudaGetLastError();
 }
 

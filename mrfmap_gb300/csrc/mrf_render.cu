@@ -31,6 +31,7 @@ __device__ float render_pixel(const Geom& g, const Pose& P, const float* __restr
   bool run_open = false;
   Dda r;
   if (dda_init(r, g, ray)) {
+    const Corner corner(r);
     while (r.alive && r.guard > 0) {
       // simple accuracy: a brick that ends past the return is a miss
       if (kMode == 2 && run_open && s_last >= d) return 0.0f;
@@ -51,10 +52,9 @@ __device__ float render_pixel(const Geom& g, const Pose& P, const float* __restr
       // the brick's voxels, the lanes of a warp together
       bool left;
       do {
-        const uint32_t xyz = r.loc;
         const float p = bel[dda_local(r)];
+        const float vx = corner.x(r), vy = corner.y(r), vz = corner.z(r);
         float l, tin, te;
-        const int kx = r.kx, ky = r.ky, kz = r.kz;
         left = dda_step(r, g, l, tin, te);
         const float s = fm(te, ray.mult);
         s_last = s;
@@ -66,12 +66,10 @@ __device__ float render_pixel(const Geom& g, const Pose& P, const float* __restr
         }
         if (kMode == 0 && p != 0.0f) {
           const float dA = log_free(p) * l;
-          const float dv = Vprev * -expm1f(dA);
+          const float dv = Vprev * -expm1_free(dA);
           A += dA;
           Vprev = expf(A);
           // z-depth of the voxel's corner (the GVDB atlas-to-world position)
-          const float vx = (float)(8 * kx + (int)(xyz >> 8)), vy = (float)(8 * ky + (int)(xyz >> 4 & 7)),
-                      vz = (float)(8 * kz + (int)(xyz & 7));
           const float zc = fabsf(P.m[2] * (vx - ray.o[0]) + P.m[6] * (vy - ray.o[1]) + P.m[10] * (vz - ray.o[2])) *
                            g.res;
           sum += dv * zc;
@@ -99,6 +97,64 @@ __device__ float render_pixel(const Geom& g, const Pose& P, const float* __restr
   }
   if (kMode == 2) return (run_open && s_last >= d) ? 0.0f : -1.0f;
   return (float)occ;
+}
+
+// Expected depth by kSplit lanes per pixel, as likelihood_pixel_split: a
+// brick's depth sum relative to the visibility at its start.
+__device__ __forceinline__ float depth_pixel_split(const Geom& g, const Pose& P, const float* __restrict__ belief,
+                                                   int pix, unsigned mask, int sub) {
+  Ray ray;
+  ray_setup(g, P, pix % g.cols, pix / g.cols, ray);
+  float A = 0.0f, sum = 0.0f;
+  Dda r;
+  const bool in = dda_init(r, g, ray);
+  if (!in) r = Dda{};
+  const Corner corner(r);
+  int slot = in ? dda_next_active(r, g, ray) : -1;
+  auto skip = [&](int n) {
+    for (int k = 0; k < n && slot >= 0; ++k) {
+      int steps;
+      dda_cross(r, g, ray, steps);
+      slot = dda_next_active(r, g, ray);
+    }
+  };
+  skip(sub);
+  while (__any_sync(mask, slot >= 0)) {
+    float a = 0.0f, rel = 0.0f;
+    if (slot >= 0) {
+      const float* __restrict__ bel = belief + (int64_t)slot * kBrickVox;
+      bool left;
+      do {
+        const float p = bel[dda_local(r)];
+        const float vx = corner.x(r), vy = corner.y(r), vz = corner.z(r);
+        float l, tin, te;
+        left = dda_step(r, g, l, tin, te);
+        if (p != 0.0f) {
+          const float dA = log_free(p) * l;
+          rel += expf(a) * -expm1_free(dA) *
+                 (fabsf(P.m[2] * (vx - ray.o[0]) + P.m[6] * (vy - ray.o[1]) + P.m[10] * (vz - ray.o[2])) * g.res);
+          a += dA;
+        }
+      } while (!left && r.guard > 0);
+      slot = dda_next_active(r, g, ray);
+      skip(kSplit - 1);
+    }
+    float total;
+    sum += expf(A + split_prefix(a, mask, sub, total)) * rel;
+    A += total;
+    if (A < -69.0f && split_sum(sum, mask) > 1e-18f) break;
+  }
+  return split_sum(sum, mask) / (1.0f - expf(A) + kFEps);
+}
+
+__global__ void __launch_bounds__(kRenderThreads)
+    k_depth_split(Geom g, Pose P, const float* __restrict__ belief, float* __restrict__ out) {
+  const int lane = threadIdx.x & 31, sub = lane % kSplit;
+  const int pix =
+      tile_pixel<4, 2>(g.rows, g.cols, (blockIdx.x * (int64_t)kRenderThreads + threadIdx.x) >> 5, lane / kSplit);
+  if (pix < 0) return;
+  const float v = depth_pixel_split(g, P, belief, pix, ((1u << kSplit) - 1u) << (lane - sub), sub);
+  if (sub == 0) out[pix] = v;
 }
 
 template <int kMode>
@@ -191,7 +247,13 @@ cudaError_t launch_pixel_diag(const Geom& g, const Pose& P, const float* belief,
 
 cudaError_t launch_render(int mode, const Geom& g, const Pose& P, const float* depth,
                           const float* belief, float thresh, float* out, unsigned long long* counts,
-                          cudaStream_t s) {
+                          int num_sms, cudaStream_t s) {
+  if (mode == 0 && split_rays(g.rows, g.cols, num_sms)) {
+    const int64_t warps = (int64_t)((g.cols + 3) / 4) * ((g.rows + 1) / 2);
+    k_depth_split<<<(unsigned)((warps + kRenderThreads / 32 - 1) / (kRenderThreads / 32)), kRenderThreads, 0, s>>>(
+        g, P, belief, out);
+    return cudaGetLastError();
+  }
   constexpr int kTiles = kRenderThreads / 32;
   const int nb = (int)((pixel_tiles(g.rows, g.cols) + kTiles - 1) / kTiles);
   switch (mode) {
