@@ -73,6 +73,43 @@ __global__ void __launch_bounds__(kPrepThreads)
   }
 }
 
+// the same over the views' loud pairs only (Jacobi, later iterations of a
+// call): element i of the views' loud ranges back to back (prefix[v] the first
+// of view v, whose pairs start at base[v])
+__global__ void __launch_bounds__(kPrepThreads)
+    k_pair_prepare_loud(const uint32_t* __restrict__ pair_vox, const float* __restrict__ m,
+                        const float* __restrict__ L, float* __restrict__ lnq, __half* __restrict__ lnq16,
+                        float* __restrict__ dm, const uint32_t* __restrict__ prefix,
+                        const uint32_t* __restrict__ base, int nv) {
+  const uint32_t n = prefix[nv];
+  const uint32_t i0 = blockIdx.x * (kPrepThreads * kPrepPer) + threadIdx.x;
+  int v = 0;
+  for (int hi = nv; hi - v > 1;) {
+    const int mid = (v + hi) >> 1;
+    if (prefix[mid] <= i0) v = mid;
+    else hi = mid;
+  }
+  float eta[kPrepPer];
+  uint32_t p[kPrepPer];
+#pragma unroll
+  for (int k = 0; k < kPrepPer; ++k) {
+    const uint32_t i = i0 + k * kPrepThreads;
+    while (v + 1 < nv && i >= prefix[v + 1]) ++v;
+    p[k] = base[v] + (i - prefix[v]);
+    eta[k] = i < n ? L[pair_vox[p[k]]] - m[p[k]] : 0.0f;
+  }
+#pragma unroll
+  for (int k = 0; k < kPrepPer; ++k) {
+    if (i0 + k * kPrepThreads >= n) break;
+    const float qq = clampf(1.0f / (1.0f + expf(eta[k])), kFEps, 1.0f - kFEps);
+    if (lnq16)
+      lnq16[p[k]] = __float2half_rn(logf(qq));
+    else
+      lnq[p[k]] = logf(qq);
+    dm[p[k]] = __int_as_float(0x7fc00000);
+  }
+}
+
 // ---- ray messages ----------------------------------------------------------
 // A group of kG lanes per ray, 32 / kG rays per warp.  Each lane owns kE = 4
 // consecutive incidences of a chunk of 4 kG (ray offsets are padded to
@@ -600,13 +637,14 @@ __global__ void k_ray_keys(const RayMeta* __restrict__ meta, uint32_t n, uint32_
 // in flight) together with the segment bounds of the pairs the tile
 // touches; each thread then sums whole pairs sequentially from shared memory
 // (a fixed order) and updates them.  A block owns the pairs that start in its
-// tile: the rest of the one that crosses into the next tile is summed by the
-// whole block (lane-strided, then a fixed tree), so no tile waits for another
-// and no second kernel adds carries (4.5 us per view and iteration, 14 % of
-// an iteration on 160x120 views).  A pair of thousands of messages takes its
-// block a few more rounds.
+// tile, so no tile waits for another and no second kernel adds carries (4.5 us
+// per view and iteration, 14 % of an iteration on 160x120 views).  It gathers
+// kAhead positions of the next tile too, which ends nearly every pair that
+// crosses over; a longer one is summed on by the whole block (lane-strided,
+// then a fixed tree).
 constexpr int kTileThreads = 256;
 constexpr int kTile = 4 * kTileThreads;
+constexpr uint32_t kAhead = 32;
 
 // a dynamic run's update with its old message mo and the voxel's old total
 // Lo already loaded (the gate c > kCumLenGate already checked)
@@ -664,14 +702,14 @@ __global__ void __launch_bounds__(kTileThreads, kTwo ? 5 : 8)
                   const uint32_t* __restrict__ seg, const uint32_t* __restrict__ tile_first,
                   uint32_t k0, uint32_t k1, uint32_t p_end, const uint4* __restrict__ drun, float* __restrict__ m, float* __restrict__ L,
                   float* __restrict__ dm, int jacobi) {
-  __shared__ float sv[kTile];
+  __shared__ float sv[kTile + kAhead];
   __shared__ uint32_t sseg[kTile + 2];
-  __shared__ float open_sum, open_m, open_L, part[kTileThreads / 32];
-  __shared__ uint4 open_run;
+  __shared__ float open_sum, part[kTileThreads / 32];
   const int t = threadIdx.x;
   const uint32_t base = k0 + blockIdx.x * kTile;
   const uint32_t n = min((uint32_t)kTile, k1 - base);
   const uint32_t end = base + n;
+  const uint32_t ahead = min(kAhead, k1 - end);
   const uint32_t pf = tile_first[blockIdx.x];
   // a tile touches at most n pairs: their starts and the next pair's start
   const uint32_t nseg = min(n + 1, p_end - pf) + 1;
@@ -692,6 +730,7 @@ __global__ void __launch_bounds__(kTileThreads, kTwo ? 5 : 8)
     uint32_t i = j * kTileThreads + t;
     if (i < n) sv[i] = pl[perm[base + i]];
   }
+  if (t < ahead) sv[n + t] = pl[perm[end + t]];
   for (uint32_t q = t; q < nseg; q += kTileThreads) sseg[q] = seg[pf + q];
   const bool gate0 = pre && __uint_as_float(r0.z) > kCumLenGate;
   if (gate0) {
@@ -703,21 +742,14 @@ __global__ void __launch_bounds__(kTileThreads, kTwo ? 5 : 8)
     mo1 = m[r1.x];
     if (!jacobi) Lo1 = L[r1.y];
   }
-  if (t == kTileThreads - 1) {
-    // the pair at the next tile's first position, which this block may own
-    const uint4 r = drun[last];
-    open_run = r;
-    open_m = m[r.x];
-    open_L = jacobi ? 0.0f : L[r.y];
-  }
   __syncthreads();
   for (uint32_t q = t; q < n && pf + q < p_end && sseg[q] < end; q += kTileThreads) {
     const uint32_t s0 = sseg[q], s1 = sseg[q + 1];
     if (s0 < base) continue;  // an earlier tile's
-    const uint32_t a = s0 - base, b = min(s1, end) - base;
+    const uint32_t a = s0 - base, b = min(s1, end + ahead) - base;
     float acc = 0.0f;
     for (uint32_t i = a; i < b; ++i) acc += sv[i];
-    if (s1 > end) {  // the last one
+    if (s1 > end + ahead) {  // the last one
       open_sum = acc;
       continue;
     }
@@ -729,19 +761,18 @@ __global__ void __launch_bounds__(kTileThreads, kTwo ? 5 : 8)
       apply_run(drun[pf + q], acc, m, L, dm, jacobi);
     }
   }
-  // the pair that goes on behind the tile, if it starts in it
+  // a pair that goes on for longer, if it starts in the tile
   const uint32_t ql = last - pf;
-  if (sseg[ql] < base || sseg[ql] >= end || sseg[ql + 1] <= end) return;
+  if (sseg[ql] < base || sseg[ql] >= end || sseg[ql + 1] <= end + ahead) return;
   const uint32_t s1 = sseg[ql + 1];
   float x = 0.0f;
-  for (uint32_t i = end + t; i < s1; i += kTileThreads) x += pl[perm[i]];
+  for (uint32_t i = end + ahead + t; i < s1; i += kTileThreads) x += pl[perm[i]];
   x = warp_sum(x);
   if ((t & 31) == 0) part[t >> 5] = x;
   __syncthreads();  // open_sum and the warps' parts
   if (t == 0) {
     for (int w = 1; w < kTileThreads / 32; ++w) x += part[w];
-    if (__uint_as_float(open_run.z) > kCumLenGate)
-      apply_run_loaded(open_run, open_m, open_L, open_sum + x, m, L, dm, jacobi);
+    apply_run(drun[last], open_sum + x, m, L, dm, jacobi);
   }
 }
 
@@ -965,18 +996,28 @@ __global__ void k_fill(float* p, int64_t n, float v) {
   if (i < n) p[i] = v;
 }
 
+// sort keys of the pairs' voxels: voxels without a dynamic incidence behind
+// the others (top: a bit above every voxel id)
+__global__ void k_voxel_keys(const uint32_t* __restrict__ pair_vox, uint32_t n, const uint8_t* __restrict__ loud,
+                             uint32_t top, uint32_t* __restrict__ key) {
+  const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p < n) key[p] = pair_vox[p] | (loud[pair_vox[p]] ? 0u : top);
+}
+
 __global__ void k_vflag(const uint32_t* __restrict__ sk, uint32_t n, uint32_t* __restrict__ flag) {
   uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k < n) flag[k] = (k == 0 || sk[k] != sk[k - 1]) ? 1u : 0u;
 }
 
 __global__ void k_vassign(const uint32_t* __restrict__ sk, const uint32_t* __restrict__ flag,
-                          const uint32_t* __restrict__ scan, uint32_t n, uint32_t* __restrict__ vvox,
-                          uint32_t* __restrict__ vseg) {
+                          const uint32_t* __restrict__ scan, uint32_t n, uint32_t top,
+                          uint32_t* __restrict__ vvox, uint32_t* __restrict__ vseg, uint32_t* __restrict__ n_loud) {
   uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n || !flag[k]) return;
-  vvox[scan[k]] = sk[k];
+  vvox[scan[k]] = sk[k] & ~top;
   vseg[scan[k]] = k;
+  // the loud voxels end where the first other one begins
+  if (top && (sk[k] & top) && (k == 0 || !(sk[k - 1] & top))) *n_loud = scan[k];
 }
 
 __global__ void k_scatter_const(const uint32_t* __restrict__ idx, uint32_t n, float v,
@@ -1019,6 +1060,14 @@ cudaError_t launch_pair_prepare(const BpArrays& a, uint32_t p0, uint32_t p1, int
   return cudaGetLastError();
 }
 
+
+cudaError_t launch_pair_prepare_loud(const BpArrays& a, const uint32_t* prefix, const uint32_t* base, int nv,
+                                     uint32_t n, cudaStream_t s) {
+  if (!n) return cudaSuccess;
+  k_pair_prepare_loud<<<blocks(n, kPrepThreads * kPrepPer), kPrepThreads, 0, s>>>(
+      a.pair_vox, a.pair_m, a.L, a.pair_lnq, a.half_streams ? a.pair_lnq16 : nullptr, a.pair_dm, prefix, base, nv);
+  return cudaGetLastError();
+}
 
 // ray-kernel variants: (id, resident-block target, load policy, chunk
 // prefetch, schedule: 0 longest first, 1 SM regions)
@@ -1292,10 +1341,17 @@ cudaError_t launch_vflag(const uint32_t* sk, uint32_t n, uint32_t* flag, cudaStr
   return cudaGetLastError();
 }
 
-cudaError_t launch_vassign(const uint32_t* sk, const uint32_t* flag, const uint32_t* scan,
-                           uint32_t n, uint32_t* vvox, uint32_t* vseg, cudaStream_t s) {
+cudaError_t launch_voxel_keys(const uint32_t* pair_vox, uint32_t n, const uint8_t* loud, uint32_t top,
+                              uint32_t* key, cudaStream_t s) {
   if (!n) return cudaSuccess;
-  k_vassign<<<blocks(n, 256), 256, 0, s>>>(sk, flag, scan, n, vvox, vseg);
+  k_voxel_keys<<<blocks(n, 256), 256, 0, s>>>(pair_vox, n, loud, top, key);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_vassign(const uint32_t* sk, const uint32_t* flag, const uint32_t* scan, uint32_t n, uint32_t top,
+                           uint32_t* vvox, uint32_t* vseg, uint32_t* n_loud, cudaStream_t s) {
+  if (!n) return cudaSuccess;
+  k_vassign<<<blocks(n, 256), 256, 0, s>>>(sk, flag, scan, n, top, vvox, vseg, n_loud);
   return cudaGetLastError();
 }
 

@@ -235,7 +235,9 @@ struct mrf_map {
   bool has_base = false;
   // jacobi voxel CSR
   DBuf vseg, vpairs, vvox;
-  uint32_t n_vvox = 0;
+  uint32_t n_vvox = 0, n_vvox_loud = 0;  // its voxels; those with a dynamic incidence come first
+  DBuf loud_ranges;                      // the views' loud pairs: prefix (V + 1), first pair (V)
+  uint32_t n_loud_pairs = 0;
   int jacobi_version = -1;
   // scratch
   DBuf s_pf, s_ps, s_flags, s_ind, s_scan, s_tmp, s_counts, s_offs, s_vox, s_k0, s_k1, s_v0, s_v1,
@@ -1317,16 +1319,21 @@ void build_jacobi_csr(mrf_map* m) {
   m->s_k1.reserve((size_t)np * 4 + 4, false, m->stream);
   m->s_v1.reserve((size_t)np * 4 + 4, false, m->stream);
   if (np == 0) {
-    m->n_vvox = 0;
+    m->n_vvox = m->n_vvox_loud = m->n_loud_pairs = 0;
     m->jacobi_version = m->built_version;
     return;
   }
   CK(launch_iota(m->s_v0.as<uint32_t>(), np, m->stream));
   int bits = 1;
   while (bits < 32 && ((uint64_t)1 << bits) <= (uint64_t)(m->n_bricks * kBrickVox)) ++bits;
+  // voxels with a dynamic incidence first, where a key has a bit left to say so
+  const uint32_t top = bits < 32 ? 1u << bits : 0u;
+  if (top) ++bits;
   size_t t = sort_temp_bytes(np, bits);
   m->s_tmp.reserve(t, false, m->stream);
-  CK(sort_pairs_u32(m->s_tmp.p, t, m->pair_vox.as<uint32_t>(), m->s_k1.as<uint32_t>(),
+  CK(launch_voxel_keys(m->pair_vox.as<uint32_t>(), np, m->s_loud.as<uint8_t>(), top, m->s_k0.as<uint32_t>(),
+                       m->stream));
+  CK(sort_pairs_u32(m->s_tmp.p, t, m->s_k0.as<uint32_t>(), m->s_k1.as<uint32_t>(),
                     m->s_v0.as<uint32_t>(), m->vpairs.as<uint32_t>(), np, bits, m->stream));
   CK(launch_vflag(m->s_k1.as<uint32_t>(), np, m->s_k0.as<uint32_t>(), m->stream));
   CK(cudaMemsetAsync(m->s_k0.as<uint32_t>() + np, 0, 4, m->stream));
@@ -1335,10 +1342,22 @@ void build_jacobi_csr(mrf_map* m) {
   CK(exclusive_scan_u32(m->s_tmp.p, t2, m->s_k0.as<uint32_t>(), m->s_v1.as<uint32_t>(), np + 1,
                         m->stream));
   uint32_t nv = read1(m, m->s_v1.as<uint32_t>() + np);
-  CK(launch_vassign(m->s_k1.as<uint32_t>(), m->s_k0.as<uint32_t>(), m->s_v1.as<uint32_t>(), np,
-                    m->vvox.as<uint32_t>(), m->vseg.as<uint32_t>(), m->stream));
+  m->s_delta.reserve(64, false, m->stream);
+  CK(launch_fill_u32(m->s_delta.as<uint32_t>(), 1, nv, m->stream));
+  CK(launch_vassign(m->s_k1.as<uint32_t>(), m->s_k0.as<uint32_t>(), m->s_v1.as<uint32_t>(), np, top,
+                    m->vvox.as<uint32_t>(), m->vseg.as<uint32_t>(), m->s_delta.as<uint32_t>(), m->stream));
   CK(cudaMemcpyAsync(m->vseg.as<uint32_t>() + nv, &np, 4, cudaMemcpyHostToDevice, m->stream));
-  sync(m);
+  // the views' loud pair ranges
+  const size_t V = m->views.size();
+  std::vector<uint32_t> lr(2 * V + 1, 0u);
+  for (size_t c = 0; c < V; ++c) {
+    lr[c + 1] = lr[c] + m->views[c].n_loud;
+    lr[V + 1 + c] = m->views[c].pair_base;
+  }
+  m->loud_ranges.reserve(lr.size() * 4, false, m->stream);
+  CK(cudaMemcpyAsync(m->loud_ranges.p, lr.data(), lr.size() * 4, cudaMemcpyHostToDevice, m->stream));
+  m->n_loud_pairs = lr[V];
+  m->n_vvox_loud = read1(m, m->s_delta.as<uint32_t>());
   m->n_vvox = nv;
   m->jacobi_version = m->built_version;
 }
@@ -1540,7 +1559,11 @@ void enqueue_iteration(mrf_map* m, const BpArrays& a, bool jacobi, int fix, int 
   } else {
     uint32_t P = (uint32_t)m->n_pairs;
     prof.begin(0);
-    CK(launch_pair_prepare(a, 0, P, 1, m->stream));
+    if (phase >= 2)
+      CK(launch_pair_prepare_loud(a, m->loud_ranges.as<uint32_t>(), m->loud_ranges.as<uint32_t>() + V + 1, V,
+                                  m->n_loud_pairs, m->stream));
+    else
+      CK(launch_pair_prepare(a, 0, P, 1, m->stream));
     prof.end();
     prof.begin(1);
     // the queues of all views are contiguous: one launch over all rays
@@ -1552,8 +1575,9 @@ void enqueue_iteration(mrf_map* m, const BpArrays& a, bool jacobi, int fix, int 
     if (first) CK(launch_static_pairs(a, 0, P, 1, m->stream));
     prof.end();
     prof.begin(3);
+    // quiet voxels move with the static pairs only, in the first iteration
     CK(launch_voxel_apply(m->vseg.as<uint32_t>(), m->vpairs.as<uint32_t>(), m->vvox.as<uint32_t>(),
-                          m->n_vvox, m->pair_dm.as<float>(), m->d_L.as<float>(), m->stream));
+                          phase >= 2 ? m->n_vvox_loud : m->n_vvox, m->pair_dm.as<float>(), m->d_L.as<float>(), m->stream));
     prof.end();
     launches += 4 + (first ? 1 : 0);
   }
@@ -1770,7 +1794,7 @@ void destroy_bufs(mrf_map* m) {
                  &m->ray_order, &m->ray_queue, &m->region_q, &m->rstart, &m->rcounters, &m->counters, &m->tile_first,
                  &m->lbase, &m->lsingle, &m->lprefix, &m->queue_ids, &m->region_ids, &m->loud_off,
                  &m->loud, &m->quiet_ray,
-                 &m->vseg, &m->vpairs, &m->vvox, &m->vox_active, &m->d_Lbase, &m->inc_len16, &m->pair_q16,
+                 &m->vseg, &m->vpairs, &m->vvox, &m->loud_ranges, &m->vox_active, &m->d_Lbase, &m->inc_len16, &m->pair_q16,
                  &m->s_pf, &m->s_ps,
                  &m->s_flags, &m->s_ind, &m->s_scan,
                  &m->s_q0, &m->s_q1, &m->s_q2, &m->s_q3, &m->s_q4, &m->s_bf, &m->s_bc, &m->s_first, &m->s_len, &m->s_loud,

@@ -228,6 +228,10 @@ struct BpArrays {
 uint32_t pair_update_tiles(uint32_t n);
 cudaError_t launch_pair_prepare(const BpArrays& a, uint32_t p0, uint32_t p1, int jacobi,
                                 cudaStream_t s);
+// the loud pairs of nv views (prefix: their counts summed, nv + 1; base: first
+// pair of each view), Jacobi
+cudaError_t launch_pair_prepare_loud(const BpArrays& a, const uint32_t* prefix, const uint32_t* base, int nv,
+                                     uint32_t n, cudaStream_t s);
 // ray-kernel variants (register budget x load policy; identical arithmetic)
 int ray_bp_variants();
 // resident blocks per SM of a variant of the persistent ray kernel (queried once)
@@ -328,8 +332,12 @@ constexpr int kRayCounters = 7;
 cudaError_t launch_touch_counts(const uint32_t* pair_vox, const float* cum, uint32_t np, uint8_t* flag,
                                 int64_t nvox, unsigned long long* out2, cudaStream_t s);
 cudaError_t launch_vflag(const uint32_t* sk, uint32_t n, uint32_t* flag, cudaStream_t s);
-cudaError_t launch_vassign(const uint32_t* sk, const uint32_t* flag, const uint32_t* scan,
-                           uint32_t n, uint32_t* vvox, uint32_t* vseg, cudaStream_t s);
+// voxel CSR: keys with the voxels without a dynamic incidence behind the
+// others; the first of those goes to *n_loud (untouched if there is none)
+cudaError_t launch_voxel_keys(const uint32_t* pair_vox, uint32_t n, const uint8_t* loud, uint32_t top,
+                              uint32_t* key, cudaStream_t s);
+cudaError_t launch_vassign(const uint32_t* sk, const uint32_t* flag, const uint32_t* scan, uint32_t n, uint32_t top,
+                           uint32_t* vvox, uint32_t* vseg, uint32_t* n_loud, cudaStream_t s);
 cudaError_t launch_scatter_const(const uint32_t* idx, uint32_t n, float v, float* dense,
                                  cudaStream_t s);
 
