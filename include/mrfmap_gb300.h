@@ -162,6 +162,16 @@ MRF_API mrf_status mrf_test_brick_footprint(mrf_map* map, int view_id, int64_t b
 MRF_API mrf_status mrf_test_region_lists(const int32_t* records, int64_t n_pix, int regions, int share,
                                          uint32_t* home, int64_t* n_home, uint32_t* starts, uint32_t* left,
                                          int64_t* n_left);
+/* The same schedule by the device path that builds take, on map's stream, of
+ * n_views views (at most 64) with equal shares of the records.  queue: each
+ * view's BP rays longest first, the views back to back; lists: each view's
+ * home rays and then its leftovers, the views back to back; starts: n_views
+ * rows of regions + 1 positions in lists; lefts: the n_views first leftovers,
+ * then n_views pairs {0, number of leftovers}.  queue and lists must hold
+ * n_pix entries. */
+MRF_API mrf_status mrf_test_region_lists_device(mrf_map* map, const int32_t* records, int64_t n_pix, int n_views,
+                                                int regions, int share, uint32_t* lists, uint32_t* starts,
+                                                uint32_t* lefts, uint32_t* queue);
 /* Test hook, no reference counterpart: the next build that appends new
  * views' lists fails with `status` once their pairs are built (a host-side
  * stand-in for a failing allocation or CUDA call part-way through).  An

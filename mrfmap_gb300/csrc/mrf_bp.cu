@@ -532,18 +532,6 @@ __global__ void __launch_bounds__(kRayWarps * 32, kMinBlocks)
   }
 }
 
-// queue records: queue[i] = meta[base + order[i]] (order: view-local ray
-// indices, longest first)
-__global__ void k_ray_queue(const RayMeta* __restrict__ meta, const uint32_t* __restrict__ order,
-                            uint32_t n, RayMeta* __restrict__ queue, uint32_t* __restrict__ ids,
-                            uint32_t id_base) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) {
-    queue[i] = meta[order[i]];
-    ids[i] = id_base + order[i];
-  }
-}
-
 // The static prefix of each queued ray of one view (rays r0..r0+n of the
 // pixel arrays; a warp per ray): the loud incidences in [0, k4) -- those
 // whose pair is among the view's first n_loud, the pairs on voxels with a
@@ -621,13 +609,148 @@ __global__ void k_quiet_prefix(const RayMeta* __restrict__ meta, uint32_t r_firs
 }
 
 // ray queue of one build: active rays sorted by decreasing length
-__global__ void k_ray_keys(const RayMeta* __restrict__ meta, uint32_t n, uint32_t* __restrict__ keys,
-                           uint32_t* __restrict__ vals) {
-  uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= n) return;
+// The views of a batch: view v has pixels pix[v] .. pix[v + 1] (from the
+// batch's first) and act[v + 1] - act[v] rays in BP.
+__device__ __forceinline__ uint32_t batch_view(const uint32_t* first, uint32_t n, uint32_t i) {
+  uint32_t lo = 0, hi = n;
+  while (hi - lo > 1) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (first[mid] <= i) lo = mid;
+    else hi = mid;
+  }
+  return lo;
+}
+// the last view that begins at or before i is the one that holds it: of views
+// without rays, which share their successor's first, it is the successor
+__device__ __forceinline__ uint32_t ray_at(const QueueBatch& b, uint32_t v, uint32_t a) {
+  return b.pix[v] + (a - b.act[v]);
+}
+
+// sort keys (by view, longest first, rays outside BP last), pixel numbers
+// and, for the rays in BP, n_pre
+__global__ void k_ray_keys(const __grid_constant__ QueueBatch b, const RayMeta* __restrict__ meta,
+                           uint32_t* __restrict__ keys, uint32_t* __restrict__ vals, uint32_t* __restrict__ work) {
+  const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x, n = b.pix[b.views];
+  if (r > n) return;
+  if (r == n) {
+    work[n] = 0u;
+    return;
+  }
   const RayMeta me = meta[r];
-  keys[r] = ray_in_bp(me) ? 0xFFFFu - me.n_pre : 0x10000u;  // rays left out sort last
+  const bool in = ray_in_bp(me);
+  keys[r] = batch_view(b.pix, b.views, r) << 17 | (in ? 0xFFFFu - me.n_pre : 0x10000u);
   vals[r] = r;
+  work[r] = in ? me.n_pre : 0u;
+}
+
+// The queues of a batch of views from their sorted rays.
+//
+// The queue of all rays: each view's rays longest first.  The SM-affine region
+// lists (see region_lists, which states them on the host): each ray's region
+// from the work before its pixel, a stable sort by region, which leaves a
+// region's rays longest first, the work before a ray inside its region, which
+// says whether it is a home ray, and one scan that places each view's home
+// rays (by region) and behind them its leftovers (longest first).  A dozen
+// passes over a few hundred thousand rays at launch latency, which is why
+// views go through them together (5 views of 160x120 one by one: 0.5 ms).  With
+// the ray records copied down, the lists made by host threads and copied up, an
+// appended 640x480 frame took 1.5 ms longer and a build of twelve 4 ms.
+__global__ void k_region_keys(const __grid_constant__ QueueBatch b, const RayMeta* __restrict__ meta,
+                              const uint32_t* __restrict__ sorted, const uint32_t* __restrict__ before, uint32_t R,
+                              uint32_t* __restrict__ region, uint32_t* __restrict__ rank,
+                              RayMeta* __restrict__ queue, uint32_t* __restrict__ ids, uint32_t id_base) {
+  const uint32_t a = blockIdx.x * blockDim.x + threadIdx.x;
+  if (a >= b.act[b.views]) return;
+  const uint32_t v = batch_view(b.act, b.views, a), pix = sorted[ray_at(b, v, a)];
+  const uint32_t w0 = before[b.pix[v]];
+  const uint64_t work = max(before[b.pix[v + 1]] - w0, 1u);
+  region[a] = v * R + (uint32_t)min((uint64_t)(R - 1), (uint64_t)(before[pix] - w0) * R / work);
+  rank[a] = a;
+  if (queue) {
+    queue[a] = meta[pix];
+    ids[a] = id_base + pix;
+  }
+}
+
+// by region: bounds[x], the first ray of a region >= x (x <= views R), and
+// the rays' work, from the sort keys of their ranks
+__global__ void k_region_bounds(const __grid_constant__ QueueBatch b, const uint32_t* __restrict__ region,
+                                const uint32_t* __restrict__ rank, const uint32_t* __restrict__ keys, uint32_t R,
+                                uint32_t* __restrict__ bounds, uint32_t* __restrict__ work) {
+  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x, n = b.act[b.views];
+  if (k > n) return;
+  const uint32_t hi = k == n ? b.views * R : region[k];
+  for (uint32_t x = k == 0 ? 0u : region[k - 1] + 1u; x <= hi; ++x) bounds[x] = k;
+  uint32_t w = 0u;
+  if (k < n) {
+    const uint32_t a = rank[k], v = batch_view(b.act, b.views, a);
+    w = 0xFFFFu - (keys[ray_at(b, v, a)] & 0x1FFFFu);
+  }
+  work[k] = w;
+}
+
+// Flags of a view, at twice its first ray: its rays by region that are home
+// rays, then its rays by length that are leftovers.
+__global__ void k_region_home(const __grid_constant__ QueueBatch b, const uint32_t* __restrict__ region,
+                              const uint32_t* __restrict__ rank, const uint32_t* __restrict__ before,
+                              const uint32_t* __restrict__ bounds, uint32_t share, uint32_t* __restrict__ flag) {
+  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x, n = b.act[b.views];
+  if (k > n) return;
+  if (k == n) {
+    flag[2 * (size_t)n] = 0u;
+    return;
+  }
+  const uint32_t v = batch_view(b.act, b.views, k);
+  const uint32_t x = region[k], lo = before[bounds[x]], hi = before[bounds[x + 1]];
+  const bool home = (uint64_t)(before[k] - lo) * 100u < (uint64_t)(hi - lo) * share;
+  flag[(size_t)b.act[v] + k] = home;
+  flag[(size_t)b.act[v + 1] + rank[k]] = !home;
+}
+
+// the lists, and each view's row of region starts (R and the end of its home
+// rays), first leftover and {0, leftovers}
+__global__ void k_region_emit(const __grid_constant__ QueueBatch b, const RayMeta* __restrict__ meta,
+                              const uint32_t* __restrict__ sorted, const uint32_t* __restrict__ rank,
+                              const uint32_t* __restrict__ place, const uint32_t* __restrict__ bounds, uint32_t R,
+                              uint32_t at, uint32_t id_base, RayMeta* __restrict__ queue, uint32_t* __restrict__ ids,
+                              uint32_t* __restrict__ rstart, uint32_t* __restrict__ lbase,
+                              uint32_t* __restrict__ lsingle) {
+  const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x, n = b.act[b.views];
+  if (e < b.views * (R + 1)) {
+    const uint32_t v = e / (R + 1), r = e - v * (R + 1);
+    // a bound at the view's end: the first of its leftovers' flags
+    const uint32_t k = r < R ? bounds[v * R + r] : b.act[v + 1];
+    const uint32_t p = place[(size_t)b.act[v] + k];
+    rstart[e] = at + p;
+    if (r == R) {
+      lbase[v] = at + p;
+      lsingle[2 * v] = 0u;
+      lsingle[2 * v + 1] = b.act[v + 1] - p;
+    }
+  }
+  if (e >= 2 * n || place[e + 1] == place[e]) return;
+  const uint32_t v = batch_view(b.act, b.views, e >> 1);
+  const uint32_t i = e - 2 * b.act[v], m = b.act[v + 1] - b.act[v];
+  const uint32_t a = i < m ? rank[b.act[v] + i] : b.act[v] + (i - m);
+  const uint32_t pix = sorted[ray_at(b, v, a)];
+  queue[at + place[e]] = meta[pix];
+  ids[at + place[e]] = id_base + pix;
+}
+
+// prefix of the views' leftover counts (lsingle[2 c + 1]), V + 1 entries; one warp
+__global__ void k_leftover_prefix(const uint32_t* __restrict__ lsingle, uint32_t V, uint32_t* __restrict__ prefix) {
+  uint32_t run = 0;
+  for (uint32_t c0 = 0; c0 <= V; c0 += 32) {
+    const uint32_t c = c0 + threadIdx.x;
+    const uint32_t v = c < V ? lsingle[2 * c + 1] : 0u;
+    uint32_t incl = v;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t u = __shfl_up_sync(kFull, incl, o);
+      if ((int)threadIdx.x >= o) incl += u;
+    }
+    if (c <= V) prefix[c] = run + incl - v;
+    run += __shfl_sync(kFull, incl, 31);
+  }
 }
 
 // Pair update: a load-balanced segmented reduction over the pair-grouped
@@ -1142,17 +1265,46 @@ cudaError_t launch_ray_bp(const BpArrays& a, const RayWork& w, int fix_reset, in
   return cudaGetLastError();
 }
 
-cudaError_t launch_ray_keys(const RayMeta* meta, uint32_t n, uint32_t* keys, uint32_t* vals,
+cudaError_t launch_ray_keys(const QueueBatch& b, const RayMeta* meta, uint32_t* keys, uint32_t* vals, uint32_t* work,
                             cudaStream_t s) {
-  if (!n) return cudaSuccess;
-  k_ray_keys<<<blocks(n, 256), 256, 0, s>>>(meta, n, keys, vals);
+  k_ray_keys<<<blocks((uint64_t)b.pix[b.views] + 1, 256), 256, 0, s>>>(b, meta, keys, vals, work);
   return cudaGetLastError();
 }
 
-cudaError_t launch_ray_queue(const RayMeta* meta, const uint32_t* order, uint32_t n, RayMeta* queue,
-                             uint32_t* ids, uint32_t id_base, cudaStream_t s) {
-  if (!n) return cudaSuccess;
-  k_ray_queue<<<blocks(n, 256), 256, 0, s>>>(meta, order, n, queue, ids, id_base);
+cudaError_t launch_region_keys(const QueueBatch& b, const RayMeta* meta, const uint32_t* sorted,
+                               const uint32_t* before, uint32_t R, uint32_t* region, uint32_t* rank, RayMeta* queue,
+                               uint32_t* ids, uint32_t id_base, cudaStream_t s) {
+  if (!b.act[b.views]) return cudaSuccess;
+  k_region_keys<<<blocks(b.act[b.views], 256), 256, 0, s>>>(b, meta, sorted, before, R, region, rank, queue, ids,
+                                                           id_base);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_region_bounds(const QueueBatch& b, const uint32_t* region, const uint32_t* rank,
+                                 const uint32_t* keys, uint32_t R, uint32_t* bounds, uint32_t* work, cudaStream_t s) {
+  k_region_bounds<<<blocks((uint64_t)b.act[b.views] + 1, 256), 256, 0, s>>>(b, region, rank, keys, R, bounds, work);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_region_home(const QueueBatch& b, const uint32_t* region, const uint32_t* rank,
+                               const uint32_t* before, const uint32_t* bounds, uint32_t share, uint32_t* flag,
+                               cudaStream_t s) {
+  k_region_home<<<blocks((uint64_t)b.act[b.views] + 1, 256), 256, 0, s>>>(b, region, rank, before, bounds, share, flag);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_region_emit(const QueueBatch& b, const RayMeta* meta, const uint32_t* sorted, const uint32_t* rank,
+                               const uint32_t* place, const uint32_t* bounds, uint32_t R, uint32_t at,
+                               uint32_t id_base, RayMeta* queue, uint32_t* ids, uint32_t* rstart, uint32_t* lbase,
+                               uint32_t* lsingle, cudaStream_t s) {
+  const uint64_t rays = 2 * (uint64_t)b.act[b.views], rows = (uint64_t)b.views * (R + 1);
+  k_region_emit<<<blocks(rays > rows ? rays : rows, 256), 256, 0, s>>>(b, meta, sorted, rank, place, bounds, R, at,
+                                                                      id_base, queue, ids, rstart, lbase, lsingle);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_leftover_prefix(const uint32_t* lsingle, uint32_t V, uint32_t* prefix, cudaStream_t s) {
+  k_leftover_prefix<<<1, 32, 0, s>>>(lsingle, V, prefix);
   return cudaGetLastError();
 }
 

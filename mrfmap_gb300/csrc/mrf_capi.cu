@@ -23,7 +23,6 @@
 #include <atomic>
 #include <cmath>
 #include <mutex>
-#include <thread>
 #include <cstdio>
 #include <cstring>
 #include <string>
@@ -151,7 +150,6 @@ struct View {
   uint32_t dperm_base = 0, n_dperm = 0;   // pair-grouped positions of the dynamic incidences
   uint32_t dpair_base = 0, n_dpairs = 0;  // runs of dynamic incidences (one per pair)
   uint32_t order_base = 0, n_active = 0;  // ray queue (longest first)
-  uint32_t left_base = 0, n_left = 0;     // leftover queue of the SM-affine schedule
   uint32_t n_loud = 0;                    // pairs on voxels with a dynamic incidence (numbered first)
   uint32_t tile_base = 0;                 // first pair of each pair-update tile
   bool retired = false;                   // out of the window: no lists, no pairs, no depth
@@ -216,7 +214,7 @@ struct mrf_map {
   std::vector<View> views;
   // arenas
   DBuf meta, inc_pair, inc_len, inc_mu, inc_pl, pair_vox, pair_m, pair_cum, pair_stat, pair_ndyn, pair_hit,
-      pair_q, pair_dm, dperm, s_q0, s_q1, s_q2, s_q3, s_q4, s_bf, s_bc, s_first, s_len, s_loud, dpair, dseg, drun, ray_order, ray_queue, region_q, rstart, rcounters, counters,
+      pair_q, pair_dm, dperm, s_q0, s_q1, s_q2, s_q3, s_q4, s_bf, s_bc, s_first, s_len, s_loud, s_rg, dpair, dseg, drun, ray_queue, region_q, rstart, rcounters, counters,
       tile_first, lbase, lsingle, lprefix, queue_ids, region_ids, loud_off, loud, quiet_ray;
   uint32_t jac_tile_base = 0;
   int64_t n_inc = 0, n_pairs = 0, n_dperm = 0, n_dpairs = 0;
@@ -403,18 +401,13 @@ void rebuild(mrf_map* m) {
 
 // ---- per-view pieces of a build ------------------------------------------
 
-// The counters of the given views' rays (s_vcnt, from the emit pass), and the
-// records of pixels [hm_base, hm_base + hm.size()) copied to the host for the
-// region lists: one synchronisation.
-void ray_records_and_counters(mrf_map* m, const std::vector<int>& views, int64_t hm_base,
-                              std::vector<RayMeta>& hm) {
+// The counters of the given views' rays (s_vcnt, from the emit pass): one
+// synchronisation.
+void ray_counters(mrf_map* m, const std::vector<int>& views) {
   const size_t K = (size_t)kRayCounters;
   std::vector<unsigned long long> hc(views.size() * K, 0ull);
   if (!hc.empty())
     CK(cudaMemcpyAsync(hc.data(), m->s_vcnt.p, hc.size() * 8, cudaMemcpyDeviceToHost, m->stream));
-  if (!hm.empty())
-    CK(cudaMemcpyAsync(hm.data(), m->meta.as<RayMeta>() + hm_base, hm.size() * sizeof(RayMeta),
-                       cudaMemcpyDeviceToHost, m->stream));
   sync(m);
   check_device_err(m);
   for (size_t k = 0; k < views.size(); ++k) {
@@ -551,10 +544,11 @@ void view_pairs(mrf_map* m, int c, int64_t& pair_total, int64_t& dperm_total, in
 // the view's leftover queue (longest first) that the blocks drain
 // afterwards, which evens out the regions' finishing times (the home share,
 // 75 % unless mrf_set_home_share or mrf_autotune_home_share chose another;
-// it moves rays between warps only, never a result).  Built on
-// the host in linear time: a counting sort by length feeds the regions'
-// buckets in order, so each bucket is longest first.  Pixel indices are
-// absolute (v.pix_base + i); starts are positions in home.
+// it moves rays between warps only, never a result).  A build makes
+// them on the device (view_regions); this is the same on the host, in linear
+// time, to check that by: a counting sort by length feeds the regions' buckets
+// in order, so each bucket is longest first.  Pixel indices are absolute
+// (v.pix_base + i); starts are positions in home.
 struct RegionLists {
   std::vector<uint32_t> home, left, starts;
 };
@@ -607,141 +601,123 @@ void region_lists(const View& v, const RayMeta* vm, int R, int64_t share, Region
     if (!is_home[i]) out.left.push_back((uint32_t)(v.pix_base + i));
 }
 
-// region lists of several views in parallel host threads (at most one per
-// core, the views taken in turn); hm holds the ray records of every view in
-// `views` at their pix_base
-void region_lists_parallel(mrf_map* m, const std::vector<int>& views, const std::vector<RayMeta>& hm,
-                           int64_t hm_base, std::vector<RegionLists>& lists) {
-  const int R = std::max(1, m->num_sms);
-  const int nv = (int)views.size();
-  const int nt = std::max(1, std::min<int>(nv, (int)std::thread::hardware_concurrency()));
-  std::atomic<int> next{0};
-  std::vector<std::thread> pool;
-  std::vector<char> failed((size_t)nv, 0);
-  for (int t = 0; t < nt; ++t)
-    pool.emplace_back([&] {
-      for (int k = next++; k < nv; k = next++) {
-        try {
-          const View& v = m->views[views[k]];
-          region_lists(v, hm.data() + (v.pix_base - hm_base), R, m->home_share, lists[(size_t)views[k]]);
-        } catch (...) {
-          failed[(size_t)k] = 1;
-        }
-      }
-    });
-  for (auto& t : pool) t.join();
-  for (char f : failed)
-    if (f) fail(MRF_ERR_OOM, "host memory for the region queues");
+// The queues of a batch of views whose ray records begin at meta: each view's
+// rays in BP longest first at queue, queue_ids (null: not wanted), and the
+// region lists as blocks [home rays][leftovers] of the views from position
+// `at` of region_q, region_ids on; per view the R region starts and the end of
+// its home rays at rstart (R + 1), its first leftover at lbase, {0, leftovers}
+// at lsingle.  id_base: number of the batch's first pixel.
+void batch_queues(mrf_map* m, const QueueBatch& b, const RayMeta* meta, uint32_t R, uint32_t share, uint32_t at,
+                  uint32_t id_base, RayMeta* queue, uint32_t* queue_ids, RayMeta* region_q, uint32_t* region_ids,
+                  uint32_t* rstart, uint32_t* lbase, uint32_t* lsingle) {
+  const cudaStream_t st = m->stream;
+  const uint32_t hw = b.pix[b.views], act = b.act[b.views];
+  const size_t p = (size_t)hw + 1, n = (size_t)act;
+  auto bits_for = [](uint64_t count) {
+    int bits = 1;
+    while (bits < 32 && ((uint64_t)1 << bits) < count) ++bits;
+    return bits;
+  };
+  const int kb = 17 + (b.views > 1 ? bits_for(b.views) : 0), rb = bits_for((uint64_t)b.views * R);
+  const size_t t = std::max(std::max(sort_temp_bytes(hw, kb), sort_temp_bytes(act, rb)),
+                            std::max(scan_temp_bytes(hw + 1), scan_temp_bytes(2 * act + 1)));
+  m->s_tmp.reserve(t, false, st);
+  m->s_k0.reserve(2 * p * 4, false, st);
+  m->s_k1.reserve(p * 4, false, st);
+  m->s_v0.reserve(p * 4, false, st);
+  m->s_v1.reserve(p * 4, false, st);
+  m->s_rg.reserve((6 * n + 4 + (size_t)b.views * R + 1) * 4, false, st);
+  uint32_t* k0 = m->s_k0.as<uint32_t>();
+  uint32_t* keys = m->s_k1.as<uint32_t>();
+  uint32_t* v0 = m->s_v0.as<uint32_t>();  // pixel numbers, then the work before each pixel
+  uint32_t* sorted = m->s_v1.as<uint32_t>();
+  CK(launch_ray_keys(b, meta, k0, v0, k0 + p, st));
+  if (hw) CK(sort_pairs_u32(m->s_tmp.p, t, k0, keys, v0, sorted, hw, kb, st));
+  CK(exclusive_scan_u32(m->s_tmp.p, t, k0 + p, v0, hw + 1, st));
+  uint32_t* f = m->s_rg.as<uint32_t>();  // regions and ranks, then the flags
+  uint32_t* w = f + 2 * n + 2;           // work and the work before, then the places
+  uint32_t* region = w + 2 * n + 2;
+  uint32_t* rank = region + n;
+  uint32_t* bounds = rank + n;
+  CK(launch_region_keys(b, meta, sorted, v0, R, f, f + n, queue, queue_ids, id_base, st));
+  if (act) CK(sort_pairs_u32(m->s_tmp.p, t, f, region, f + n, rank, act, rb, st));
+  CK(launch_region_bounds(b, region, rank, keys, R, bounds, w, st));
+  CK(exclusive_scan_u32(m->s_tmp.p, t, w, w + n + 1, act + 1, st));
+  CK(launch_region_home(b, region, rank, w + n + 1, bounds, share, f, st));
+  CK(exclusive_scan_u32(m->s_tmp.p, t, f, w, 2 * act + 1, st));
+  CK(launch_region_emit(b, meta, sorted, rank, w, bounds, R, at, id_base, region_q, region_ids, rstart, lbase,
+                        lsingle, st));
 }
 
-// Per-view blocks [home rays][leftovers] of views (in that order) laid out
-// in region_q from position `at` on, their ray records gathered from meta;
-// per view: rstart row c*(R+1) (R region starts and the end of the home
-// block, absolute), lbase[c] (first leftover) and lsingle {0, n_left} at 2c.
-// Returns the end position.
-uint32_t region_blocks(mrf_map* m, const std::vector<int>& views, const std::vector<RegionLists>& lists,
-                       uint32_t at) {
-  const int R = std::max(1, m->num_sms);
-  const int V = (int)m->views.size();
-  m->rstart.reserve((size_t)V * (R + 1) * 4 + 4, true, m->stream);
-  m->lbase.reserve((size_t)V * 4 + 4, true, m->stream);
-  m->lsingle.reserve((size_t)V * 8 + 8, true, m->stream);
-  std::vector<uint32_t> pix;
-  // each view's row of region starts, leftover base and leftover counter
-  // pair, staged on the host until the synchronisation below
-  const size_t nv = views.size();
-  std::vector<uint32_t> rows(nv * ((size_t)R + 1)), lbs(nv), lss(2 * nv);
-  for (size_t k = 0; k < nv; ++k) {
-    const int c = views[k];
-    View& v = m->views[c];
-    const RegionLists& l = lists[(size_t)c];
-    uint32_t* row = rows.data() + k * ((size_t)R + 1);
-    const uint32_t b = at + (uint32_t)pix.size();
-    for (int r = 0; r < R; ++r) row[r] = b + (r < (int)l.starts.size() ? l.starts[(size_t)r] : 0u);
-    row[R] = b + (uint32_t)l.home.size();
-    v.left_base = b + (uint32_t)l.home.size();
-    v.n_left = (uint32_t)l.left.size();
-    pix.insert(pix.end(), l.home.begin(), l.home.end());
-    pix.insert(pix.end(), l.left.begin(), l.left.end());
-    lbs[k] = v.left_base;
-    lss[2 * k] = 0u;
-    lss[2 * k + 1] = v.n_left;
-    CK(cudaMemcpyAsync(m->rstart.as<uint32_t>() + (size_t)c * (R + 1), row, (size_t)(R + 1) * 4,
-                       cudaMemcpyHostToDevice, m->stream));
-    CK(cudaMemcpyAsync(m->lbase.as<uint32_t>() + c, &lbs[k], 4, cudaMemcpyHostToDevice, m->stream));
-    CK(cudaMemcpyAsync(m->lsingle.as<uint32_t>() + 2 * (size_t)c, &lss[2 * k], 8, cudaMemcpyHostToDevice,
-                       m->stream));
+// The queues of views c0 .. c1: ray queues from each view's order_base on
+// (`rays` false: they stay), region lists from position `at` of region_q.
+// Retired views get empty rows.  Views go in batches of up to kQueuePixels,
+// which bounds the scratch (44 bytes a pixel).  Returns the end position.
+constexpr int64_t kQueuePixels = 1 << 20;
+uint32_t view_queues(mrf_map* m, int c0, int c1, uint32_t at, bool rays) {
+  const uint32_t R = (uint32_t)std::max(1, m->num_sms);
+  for (int c = c0; c < c1;) {
+    const uint32_t first = (uint32_t)m->views[c].pix_base;
+    const uint32_t order = m->views[c].order_base;
+    QueueBatch b{};
+    const int from = c;
+    while (c < c1 && b.views < (uint32_t)kQueueViews) {
+      View& v = m->views[c];
+      const int64_t end = v.pix_base + view_pixels(v) - first;
+      if (b.views && end > kQueuePixels) break;
+      v.n_active = view_pixels(v) ? (uint32_t)v.c_nrays_bp : 0u;  // the rays in BP (ray_in_bp)
+      if (rays) v.order_base = order + b.act[b.views];
+      b.pix[b.views] = (uint32_t)(v.pix_base - first);  // behind the pixels of a view that was retired since
+      b.act[b.views + 1] = b.act[b.views] + v.n_active;
+      b.pix[++b.views] = (uint32_t)end;
+      ++c;
+    }
+    batch_queues(m, b, m->meta.as<RayMeta>() + first, R, (uint32_t)m->home_share, at, first,
+                 rays ? m->ray_queue.as<RayMeta>() + order : nullptr,
+                 rays ? m->queue_ids.as<uint32_t>() + order : nullptr, m->region_q.as<RayMeta>(),
+                 m->region_ids.as<uint32_t>(), m->rstart.as<uint32_t>() + (size_t)from * (R + 1),
+                 m->lbase.as<uint32_t>() + from, m->lsingle.as<uint32_t>() + 2 * (size_t)from);
+    at += b.act[b.views];
+    if (rays && c < c1) m->views[c].order_base = order + b.act[b.views];
   }
-  const uint32_t end = at + (uint32_t)pix.size();
-  m->region_q.reserve(std::max<size_t>(end, 1) * sizeof(RayMeta), true, m->stream);
-  m->region_ids.reserve(std::max<size_t>(end, 1) * 4, true, m->stream);
-  if (!pix.empty()) {
-    m->ray_order.reserve(pix.size() * 4, false, m->stream);
-    CK(cudaMemcpyAsync(m->ray_order.p, pix.data(), pix.size() * 4, cudaMemcpyHostToDevice, m->stream));
-    CK(launch_ray_queue(m->meta.as<RayMeta>(), m->ray_order.as<uint32_t>(), (uint32_t)pix.size(),
-                        m->region_q.as<RayMeta>() + at, m->region_ids.as<uint32_t>() + at, 0u, m->stream));
-  }
-  sync(m);  // the host staging vectors go out of scope
-  return end;
+  return at;
 }
 
-// the leftover prefix of every view (V + 1 entries) for a launch over all
-// views (Jacobi)
-void leftover_prefix(mrf_map* m) {
-  const int V = (int)m->views.size();
-  std::vector<uint32_t> pre((size_t)V + 1, 0u);
-  for (int c = 0; c < V; ++c) pre[(size_t)c + 1] = pre[(size_t)c] + m->views[c].n_left;
-  m->lprefix.reserve(pre.size() * 4, false, m->stream);
-  CK(cudaMemcpyAsync(m->lprefix.p, pre.data(), pre.size() * 4, cudaMemcpyHostToDevice, m->stream));
-  sync(m);
+// room for `rays` queue records and `regions` records of the region lists,
+// the records so far kept
+void queue_room(mrf_map* m, size_t rays, size_t regions) {
+  const size_t V = m->views.size(), R = (size_t)std::max(1, m->num_sms);
+  m->ray_queue.reserve(std::max<size_t>(rays, 1) * sizeof(RayMeta), true, m->stream);
+  m->queue_ids.reserve(std::max<size_t>(rays, 1) * 4, true, m->stream);
+  m->region_q.reserve(std::max<size_t>(regions, 1) * sizeof(RayMeta), true, m->stream);
+  m->region_ids.reserve(std::max<size_t>(regions, 1) * 4, true, m->stream);
+  m->rstart.reserve(V * (R + 1) * 4 + 4, true, m->stream);
+  m->lbase.reserve(V * 4 + 4, true, m->stream);
+  m->lsingle.reserve(V * 8 + 8, true, m->stream);
+  m->counters.reserve((V + 1) * 4, false, m->stream);
+  m->rcounters.reserve((2 * V * R + 2 * V + 2) * 4, false, m->stream);
 }
 
-// the region blocks of every built view again, from their ray records (the
-// home share changed); the incidence lists stay as they are.  The caller
-// drops the captured graphs.
+// the leftover prefix of the V views (V + 1 entries) for a launch over all
+// of them (Jacobi)
+void leftover_prefix(mrf_map* m, uint32_t V) {
+  m->lprefix.reserve(((size_t)V + 1) * 4, false, m->stream);
+  CK(launch_leftover_prefix(m->lsingle.as<uint32_t>(), V, m->lprefix.as<uint32_t>(), m->stream));
+}
+
+bool can_append(const mrf_map* m);
+
+// the region lists of every built view again, from their ray records (the
+// home share changed); the incidence lists stay as they are.  Nothing to do
+// where the next build is a full one: it makes them.  The caller drops the
+// captured graphs.
 void rebuild_regions(mrf_map* m) {
   const int B = m->built_views;
   if (m->built_version < 0 || B == 0 || m->npix_total == 0) return;
-  std::vector<RayMeta> hm((size_t)m->npix_total);
-  CK(cudaMemcpyAsync(hm.data(), m->meta.p, hm.size() * sizeof(RayMeta), cudaMemcpyDeviceToHost, m->stream));
+  if (m->built_version != m->version && !can_append(m)) return;
+  m->region_end = view_queues(m, 0, B, 0u, false);
+  leftover_prefix(m, (uint32_t)B);
   sync(m);
-  std::vector<int> live, built;
-  for (int c = 0; c < B; ++c) {
-    built.push_back(c);
-    if (!m->views[c].retired) live.push_back(c);
-  }
-  std::vector<RegionLists> lists(m->views.size());
-  region_lists_parallel(m, live, hm, 0, lists);
-  for (int c : built)
-    if (m->views[c].retired) {
-      m->views[c].n_left = 0;
-      m->views[c].left_base = 0;
-    }
-  m->region_end = region_blocks(m, built, lists, 0u);
-  leftover_prefix(m);
-}
-
-// view c's active rays longest first (17-bit key radix sort on the GPU),
-// their records copied into queue order at ray_queue + v.order_base
-void view_ray_queue(mrf_map* m, int c) {
-  View& v = m->views[c];
-  const int64_t hw = view_pixels(v);
-  const int64_t act = hw ? v.c_nrays_bp : 0;  // the rays in BP (ray_in_bp)
-  v.n_active = (uint32_t)act;
-  if (hw == 0) return;
-  m->s_k0.reserve((size_t)hw * 4 + 4, false, m->stream);
-  m->s_k1.reserve((size_t)hw * 4 + 4, false, m->stream);
-  m->s_v0.reserve((size_t)hw * 4 + 4, false, m->stream);
-  m->s_v1.reserve((size_t)hw * 4 + 4, false, m->stream);
-  CK(launch_ray_keys(m->meta.as<RayMeta>() + v.pix_base, (uint32_t)hw, m->s_k0.as<uint32_t>(),
-                     m->s_v0.as<uint32_t>(), m->stream));
-  size_t t = sort_temp_bytes((uint32_t)hw, 17);
-  m->s_tmp.reserve(t, false, m->stream);
-  CK(sort_pairs_u32(m->s_tmp.p, t, m->s_k0.as<uint32_t>(), m->s_k1.as<uint32_t>(), m->s_v0.as<uint32_t>(),
-                    m->s_v1.as<uint32_t>(), (uint32_t)hw, 17, m->stream));
-  CK(launch_ray_queue(m->meta.as<RayMeta>() + v.pix_base, m->s_v1.as<uint32_t>(), (uint32_t)act,
-                      m->ray_queue.as<RayMeta>() + v.order_base, m->queue_ids.as<uint32_t>() + v.order_base,
-                      (uint32_t)v.pix_base, m->stream));
 }
 
 // the statistics of the live views
@@ -990,62 +966,23 @@ void rebuild_lists(mrf_map* m, OldPairs& old) {
   CK(cudaMemsetAsync(m->s_loud.p, 0, (size_t)std::max<int64_t>(m->n_bricks * kBrickVox, 1), m->stream));
   m->loud_n = m->n_bricks * kBrickVox;
   emit_views(m, live, coff);
-  std::vector<RayMeta> hm((size_t)npix);
-  ray_records_and_counters(m, live, 0, hm);
+  ray_counters(m, live);
   for (View& v : m->views)
     if (v.retired) v.c_npre = v.c_nrays = v.c_npost = v.c_ndyn = v.c_nrays_bp = v.c_npre_bp = v.c_nfast_bp = 0;
-  // the region lists of the SM-affine schedule are host work on the ray
-  // records alone: built on host threads while the GPU builds the pairs
-  std::vector<RegionLists> lists((size_t)V);
-  bool lists_failed = false;
-  std::thread lists_thread([&] {
-    try {
-      region_lists_parallel(m, live, hm, 0, lists);
-    } catch (...) {
-      lists_failed = true;
-    }
-  });
   // 4. pairs per view
   int64_t pair_total = 0, dperm_total = 0, dpair_total = 0, nd_all = 0;
   for (int c : live) nd_all += m->views[c].c_ndyn;
-  try {
-    m->dperm.reserve((size_t)std::max<int64_t>(nd_all, 1) * 4, false, m->stream);
-    for (int c = 0; c < V; ++c) view_pairs(m, c, pair_total, dperm_total, dpair_total);
-  } catch (...) {
-    lists_thread.join();
-    throw;
-  }
-  lists_thread.join();
-  if (lists_failed) fail(MRF_ERR_OOM, "host memory for the region queues");
+  m->dperm.reserve((size_t)std::max<int64_t>(nd_all, 1) * 4, false, m->stream);
+  for (int c = 0; c < V; ++c) view_pairs(m, c, pair_total, dperm_total, dpair_total);
   // 5. ray queues: per view the active rays longest first, and the
-  //    SM-affine region blocks
+  //    SM-affine region lists
   {
-    m->ray_queue.reserve((size_t)std::max<int64_t>(npix, 1) * sizeof(RayMeta), false, m->stream);
-    m->queue_ids.reserve((size_t)std::max<int64_t>(npix, 1) * 4, false, m->stream);
-    int64_t base = 0;
-    for (int c = 0; c < V; ++c) {
-      View& v = m->views[c];
-      v.order_base = (uint32_t)base;
-      view_ray_queue(m, c);
-      base += v.n_active;
-    }
-    m->queue_end = base;
-    m->counters.reserve((size_t)(V + 1) * 4, false, m->stream);
-    const int R = std::max(1, m->num_sms);
-    m->nreg = (uint32_t)R;
-    m->rcounters.reserve(((size_t)2 * V * R + 2 * (size_t)V + 2) * 4, false, m->stream);
-    // retired views: empty rows
-    for (int c = 0; c < V; ++c) {
-      View& v = m->views[c];
-      if (v.retired) {
-        v.n_left = 0;
-        v.left_base = 0;
-      }
-    }
-    std::vector<int> all;
-    for (int c = 0; c < V; ++c) all.push_back(c);
-    m->region_end = region_blocks(m, all, lists, 0u);
-    leftover_prefix(m);
+    m->nreg = (uint32_t)std::max(1, m->num_sms);
+    queue_room(m, (size_t)npix, (size_t)npix);
+    if (V) m->views[0].order_base = 0u;
+    m->region_end = view_queues(m, 0, V, 0u, true);
+    m->queue_end = m->region_end;
+    leftover_prefix(m, (uint32_t)V);
   }
   m->n_inc = n_inc;
   m->n_pairs = pair_total;
@@ -1185,27 +1122,7 @@ void append_lists(mrf_map* m) {
     CK(cudaMemsetAsync(m->s_loud.as<uint8_t>() + m->loud_n, 0, (size_t)(nvox - m->loud_n), m->stream));
   m->loud_n = nvox;
   emit_views(m, added, coff);
-  // the new views' ray records on the host, and their counters
-  const int64_t hw_new = npix - m->npix_total;
-  std::vector<RayMeta> hm((size_t)std::max<int64_t>(hw_new, 0));
-  ray_records_and_counters(m, added, m->npix_total, hm);
-  // the new views' region lists: host work on their ray records, on host
-  // threads while the GPU builds their pairs
-  std::vector<RegionLists> lists((size_t)V);
-  bool lists_failed = false;
-  std::thread lists_thread([&] {
-    try {
-      region_lists_parallel(m, added, hm, m->npix_total, lists);
-    } catch (...) {
-      lists_failed = true;
-    }
-  });
-  struct Joiner {
-    std::thread& t;
-    ~Joiner() {
-      if (t.joinable()) t.join();
-    }
-  } joiner{lists_thread};
+  ray_counters(m, added);
   // an old view's quiet pairs (numbered after its loud ones) must all stay
   // quiet: where one became loud, the view prepares every pair
   m->s_k1.reserve(64, false, m->stream);
@@ -1228,34 +1145,17 @@ void append_lists(mrf_map* m) {
     m->test_append_fail = 0;
     fail(st, "append of the new views' lists: injected failure (mrf_test_fail_next_append)");
   }
-  // 5. ray queues and region blocks of the new views
+  // 5. ray queues and region lists of the new views
   {
     int64_t base = 0;
     for (int c = 0; c < m->built_views; ++c) base = std::max<int64_t>(base, (int64_t)m->views[c].order_base + m->views[c].n_active);
     base = std::max<int64_t>(base, m->queue_end);
-    m->ray_queue.reserve((size_t)std::max<int64_t>(base + hw_new, 1) * sizeof(RayMeta), true, m->stream);
-    m->queue_ids.reserve((size_t)std::max<int64_t>(base + hw_new, 1) * 4, true, m->stream);
-    for (int c = m->built_views; c < V; ++c) {
-      View& v = m->views[c];
-      v.order_base = (uint32_t)base;
-      view_ray_queue(m, c);
-      base += v.n_active;
-    }
-    m->queue_end = base;
-    const int R = std::max(1, m->num_sms);
-    m->counters.reserve((size_t)(V + 1) * 4, false, m->stream);
-    m->rcounters.reserve(((size_t)2 * V * R + 2 * (size_t)V + 2) * 4, false, m->stream);
-    lists_thread.join();
-    if (lists_failed) fail(MRF_ERR_OOM, "host memory for the region queues");
-    std::vector<int> newv;
-    for (int c = m->built_views; c < V; ++c) {
-      if (m->views[c].retired) {
-        m->views[c].n_left = 0;
-        m->views[c].left_base = 0;
-      }
-      newv.push_back(c);
-    }
-    m->region_end = region_blocks(m, newv, lists, m->region_end);
+    const int64_t hw_new = npix - m->npix_total;
+    queue_room(m, (size_t)(base + hw_new), (size_t)m->region_end + (size_t)hw_new);
+    const uint32_t region0 = m->region_end;
+    if (m->built_views < V) m->views[m->built_views].order_base = (uint32_t)base;
+    m->region_end = view_queues(m, m->built_views, V, region0, true);
+    m->queue_end = base + (m->region_end - region0);
   }
   m->n_inc = n_inc;
   m->n_pairs = pair_total;
@@ -1383,13 +1283,15 @@ void ensure_compact(mrf_map* m) {
 // memory grows with them: no per-frame pass reads a retired view's data.
 constexpr int64_t kDeadRatio = 8;
 
+bool can_append(const mrf_map* m) {
+  return !m->needs_full && m->built_version >= 0 && m->prm.activation == MRF_ACT_FULL_RAY &&
+         m->built_views <= (int)m->views.size() && m->dead_inc * (kDeadRatio + 1) <= m->n_inc * kDeadRatio;
+}
+
 void ensure_built(mrf_map* m) {
   if (m->built_version != m->version) {
-    const bool can_append = !m->needs_full && m->built_version >= 0 &&
-                            m->prm.activation == MRF_ACT_FULL_RAY && m->built_views <= (int)m->views.size() &&
-                            m->dead_inc * (kDeadRatio + 1) <= m->n_inc * kDeadRatio;
     bool done = false;
-    if (can_append) {
+    if (can_append(m)) {
       // a part-done append: the next build starts over, and the views it
       // was adding carry no pairs (their message range was never written)
       // into that build's message remap
@@ -1791,7 +1693,7 @@ void destroy_bufs(mrf_map* m) {
                  &m->pair_m, &m->pair_cum, &m->pair_stat, &m->pair_ndyn, &m->pair_hit, &m->pair_q,
                  &m->pair_dm,
                  &m->dperm, &m->dpair, &m->dseg, &m->drun,
-                 &m->ray_order, &m->ray_queue, &m->region_q, &m->rstart, &m->rcounters, &m->counters, &m->tile_first,
+                 &m->s_rg, &m->ray_queue, &m->region_q, &m->rstart, &m->rcounters, &m->counters, &m->tile_first,
                  &m->lbase, &m->lsingle, &m->lprefix, &m->queue_ids, &m->region_ids, &m->loud_off,
                  &m->loud, &m->quiet_ray,
                  &m->vseg, &m->vpairs, &m->vvox, &m->loud_ranges, &m->vox_active, &m->d_Lbase, &m->inc_len16, &m->pair_q16,
@@ -1992,6 +1894,22 @@ mrf_status mrf_test_raise_device_error(mrf_map* m) {
   });
 }
 
+// the ray records of {n_pre, n_post, k_dyn} triples
+static std::vector<RayMeta> test_records(const int32_t* records, int64_t n_pix) {
+  std::vector<RayMeta> hm((size_t)n_pix);
+  for (int64_t i = 0; i < n_pix; ++i) {
+    const int32_t* r = records + 3 * i;
+    for (int k = 0; k < 3; ++k)
+      if (r[k] < 0 || r[k] > 65535) fail(MRF_ERR_INVALID, "mrf_test_region_lists: fields must lie in [0, 65535]");
+    RayMeta me{};
+    me.n_pre = (uint16_t)r[0];
+    me.n_post = (uint16_t)r[1];
+    me.flags = (uint32_t)r[2] << 16;
+    hm[(size_t)i] = me;
+  }
+  return hm;
+}
+
 mrf_status mrf_test_region_lists(const int32_t* records, int64_t n_pix, int regions, int share, uint32_t* home,
                                  int64_t* n_home, uint32_t* starts, uint32_t* left, int64_t* n_left) {
   if (!records || n_pix < 0 || n_pix > (int64_t)0x7FFFFFFF || regions < 1 || share < 0 || share > 100 || !home ||
@@ -2000,17 +1918,7 @@ mrf_status mrf_test_region_lists(const int32_t* records, int64_t n_pix, int regi
     return MRF_ERR_INVALID;
   }
   return wrap([&] {
-    std::vector<RayMeta> hm((size_t)n_pix);
-    for (int64_t i = 0; i < n_pix; ++i) {
-      const int32_t* r = records + 3 * i;
-      for (int k = 0; k < 3; ++k)
-        if (r[k] < 0 || r[k] > 65535) fail(MRF_ERR_INVALID, "mrf_test_region_lists: fields must lie in [0, 65535]");
-      RayMeta me{};
-      me.n_pre = (uint16_t)r[0];
-      me.n_post = (uint16_t)r[1];
-      me.flags = (uint32_t)r[2] << 16;
-      hm[(size_t)i] = me;
-    }
+    const std::vector<RayMeta> hm = test_records(records, n_pix);
     View v;
     v.cam.rows = 1;
     v.cam.cols = (int)n_pix;
@@ -2024,6 +1932,60 @@ mrf_status mrf_test_region_lists(const int32_t* records, int64_t n_pix, int regi
     starts[regions] = (uint32_t)l.home.size();
     *n_home = (int64_t)l.home.size();
     *n_left = (int64_t)l.left.size();
+  });
+}
+
+mrf_status mrf_test_region_lists_device(mrf_map* m, const int32_t* records, int64_t n_pix, int n_views, int regions,
+                                        int share, uint32_t* lists, uint32_t* starts, uint32_t* lefts,
+                                        uint32_t* queue) {
+  if (guard(m) != MRF_OK) return MRF_ERR_INVALID;
+  if (!records || n_pix < 0 || n_pix > (1 << 24) || n_views < 1 || n_views > kQueueViews || regions < 1 ||
+      regions > (1 << 16) || share < 0 || share > 100 || !lists || !starts || !lefts || !queue) {
+    set_err("mrf_test_region_lists_device: invalid arguments");
+    return MRF_ERR_INVALID;
+  }
+  return wrap([&] {
+    const std::vector<RayMeta> hm = test_records(records, n_pix);
+    QueueBatch b{};
+    b.views = (uint32_t)n_views;
+    int64_t work = 0;
+    for (int v = 0; v < n_views; ++v) {
+      b.pix[v + 1] = (uint32_t)(n_pix * (v + 1) / n_views);
+      b.act[v + 1] = b.act[v];
+      for (uint32_t i = b.pix[v]; i < b.pix[v + 1]; ++i) {
+        b.act[v + 1] += ray_in_bp(hm[i]);
+        work += hm[i].n_pre;
+      }
+    }
+    u32_checked(work, "incidence count");
+    const size_t n = (size_t)std::max<int64_t>(n_pix, 1), V = (size_t)n_views, R = (size_t)regions;
+    const size_t act = b.act[n_views];
+    struct Hold {
+      DBuf b[6];
+      ~Hold() {
+        for (DBuf& x : b) x.release();
+      }
+    } h;
+    for (int k = 0; k < 3; ++k) h.b[k].reserve(n * sizeof(RayMeta), false, m->stream);
+    for (int k = 3; k < 5; ++k) h.b[k].reserve(n * 4, false, m->stream);
+    h.b[5].reserve(V * (R + 4) * 4, false, m->stream);
+    if (n_pix) CK(cudaMemcpyAsync(h.b[0].p, hm.data(), hm.size() * sizeof(RayMeta), cudaMemcpyHostToDevice, m->stream));
+    uint32_t* rows = h.b[5].as<uint32_t>();
+    batch_queues(m, b, h.b[0].as<RayMeta>(), (uint32_t)R, (uint32_t)share, 0u, 0u, h.b[1].as<RayMeta>(),
+                 h.b[3].as<uint32_t>(), h.b[2].as<RayMeta>(), h.b[4].as<uint32_t>(), rows, rows + V * (R + 1),
+                 rows + V * (R + 2));
+    std::vector<RayMeta> q(2 * act);
+    CK(cudaMemcpyAsync(q.data(), h.b[1].p, act * sizeof(RayMeta), cudaMemcpyDeviceToHost, m->stream));
+    CK(cudaMemcpyAsync(q.data() + act, h.b[2].p, act * sizeof(RayMeta), cudaMemcpyDeviceToHost, m->stream));
+    CK(cudaMemcpyAsync(queue, h.b[3].p, act * 4, cudaMemcpyDeviceToHost, m->stream));
+    CK(cudaMemcpyAsync(lists, h.b[4].p, act * 4, cudaMemcpyDeviceToHost, m->stream));
+    CK(cudaMemcpyAsync(starts, rows, V * (R + 1) * 4, cudaMemcpyDeviceToHost, m->stream));
+    CK(cudaMemcpyAsync(lefts, rows + V * (R + 1), V * 3 * 4, cudaMemcpyDeviceToHost, m->stream));
+    sync(m);
+    for (size_t k = 0; k < act; ++k)
+      if (std::memcmp(&q[k], &hm.at(queue[k]), sizeof(RayMeta)) ||
+          std::memcmp(&q[act + k], &hm.at(lists[k]), sizeof(RayMeta)))
+        fail(MRF_ERR_CUDA, "a queue's record is not its ray's");
   });
 }
 
@@ -2190,7 +2152,7 @@ mrf_status mrf_retire_view(mrf_map* m, int view_id) {
     // in the arenas is reclaimed by the next full build
     if (v.n_inc) m->holes = true;
     m->dead_inc += v.n_inc;
-    v.n_inc = v.n_pairs = v.n_dperm = v.n_dpairs = v.n_active = v.n_left = v.n_loud = 0;
+    v.n_inc = v.n_pairs = v.n_dperm = v.n_dpairs = v.n_active = v.n_loud = 0;
     m->version++;
   });
 }

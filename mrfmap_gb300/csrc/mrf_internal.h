@@ -278,11 +278,28 @@ cudaError_t launch_loud_prefix(const RayMeta* meta, uint32_t r_first, uint32_t n
 // quiet sums of the static prefixes of rays r_first..r_first+n of one view
 cudaError_t launch_quiet_prefix(const BpArrays& a, uint32_t r_first, uint32_t n, uint32_t pair_base,
                                 uint32_t n_loud, QuietRay* ray, cudaStream_t s);
-cudaError_t launch_ray_keys(const RayMeta* meta, uint32_t n, uint32_t* keys, uint32_t* vals,
+// A batch of consecutive views on their way into the ray queues: pixels
+// pix[v] .. pix[v + 1], rays in BP act[v] .. act[v + 1] of view v (mrf_bp.cu)
+constexpr int kQueueViews = 64;
+struct QueueBatch {
+  uint32_t views;
+  uint32_t pix[kQueueViews + 1], act[kQueueViews + 1];
+};
+cudaError_t launch_ray_keys(const QueueBatch& b, const RayMeta* meta, uint32_t* keys, uint32_t* vals, uint32_t* work,
                             cudaStream_t s);
-// queue[i] = meta[order[i]], ids[i] = id_base + order[i], i < n
-cudaError_t launch_ray_queue(const RayMeta* meta, const uint32_t* order, uint32_t n, RayMeta* queue,
-                             uint32_t* ids, uint32_t id_base, cudaStream_t s);
+cudaError_t launch_region_keys(const QueueBatch& b, const RayMeta* meta, const uint32_t* sorted,
+                               const uint32_t* before, uint32_t R, uint32_t* region, uint32_t* rank, RayMeta* queue,
+                               uint32_t* ids, uint32_t id_base, cudaStream_t s);
+cudaError_t launch_region_bounds(const QueueBatch& b, const uint32_t* region, const uint32_t* rank,
+                                 const uint32_t* keys, uint32_t R, uint32_t* bounds, uint32_t* work, cudaStream_t s);
+cudaError_t launch_region_home(const QueueBatch& b, const uint32_t* region, const uint32_t* rank,
+                               const uint32_t* before, const uint32_t* bounds, uint32_t share, uint32_t* flag,
+                               cudaStream_t s);
+cudaError_t launch_region_emit(const QueueBatch& b, const RayMeta* meta, const uint32_t* sorted, const uint32_t* rank,
+                               const uint32_t* place, const uint32_t* bounds, uint32_t R, uint32_t at,
+                               uint32_t id_base, RayMeta* queue, uint32_t* ids, uint32_t* rstart, uint32_t* lbase,
+                               uint32_t* lsingle, cudaStream_t s);
+cudaError_t launch_leftover_prefix(const uint32_t* lsingle, uint32_t V, uint32_t* prefix, cudaStream_t s);
 // dynamic positions k0..k1 hold the runs j0..j1 (dpair/dseg indices);
 // tile_first from launch_tile_first over dseg
 cudaError_t launch_pair_update(const BpArrays& a, uint32_t k0, uint32_t k1, uint32_t j0, uint32_t j1,
