@@ -156,6 +156,15 @@ constexpr int kG = 8;                    // lanes per ray
 constexpr int kRaysPerWarp = 32 / kG;
 constexpr int kE = 4;                    // incidences per lane of a chunk
 constexpr int kChunk = kG * kE;
+// Chunks of a full static prefix in flight, their pair ids a step ahead: the
+// prefix is a chain of a load and a gather that depends on it, and registers
+// hold the SM at 32 warps.  1 -> 2: five iterations over eight 640x480 views
+// at 2 cm 5.55 -> 5.33 ms, eight at 1 cm 24.2 -> 23.6, five 160x120 views
+// 1.137 -> 1.102; rays of endpoint bricks, shorter than a chunk, 7.62 -> 7.70.
+// Two without the ids ahead: 5.57, 24.0; three: 5.42, 23.5 (spills).  One where
+// more than 8 blocks share the registers (two would spill).
+template <int kMinBlocks>
+constexpr int kPrefixChunks = kMinBlocks > 8 ? 1 : 2;
 constexpr int kLoudPer = 4;              // loud prefix incidences in flight per lane
 
 // inclusive scan and sum over the lanes of a group (gl: lane in the group)
@@ -246,7 +255,7 @@ __device__ __forceinline__ float load_slice(Slice& s, const uint32_t (&pid)[kE],
 }
 
 // One ray per group (me.n_pre = me.n_post = 0: the group has none).
-template <int kPol, int kPf, bool kQuiet, typename TL, typename TQ>
+template <int kPol, int kPf, int kPre, bool kQuiet, typename TL, typename TQ>
 __device__ __forceinline__ void ray_bp_group(const RayMeta& me, uint32_t rid, const QuietPrefix& qp,
                                              const uint32_t* __restrict__ inc_pair,
                                              const TL* __restrict__ inc_len,
@@ -300,30 +309,35 @@ __device__ __forceinline__ void ray_bp_group(const RayMeta& me, uint32_t rid, co
     }
   } else {
     // k4 is a multiple of 4: no vector crosses it
-    uint32_t p[kE];
-    if (kPf) ld4<kPol>(p, inc_pair, off + kE * gl, kE * gl < k4);
-    for (int i = kE * gl; i < k4; i += kChunk) {
-      uint32_t c[kE];
-      float l[kE];
-      if (kPf) {
+    uint32_t p[kPre][kE];
 #pragma unroll
-        for (int j = 0; j < kE; ++j) c[j] = p[j];
-        ld4<kPol>(p, inc_pair, off + i + kChunk, i + kChunk < k4);
-      } else {
-        ld4<kPol>(c, inc_pair, off + i, true);
+    for (int u = 0; u < kPre; ++u) ld4<kPol>(p[u], inc_pair, off + kE * gl + u * kChunk, kE * gl + u * kChunk < k4);
+    for (int i = kE * gl; i < k4; i += kPre * kChunk) {
+      float l[kPre][kE], q[kPre][kE];
+#pragma unroll
+      for (int u = 0; u < kPre; ++u) {
+        ld4<kPol>(l[u], inc_len, off + i + u * kChunk, i + u * kChunk < k4);
+#pragma unroll
+        for (int j = 0; j < kE; ++j) q[u][j] = i + u * kChunk < k4 ? to_f(__ldg(lnq + p[u][j])) : 0.0f;
       }
-      ld4<kPol>(l, inc_len, off + i, true);
 #pragma unroll
-      for (int j = 0; j < kE; ++j) l[j] *= to_f(__ldg(lnq + c[j]));
-      if (i + kE <= r0) {
-        la += (l[0] + l[1]) + (l[2] + l[3]);
-      } else if (i >= r0) {
-        lb += (l[0] + l[1]) + (l[2] + l[3]);
-      } else {
+      for (int u = 0; u < kPre; ++u)
+        ld4<kPol>(p[u], inc_pair, off + i + (kPre + u) * kChunk, i + (kPre + u) * kChunk < k4);
 #pragma unroll
-        for (int j = 0; j < kE; ++j) {
-          if (i + j < r0) la += l[j];
-          else lb += l[j];
+      for (int u = 0; u < kPre; ++u) {
+#pragma unroll
+        for (int j = 0; j < kE; ++j) l[u][j] *= q[u][j];
+        const int iu = i + u * kChunk;
+        if (iu + kE <= r0) {
+          la += (l[u][0] + l[u][1]) + (l[u][2] + l[u][3]);
+        } else if (iu >= r0) {
+          lb += (l[u][0] + l[u][1]) + (l[u][2] + l[u][3]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < kE; ++j) {
+            if (iu + j < r0) la += l[u][j];
+            else lb += l[u][j];
+          }
         }
       }
     }
@@ -528,7 +542,8 @@ __global__ void __launch_bounds__(kRayWarps * 32, kMinBlocks)
     // the next tickets are taken before the current rays run, so the atomic's
     // latency hides behind their work
     idx = take(c);
-    ray_bp_group<kPol, kPf, kQuiet, TL, TQ>(me, rid, qp, inc_pair, inc_len, inc_mu, lnq, inc_pl, fix_reset, gl);
+    ray_bp_group<kPol, kPf, kPrefixChunks<kMinBlocks>, kQuiet, TL, TQ>(me, rid, qp, inc_pair, inc_len, inc_mu, lnq,
+                                                                       inc_pl, fix_reset, gl);
   }
 }
 
