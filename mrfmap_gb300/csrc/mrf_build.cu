@@ -651,9 +651,11 @@ __global__ void k_runs(const uint32_t* __restrict__ sk, const uint32_t* __restri
 // an error-free two-sum (Knuth's TwoSum: e collects every rounding error of
 // s), i.e. to about twice FP32's precision, and rounded once through FP64.
 // GB300 issues FP64 at 1/64 of the FP32 rate: plain FP64 accumulation would
-// make this kernel FP64-bound.  A thread sums a run; runs longer than
-// kLongRun (voxels next to a camera) are appended to a list and summed by a
-// whole block each.
+// make this kernel FP64-bound.  A thread sums a run, whose gathers are what it
+// waits for: eight incidences' are in flight together (the build of five
+// 160x120 views 2.46 -> 2.35 ms, of twelve 640x480 10.76 -> 10.45 against one
+// at a time).  Runs longer than kLongRun (voxels next to a camera) are appended
+// to a list and summed by a whole block each.
 constexpr uint32_t kLongRun = 512;
 constexpr int kStatThreads = 256;
 
@@ -670,6 +672,7 @@ struct F2 {
 };
 
 struct RunStats {
+  static constexpr int kAhead = 8;
   const uint32_t* dpair;
   const uint32_t* dseg;
   const uint32_t* dperm;
@@ -685,6 +688,26 @@ struct RunStats {
     const float l = len[i];
     d += len_fixed(l);
     h.add(__fmul_rn(mu[i], l));
+  }
+  // kAhead incidences from k on (k1: the run's end), added in their order,
+  // their gathers in flight together
+  __device__ __forceinline__ void add_some(uint32_t k, uint32_t k1, long long& d, F2& h) const {
+    uint32_t i[kAhead];
+    float l[kAhead], u[kAhead];
+#pragma unroll
+    for (int q = 0; q < kAhead; ++q) i[q] = dperm[min(k + q, k1 - 1)];
+#pragma unroll
+    for (int q = 0; q < kAhead; ++q) {
+      l[q] = len[i[q]];
+      u[q] = mu[i[q]];
+    }
+#pragma unroll
+    for (int q = 0; q < kAhead; ++q) {
+      if (k + q < k1) {
+        d += len_fixed(l[q]);
+        h.add(__fmul_rn(u[q], l[q]));
+      }
+    }
   }
   __device__ __forceinline__ void store(uint32_t j, uint32_t n, long long d, double h) const {
     const uint32_t p = dpair[j];
@@ -705,7 +728,7 @@ __global__ void k_run_stats(RunStats a, uint32_t j0, uint32_t nrun, uint32_t* __
   }
   long long d = 0;
   F2 h{0.0f, 0.0f};
-  for (uint32_t k = k0; k < k1; ++k) a.add(k, d, h);
+  for (uint32_t k = k0; k < k1; k += RunStats::kAhead) a.add_some(k, k1, d, h);
   a.store(j, k1 - k0, d, h.value());
 }
 
