@@ -111,8 +111,8 @@ typedef struct mrf_stats {
                               iteration of a call on */
   int64_t n_loud_prefix;   /* incidences before k4 on voxels with a dynamic
                               incidence in some view: the rest of the static
-                              prefixes is summed once per call (0 until the
-                              first call of 4 or more iterations counts them) */
+                              prefixes is summed once per call (0 until a call
+                              long enough to take them counts them) */
   int64_t quiet_prefix_used; /* 1 if the last mrf_infer took the static
                                 prefixes from their quiet sums */
   int64_t builds_oom_fallback; /* full builds run because appending the new
@@ -143,8 +143,7 @@ MRF_API int64_t mrf_memory_in_use(void);
  * MRF_ERR_DEVICE and clears it. */
 MRF_API mrf_status mrf_test_raise_device_error(mrf_map* map);
 /* Test hook, no reference counterpart: the pixels of built view view_id
- * whose rays may cross a brick in slots b0..b1 -- the footprint an appended
- * build re-checks after bricks were activated -- as mask[rows*cols] (0/1,
+ * whose rays may cross a brick in slots b0..b1, as mask[rows*cols] (0/1,
  * host) and *all (1: the footprint covers the whole image). */
 MRF_API mrf_status mrf_test_brick_footprint(mrf_map* map, int view_id, int64_t b0, int64_t b1,
                                             uint8_t* mask, int* all);

@@ -545,7 +545,7 @@ void view_pairs(mrf_map* m, int c, int64_t& pair_total, int64_t& dperm_total, in
 // afterwards, which evens out the regions' finishing times (the home share,
 // 75 % unless mrf_set_home_share or mrf_autotune_home_share chose another;
 // it moves rays between warps only, never a result).  A build makes
-// them on the device (view_regions); this is the same on the host, in linear
+// them on the device (batch_queues); this is the same on the host, in linear
 // time, to check that by: a counting sort by length feeds the regions' buckets
 // in order, so each bucket is longest first.  Pixel indices are absolute
 // (v.pix_base + i); starts are positions in home.
