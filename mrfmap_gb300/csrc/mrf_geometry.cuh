@@ -22,7 +22,7 @@ __device__ __forceinline__ float fd(float a, float b) { return __fdiv_rn(a, b); 
 // The traversal kernels give a warp 8 x 4 pixels: 32 pixels of a row span
 // several bricks a few metres out, and lanes that enter and leave their bricks
 // at different steps wait for one another (15 of 32 active); the tile's rays
-// mostly share a brick.
+// mostly share a brick.  (Likelihood and renders: kViewTileX x kViewTileY.)
 template <int kTileX = 8, int kTileY = 4>
 __device__ __forceinline__ int tile_pixel(int rows, int cols, int64_t tile, int lane) {
   const int tx = (cols + kTileX - 1) / kTileX;

@@ -75,6 +75,17 @@ constexpr uint32_t kNoVoxel = 0xFFFFFFFFu;  // padding incidences
 // tiles of a rows x cols image in the traversal kernels (a warp each)
 __host__ __device__ inline int64_t pixel_tiles(int rows, int cols) { return (int64_t)((cols + 7) / 8) * ((rows + 3) / 4); }
 
+// A warp's tile in the likelihood and the renders, where a lane only gathers
+// and sums: 4 x 8 pixels hold their rays together longer than 8 x 4 (expected
+// depth 320x240 381 -> 364 us, 640x480 682 -> 659; labels 231 to 392 -> 219 to
+// 371; likelihood 640x480 at 1 cm 663 -> 636, host calls; blocks of 64 or 32
+// threads no better).  The emit pass, whose rows of pixels also share the
+// sectors it writes, is 5 % slower with it.
+constexpr int kViewTileX = 4, kViewTileY = 8;
+__host__ __device__ inline int64_t image_tiles(int rows, int cols) {
+  return (int64_t)((cols + kViewTileX - 1) / kViewTileX) * ((rows + kViewTileY - 1) / kViewTileY);
+}
+
 // A ray's bricks are dealt to kSplit lanes where an image alone leaves the SMs
 // short of warps: a ray takes as long as its voxels' dependent steps.  Every
 // lane walks all bricks, whole bricks at a time, and the lanes' parts are put

@@ -15,7 +15,8 @@ constexpr int kLikeThreads = 128;
 __global__ void __launch_bounds__(kLikeThreads)
     k_likelihood(Geom g, Pose P, const float* __restrict__ depth, const float* __restrict__ belief,
                  float* __restrict__ out_img, double* __restrict__ partials) {
-  const int pix = tile_pixel(g.rows, g.cols, (blockIdx.x * (int64_t)kLikeThreads + threadIdx.x) >> 5, threadIdx.x & 31);
+  const int pix = tile_pixel<kViewTileX, kViewTileY>(
+      g.rows, g.cols, (blockIdx.x * (int64_t)kLikeThreads + threadIdx.x) >> 5, threadIdx.x & 31);
   float val = 0.0f;
   if (pix >= 0) {
     float d = depth[pix];
@@ -63,7 +64,7 @@ __global__ void k_reduce_partials(const double* __restrict__ partials, int n, fl
 int likelihood_blocks(const Geom& g, int num_sms) {
   constexpr int kTiles = kLikeThreads / 32;
   const int64_t tiles = split_rays(g.rows, g.cols, num_sms) ? (int64_t)((g.cols + 3) / 4) * ((g.rows + 1) / 2)
-                                                            : pixel_tiles(g.rows, g.cols);
+                                                            : image_tiles(g.rows, g.cols);
   return (int)((tiles + kTiles - 1) / kTiles);
 }
 

@@ -92,11 +92,11 @@ __global__ void __launch_bounds__(kNoAllocThreads)
     k_likelihood_noalloc(Geom g, Pose P, const float* __restrict__ depth,
                          const float* __restrict__ belief, float* __restrict__ out_img,
                          double* __restrict__ partials) {
-  const int64_t tiles = pixel_tiles(g.rows, g.cols);
+  const int64_t tiles = image_tiles(g.rows, g.cols);
   double sum = 0.0;
   for (int64_t tile = (blockIdx.x * (int64_t)kNoAllocThreads + threadIdx.x) >> 5; tile < tiles;
        tile += gridDim.x * (int64_t)(kNoAllocThreads / 32)) {
-    const int pix = tile_pixel(g.rows, g.cols, tile, threadIdx.x & 31);
+    const int pix = tile_pixel<kViewTileX, kViewTileY>(g.rows, g.cols, tile, threadIdx.x & 31);
     if (pix < 0) continue;
     const float d = clean_depth_value(depth[pix], pix, g.rows, g.cols);
     const float val = d > 0.0f ? likelihood_pixel(g, P, belief, pix, d) : 0.0f;
@@ -128,7 +128,7 @@ extern "C" MRF_API mrf_status mrf_likelihood_device_noalloc(mrf_map* map, const 
   const int64_t npix = (int64_t)g.rows * g.cols;
   constexpr int kTiles = kNoAllocThreads / 32;
   const int64_t nblocks =
-      std::min<int64_t>((pixel_tiles(g.rows, g.cols) + kTiles - 1) / kTiles, kNoAllocMaxBlocks);
+      std::min<int64_t>((image_tiles(g.rows, g.cols) + kTiles - 1) / kTiles, kNoAllocMaxBlocks);
   if (npix > (int64_t)kNoAllocMaxBlocks * kNoAllocThreads) {
     mrf_internal_set_error(
         "mrf_likelihood_device_noalloc: image larger than 524288 pixels (fixed scratch limit)");

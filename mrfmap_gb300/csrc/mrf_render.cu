@@ -165,7 +165,8 @@ __global__ void __launch_bounds__(kRenderThreads)
   if (threadIdx.x < 4) hist[threadIdx.x] = 0;
   __syncthreads();
   const int pix =
-      tile_pixel(g.rows, g.cols, (blockIdx.x * (int64_t)kRenderThreads + threadIdx.x) >> 5, threadIdx.x & 31);
+      tile_pixel<kViewTileX, kViewTileY>(g.rows, g.cols, (blockIdx.x * (int64_t)kRenderThreads + threadIdx.x) >> 5,
+                                         threadIdx.x & 31);
   if (pix >= 0) {
     float d = depth[pix];
     float v;
@@ -255,7 +256,7 @@ cudaError_t launch_render(int mode, const Geom& g, const Pose& P, const float* d
     return cudaGetLastError();
   }
   constexpr int kTiles = kRenderThreads / 32;
-  const int nb = (int)((pixel_tiles(g.rows, g.cols) + kTiles - 1) / kTiles);
+  const int nb = (int)((image_tiles(g.rows, g.cols) + kTiles - 1) / kTiles);
   switch (mode) {
     case 0: k_render<0><<<nb, kRenderThreads, 0, s>>>(g, P, depth, belief, thresh, out, counts); break;
     case 1: k_render<1><<<nb, kRenderThreads, 0, s>>>(g, P, depth, belief, thresh, out, counts); break;
