@@ -334,7 +334,7 @@ def run_reference(args):
 
 
 # bumped whenever k_ray_bp's memory traffic changes (profiles/ray_bp_traffic.json)
-RAY_KERNEL_VERSION = 7
+RAY_KERNEL_VERSION = 8
 
 
 HOME_SHARES = (60, 75, 90)  # per cent of an SM region's work on its home blocks, tried by the autotuner
