@@ -96,7 +96,10 @@ __device__ __forceinline__ float likelihood_pixel(const Geom& g, const Pose& P,
   return logf(sum);
 }
 
-// exclusive prefix and total over the kSplit lanes of a ray (mask: those lanes)
+// exclusive prefix and total over the kSplit lanes of a ray (mask: those lanes).
+// The prefix is shifted out of the inclusive scan, not formed as scan minus
+// value: a voxel of occupancy 1 makes a lane's value -inf, and behind a wall
+// (-100) the subtraction leaves 4e-6 in the exponent of the lane's own brick.
 __device__ __forceinline__ float split_prefix(float v, unsigned mask, int sub, float& total) {
   float incl = v;
 #pragma unroll
@@ -105,7 +108,8 @@ __device__ __forceinline__ float split_prefix(float v, unsigned mask, int sub, f
     if (sub >= o) incl += u;
   }
   total = __shfl_sync(mask, incl, kSplit - 1, kSplit);
-  return incl - v;
+  const float before = __shfl_up_sync(mask, incl, 1, kSplit);
+  return sub ? before : 0.0f;
 }
 __device__ __forceinline__ float split_sum(float v, unsigned mask) {
 #pragma unroll
