@@ -48,6 +48,11 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+__device__ __forceinline__ void add4(float (&s)[4], const float (&x)[4]) {
+#pragma unroll
+  for (int r = 0; r < 4; ++r) s[r] += x[r];
+}
+
 // four 8x8 BF16 matrices; lane l gives row l % 8 of matrix l / 8
 __device__ __forceinline__ void ldm4(uint32_t (&r)[4], uint32_t addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
@@ -359,7 +364,7 @@ __global__ void __launch_bounds__(kFwdThreads, 2)
 // ldmatrix.  A training step on 512 bricks took 455 us as 17 kernels: weight
 // gradients of every brick through memory and a thread per weight over all
 // bricks 170, the loss's sum in one thread 44, operand staging most of the
-// rest.  Now 94: 33 forward, 50 here, 10 to sum the blocks.
+// rest.  Now 97: 33 forward, 52 here, 10 to sum the blocks.
 constexpr int kBwdThreads = 512;
 constexpr int kSide = 2 * 27 * kC0 * kC1 + kC1 + kC2 + 4 * 27 * kC2 + 1;  // a block's partials but W2's
 constexpr int kSideStride = (kSide + 63) / 64 * 64;
@@ -401,8 +406,11 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
   }
   // weight gradients of the warp: layer 2's taps warp and warp + 16; layer 1's
   // row tile warp % 7 over half warp / 7 of the voxels (14 warps); layer 3's
-  // taps 8 (warp % 4) .. + 7 over quarter warp / 4
-  float d2[2][2][4] = {}, d1[2][4] = {}, d3[4] = {};
+  // taps 8 (warp % 4) .. + 7 over quarter warp / 4.  The tensor cores add a
+  // product to the accumulator by truncation: a brick's 8 to 32 steps lose
+  // 1e-6, a whole block's thousands 2e-4 (18432 bricks, 122 a block).  So a
+  // brick's accumulators start at zero and are added to these, rounded.
+  float g2[2][2][4] = {}, g1[2][4] = {}, g3[4] = {};
   float db1[2][2] = {}, db2[2][2] = {}, db3 = 0.0f;
   for (int64_t b = blockIdx.x; b < nb; b += gridDim.x) {
     __syncthreads();  // the previous brick's readers
@@ -478,6 +486,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
       const int vb = (lane & 7) + 8 * ((lane >> 3) & 1), pb = lane >> 4;
       const int n_taps = warp + 16 < 27 ? 2 : 1;
       const uint32_t o0 = 16u * (uint32_t)tap_off(warp), o1 = 16u * (uint32_t)tap_off(n_taps > 1 ? warp + 16 : warp);
+      float d2[2][2][4] = {};
       for (int ks = 0; ks < 32; ++ks) {
         uint32_t a[4], bw[4];
         ldm4t(bw, saddr(sh.dz2 + pb * kHaloVox + halo_of(ks * 16 + vb)));
@@ -491,7 +500,12 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
           mma_bf16(d2[1][1], a, bw[2], bw[3]);
         }
       }
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) add4(g2[k][j], d2[k][j]);
       // layer 3's: the columns' taps at the opposite offset of dy
+      float d3[4] = {};
       const int tap = (warp & 3) * 8 + g;
       const uint32_t* dyo = sh.dy + 2 * kCentre - (tap < 27 ? tap_off(tap) : 0);
       for (int ks = (warp >> 2) * 8; ks < (warp >> 2) * 8 + 8; ++ks) {
@@ -501,6 +515,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
         const uint32_t b0 = tap < 27 ? q[0] | (q[1] << 16) : 0u, b1 = tap < 27 ? q[10] | (q[11] << 16) : 0u;
         mma_bf16(d3, a, b0, b1);
       }
+      add4(g3, d3);
     }
     __syncthreads();
     // layer 1's weights
@@ -515,6 +530,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
         ok[h] = tap < 27;
         x[h] = reinterpret_cast<const __nv_bfloat16*>(sh.f + (ok[h] ? tap_off(tap) : 0)) + k % kC0;
       }
+      float d1[2][4] = {};
       for (int ks = half * 16; ks < half * 16 + 16; ++ks) {
         uint32_t bw[4], a[4];
         ldm4t(bw, saddr(sh.dz1 + pb * 512 + ks * 16 + vb));
@@ -527,6 +543,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
         mma_bf16(d1[0], a, bw[0], bw[1]);
         mma_bf16(d1[1], a, bw[2], bw[3]);
       }
+      add4(g1[0], d1[0]);
+      add4(g1[1], d1[1]);
     }
   }
   // the block's sums
@@ -539,7 +557,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
 #pragma unroll
     for (int j = 0; j < 2; ++j)
 #pragma unroll
-      for (int r = 0; r < 4; ++r) p2[(tap * kC1 + g + 8 * (r >> 1)) * kC2 + j * 8 + 2 * t + (r & 1)] = d2[k][j][r];
+      for (int r = 0; r < 4; ++r) p2[(tap * kC1 + g + 8 * (r >> 1)) * kC2 + j * 8 + 2 * t + (r & 1)] = g2[k][j][r];
   }
   if (warp < 14) {
 #pragma unroll
@@ -547,13 +565,13 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
         const int k = (warp % 7) * 16 + g + 8 * (r >> 1);
-        if (k < 27 * kC0) ps[sW1 + ((warp / 7) * 27 * kC0 + k) * kC1 + j * 8 + 2 * t + (r & 1)] = d1[j][r];
+        if (k < 27 * kC0) ps[sW1 + ((warp / 7) * 27 * kC0 + k) * kC1 + j * 8 + 2 * t + (r & 1)] = g1[j][r];
       }
   }
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
     const int tap = (warp & 3) * 8 + 2 * t + (r & 1), c = g + 8 * (r >> 1);
-    if (tap < 27) ps[sW3 + ((warp >> 2) * 27 + tap) * kC2 + c] = d3[r];
+    if (tap < 27) ps[sW3 + ((warp >> 2) * 27 + tap) * kC2 + c] = g3[r];
   }
   // bias sums: over the lanes of a column, then the warps
 #pragma unroll
