@@ -292,7 +292,8 @@ MRF_API mrf_status mrf_warm_features(mrf_map* map, float* feat_dev);
  * W1[27][4][16] b1[16] W2[27][16][16] b2[16] W3[27][16][1] b3[1], tap =
  * (dx*3 + dy)*3 + dz).  Every pointer is a device pointer; stream is a
  * cudaStream_t (NULL: the default stream); workspace holds
- * mrf_net_workspace_bytes(n_bricks) bytes.
+ * mrf_net_workspace_bytes(n_bricks) bytes.  Arrays and workspace may start
+ * at any 4-byte boundary; features that start on 16 bytes load fastest.
  *   mrf_net_forward: out[n_bricks x 512] predicted log-odds from
  *     feat[n_bricks x 512 x 4].
  *   mrf_net_gradients: loss = sum w (y - target)^2 / norm over the voxels

@@ -77,6 +77,15 @@ __device__ __forceinline__ uint32_t pack2f(float lo, float hi) {
 __device__ __forceinline__ float lo_f(uint32_t u) { return __uint_as_float(u << 16); }
 __device__ __forceinline__ float hi_f(uint32_t u) { return __uint_as_float(u & 0xFFFF0000u); }
 
+// A voxel's four features, as one load where the array starts on 16 bytes
+// (vec); any float array is taken, a view into a tensor may start anywhere.
+__device__ __forceinline__ bool vec_ok(const float* feat) { return (reinterpret_cast<uintptr_t>(feat) & 15u) == 0; }
+__device__ __forceinline__ float4 load_feat(const float* __restrict__ feat, int64_t v, bool vec) {
+  if (vec) return reinterpret_cast<const float4*>(feat)[v];
+  const float* f = feat + 4 * v;
+  return make_float4(f[0], f[1], f[2], f[3]);
+}
+
 // halo position of voxel v's window origin; tap offsets inside the window
 __device__ __forceinline__ int halo_base(int v) { return ((v >> 6) * 10 + ((v >> 3) & 7)) * 10 + (v & 7); }
 __host__ __device__ constexpr int tap_off(int tap) { return ((tap / 9) * 10 + (tap / 3) % 3) * 10 + tap % 3; }
@@ -194,11 +203,11 @@ __global__ void __launch_bounds__(kFwdThreads, 2)
       b2[j][e] = W[oB2 + j * 8 + 2 * t + e];
     }
   const float b3 = W[oB3];
-  const float4* src = reinterpret_cast<const float4*>(feat);
+  const bool vec = vec_ok(feat);
   float4 f0 = make_float4(0, 0, 0, 0), f1 = f0;
   if (blockIdx.x < nb) {
-    f0 = src[(int64_t)blockIdx.x * 512 + tid];
-    f1 = src[(int64_t)blockIdx.x * 512 + tid + 256];
+    f0 = load_feat(feat, (int64_t)blockIdx.x * 512 + tid, vec);
+    f1 = load_feat(feat, (int64_t)blockIdx.x * 512 + tid + 256, vec);
   }
   __syncthreads();  // the halos are zero
   for (int64_t b = blockIdx.x; b < nb; b += gridDim.x) {
@@ -206,8 +215,8 @@ __global__ void __launch_bounds__(kFwdThreads, 2)
     sh.f[halo_of(tid + 256)] = make_uint2(pack2f(f1.x, f1.y), pack2f(f1.z, f1.w));
     __syncthreads();
     if (b + gridDim.x < nb) {  // the next brick's features, while this one runs
-      f0 = src[(b + gridDim.x) * 512 + tid];
-      f1 = src[(b + gridDim.x) * 512 + tid + 256];
+      f0 = load_feat(feat, (b + gridDim.x) * 512 + tid, vec);
+      f1 = load_feat(feat, (b + gridDim.x) * 512 + tid + 256, vec);
     }
     float acc[4][2][4];
     // layer 1: k = tap * 4 + channel; a lane's words: taps 4 ks + t / 2 and + 2
@@ -412,13 +421,14 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
   // brick's accumulators start at zero and are added to these, rounded.
   float g2[2][2][4] = {}, g1[2][4] = {}, g3[4] = {};
   float db1[2][2] = {}, db2[2][2] = {}, db3 = 0.0f;
+  const bool vec = vec_ok(feat);
   for (int64_t b = blockIdx.x; b < nb; b += gridDim.x) {
     __syncthreads();  // the previous brick's readers
     {
       const int v = tid, h = halo_of(v);
       const uint4* p1 = reinterpret_cast<const uint4*>(g_a1) + (b * 512 + v) * 2;
       const uint4* p2 = reinterpret_cast<const uint4*>(g_a2) + (b * 512 + v) * 2;
-      const float4 f = reinterpret_cast<const float4*>(feat)[b * 512 + v];
+      const float4 f = load_feat(feat, b * 512 + v, vec);
       const __nv_bfloat16 dy = __float2bfloat16_rn(g_dy[b * 512 + v]);
       sh.a1[h] = p1[0];
       sh.a1[kHaloVox + h] = p1[1];
@@ -693,16 +703,18 @@ __global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float
 // The workspace: activations, the output gradient, the blocks' partial sums
 // (layer 2's in part; the others in side, two activations' room per brick, of
 // which a block of at least one brick needs kSideStride floats) and the loss
-// per brick.
+// per brick.  It may start at any float: the base is rounded up to the 16
+// bytes that the activations' loads want, into the room at the end.
 struct Work {
   __nv_bfloat16 *a1, *a2;
-  float *side, *y, *dy, *part, *lpart;
+  float *side, *dy, *part, *lpart;
 };
 static_assert(kSideStride * 4 <= 2 * 512 * kC1 * 2, "a block's partials fit a brick's room");
 
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 inline size_t work_bytes(int64_t nb, Work* w, char* base) {
+  base = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(base) + 15) & ~(uintptr_t)15);
   size_t off = 0;
   auto take = [&](size_t bytes) {
     char* p = base ? base + off : nullptr;
@@ -714,16 +726,15 @@ inline size_t work_bytes(int64_t nb, Work* w, char* base) {
   char* a2 = take(vox * kC2 * 2);
   char* side = take(vox * kC2 * 2);
   take(vox * kC1 * 2);
-  char* y = take(vox * 4);
   char* dy = take(vox * 4);
   char* part = take((size_t)nb * 27 * kC1 * kC2 * 4);
-  take((size_t)nb * kC1 * 4);
   char* lpart = take((size_t)nb * 4);
+  take(vox * 4);
+  take((size_t)nb * kC1 * 4);
   if (w) {
     w->a1 = reinterpret_cast<__nv_bfloat16*>(a1);
     w->a2 = reinterpret_cast<__nv_bfloat16*>(a2);
     w->side = reinterpret_cast<float*>(side);
-    w->y = reinterpret_cast<float*>(y);
     w->dy = reinterpret_cast<float*>(dy);
     w->part = reinterpret_cast<float*>(part);
     w->lpart = reinterpret_cast<float*>(lpart);
