@@ -312,9 +312,13 @@ MRF_API mrf_status mrf_net_adam(float* params, const float* grads, float* m1, fl
 /* Autotuner (no reference counterpart).  The ray-message kernel comes in
  * variants that differ in the cache policy of its streamed loads, in
  * whether a chunk's pair ids are requested one chunk ahead, in the ray
- * schedule (longest first or SM regions) and in the register budget (a
- * 12-block-per-SM target caps a thread at 40 registers); their arithmetic
- * is identical, so the choice never changes a result.
+ * schedule (longest first or SM regions) and in the register budget (7, 8 or
+ * 10 resident blocks per SM); their arithmetic is identical, so the choice
+ * never changes a result.  A launch over one view (Gauss-Seidel, and Jacobi
+ * on a map of one view) runs variant 4 unless told otherwise, a launch over
+ * several (Jacobi) variant 1.  mrf_set_ray_variant and the autotuners choose
+ * for both; the _flags forms set and report one of them (MRF_JACOBI in
+ * flags: launches over several views), which is what to save and restore.
  * The pair reduction has two variants as well (one or two pairs' records
  * requested ahead per thread, at 8 or 5 resident blocks per SM), with the
  * same arithmetic; mrf_autotune times both after choosing the ray variant
@@ -326,6 +330,8 @@ MRF_API mrf_status mrf_net_adam(float* params, const float* grads, float* m1, fl
  * ms_out[0..min(cap, mrf_ray_variants())). */
 MRF_API int mrf_ray_variants(void);
 MRF_API mrf_status mrf_set_ray_variant(mrf_map* map, int variant);
+MRF_API mrf_status mrf_set_ray_variant_flags(mrf_map* map, int flags, int variant);
+MRF_API mrf_status mrf_get_ray_variant_flags(mrf_map* map, int flags, int* variant);
 MRF_API mrf_status mrf_autotune(mrf_map* map, int reps, double* ms_out, int cap, int* chosen);
 /* The same with the schedule of the timed iterations in flags (MRF_JACOBI:
  * Jacobi iterations, one ray launch over every view; else Gauss-Seidel). */
@@ -338,11 +344,15 @@ MRF_API mrf_status mrf_autotune_flags(mrf_map* map, int reps, int flags, double*
  * results do not change.  mrf_autotune_home_share times `n` shares
  * (1..100) on this map's lists (reps iterations each after a warm-up, the
  * map state restored after each), keeps the fastest, and returns the
- * per-share milliseconds per iteration in ms_out[0..n) (may be NULL).
+ * per-share milliseconds per iteration in ms_out[0..n) (may be NULL).  With
+ * MRF_JACOBI it times Jacobi iterations where their variant uses the regions;
+ * where it does not, their time does not depend on the share, and it times
+ * Gauss-Seidel iterations, which the share then governs.
  * The pair-update tile and the ray chunk are not tuned: both change the
  * order of floating-point sums, and a choice made from timings would make
  * results differ from run to run.  mrf_get_tuning reports the current
- * ray-kernel variant, home share and pair-reduction variant. */
+ * ray-kernel variant of launches over one view, home share and pair-reduction
+ * variant. */
 MRF_API mrf_status mrf_set_home_share(mrf_map* map, int percent);
 MRF_API mrf_status mrf_autotune_home_share(mrf_map* map, int reps, int flags, const int* shares, int n,
                                            double* ms_out, int* chosen);

@@ -1243,6 +1243,8 @@ int resident_of(K kernel) {
 }
 }  // namespace
 
+bool ray_bp_regions(int variant) { return variant >= 0 && variant < kRayVariants && kRayRegions[variant]; }
+
 int ray_bp_resident_blocks(int variant, int half_streams, int quiet) {
   static int resident[2][2][kRayVariants] = {{{0}}};
   if (variant < 0 || variant >= kRayVariants) return 1;

@@ -181,14 +181,15 @@ struct mrf_map {
   int64_t nb_grid = 0, n_bricks = 0;
   std::vector<int> h_coord;
   int version = 0, built_version = -1;
-  // ray-kernel variant: the caller's (mrf_autotune / mrf_set_ray_variant) once
-  // chosen, else 4 (SM regions, pair-id prefetch), and 1 (longest first) for a
-  // launch over several views: its V x R regions are served one after the
-  // other and end unevenly (Jacobi iteration of 32 views at 2 cm: 1.43 ms
-  // with 1, 1.84 with 4; Gauss-Seidel, 8 x 640x480 at 1 cm: 2.15 and 2.07)
-  int ray_variant = 4;
-  bool ray_variant_chosen = false;
-  int variant_for(bool all_views) const { return ray_variant_chosen || !all_views ? ray_variant : 1; }
+  // Ray-kernel variants of launches over one view and over several, unless the
+  // caller chose (mrf_autotune, mrf_set_ray_variant): 4 (SM regions, pair-id
+  // prefetch), and 1 (longest first).  Over several views neither always wins.
+  // Their V x R regions are served one after the other, which ends unevenly
+  // where the views differ.  Jacobi iteration with 1 and 4, ms: 2 scenes of 4
+  // views of mixed sizes 0.19 and 0.35, 8 scenes 1.03 and 1.19, 8 views of
+  // mixed sizes in a room 0.59 and 0.88; but 8 views of 640x480 there 1.22 and
+  // 1.15, at 4 cm 1.08 and 0.95.  1 risks less: at most 1.45x against 2.1x.
+  int ray_variant[2] = {4, 1};
   uint32_t nreg = 1;    // SM regions per view of the region queues
   // what the last build left: views with lists, per-pixel entries, the ends
   // of the region blocks, the queues and the tiles
@@ -1442,7 +1443,7 @@ void enqueue_iteration(mrf_map* m, const BpArrays& a, bool jacobi, int fix, int 
                              m->stream));
       prof.end();
       prof.begin(1);
-      CK(launch_ray_bp(a, ray_work(m, c), fix, m->num_sms, m->variant_for(false), quiet && phase >= 2, m->stream));
+      CK(launch_ray_bp(a, ray_work(m, c), fix, m->num_sms, m->ray_variant[0], quiet && phase >= 2, m->stream));
       prof.end();
       prof.begin(2);
       if (v.n_dperm) {
@@ -1469,7 +1470,7 @@ void enqueue_iteration(mrf_map* m, const BpArrays& a, bool jacobi, int fix, int 
     prof.end();
     prof.begin(1);
     // the queues of all views are contiguous: one launch over all rays
-    CK(launch_ray_bp(a, ray_work(m, -1), fix, m->num_sms, m->variant_for(V > 1), quiet && phase >= 2, m->stream));
+    CK(launch_ray_bp(a, ray_work(m, -1), fix, m->num_sms, m->ray_variant[V > 1], quiet && phase >= 2, m->stream));
     prof.end();
     prof.begin(2);
     CK(launch_pair_update(a, 0, (uint32_t)m->n_dperm, 0, (uint32_t)m->n_dpairs,
@@ -2233,7 +2234,7 @@ static void warm_start_impl(mrf_map* m, const float* L_pred, bool device_ptr, in
   for (int k = 0; k < sweeps; ++k) {
     zero_counters(m);
     CK(launch_pair_prepare(a, 0, P, 1, m->stream));
-    CK(launch_ray_bp(a, ray_work(m, -1), 0, m->num_sms, m->variant_for(V > 1), false, m->stream));
+    CK(launch_ray_bp(a, ray_work(m, -1), 0, m->num_sms, m->ray_variant[V > 1], false, m->stream));
     CK(launch_pair_update(a, 0, (uint32_t)m->n_dperm, 0, (uint32_t)m->n_dpairs,
                           m->tile_first.as<uint32_t>() + m->jac_tile_base, 1, m->stream));
   }
@@ -2374,9 +2375,29 @@ mrf_status mrf_set_ray_variant(mrf_map* m, int variant) {
     set_err("invalid ray-kernel variant");
     return MRF_ERR_INVALID;
   }
-  m->ray_variant = variant;
-  m->ray_variant_chosen = true;
+  m->ray_variant[0] = m->ray_variant[1] = variant;
   drop_graphs(m);
+  return MRF_OK;
+}
+
+mrf_status mrf_set_ray_variant_flags(mrf_map* m, int flags, int variant) {
+  if (guard(m) != MRF_OK) return MRF_ERR_INVALID;
+  if (variant < 0 || variant >= ray_bp_variants()) {
+    set_err("invalid ray-kernel variant");
+    return MRF_ERR_INVALID;
+  }
+  m->ray_variant[(flags & MRF_JACOBI) ? 1 : 0] = variant;
+  drop_graphs(m);
+  return MRF_OK;
+}
+
+mrf_status mrf_get_ray_variant_flags(mrf_map* m, int flags, int* variant) {
+  if (guard(m) != MRF_OK) return MRF_ERR_INVALID;
+  if (!variant) {
+    set_err("null argument");
+    return MRF_ERR_INVALID;
+  }
+  *variant = m->ray_variant[(flags & MRF_JACOBI) ? 1 : 0];
   return MRF_OK;
 }
 
@@ -2438,7 +2459,7 @@ mrf_status mrf_set_pair_variant(mrf_map* m, int variant) {
 
 mrf_status mrf_get_tuning(mrf_map* m, int* ray_variant, int* home_share, int* pair_variant) {
   if (guard(m) != MRF_OK) return MRF_ERR_INVALID;
-  if (ray_variant) *ray_variant = m->ray_variant;
+  if (ray_variant) *ray_variant = m->ray_variant[0];
   if (home_share) *home_share = m->home_share;
   if (pair_variant) *pair_variant = m->pair_variant;
   return MRF_OK;
@@ -2463,12 +2484,15 @@ mrf_status mrf_autotune_home_share(mrf_map* m, int reps, int flags, const int* s
     else
       ensure_built(m);
     if (jacobi && m->jacobi_version != m->built_version) build_jacobi_csr(m);
+    // the launches that the share governs: Jacobi iterations whose variant
+    // reads no regions run the same whatever the share
+    const bool regions = jacobi && ray_bp_regions(m->ray_variant[m->views.size() > 1]);
     std::vector<double> ms((size_t)n, 0.0);
     for (int k = 0; k < n; ++k) {
       m->home_share = shares[k];
       rebuild_regions(m);
       drop_graphs(m);
-      ms[(size_t)k] = time_schedule(m, jacobi, reps);
+      ms[(size_t)k] = time_schedule(m, regions, reps);
     }
     int best = 0;
     for (int k = 1; k < n; ++k)
@@ -2514,14 +2538,12 @@ mrf_status mrf_autotune_flags(mrf_map* m, int reps, int flags, double* ms_out, i
       CK(cudaMemcpyAsync(snap, m->d_L.p, nv, cudaMemcpyDeviceToDevice, m->stream));
       CK(cudaMemcpyAsync(snap + nv, m->d_belief.p, nv, cudaMemcpyDeviceToDevice, m->stream));
       CK(cudaMemcpyAsync(snap + 2 * nv, m->pair_m.p, npb, cudaMemcpyDeviceToDevice, m->stream));
-      const int keep = m->ray_variant;
-      const bool keep_chosen = m->ray_variant_chosen;
-      m->ray_variant_chosen = true;
+      const int keep[2] = {m->ray_variant[0], m->ray_variant[1]};
       Profiler off{m, false};
       int64_t launches = 0;
       if (quiet) quiet_prefix_all(m, a);
       for (int k = 0; k < NV; ++k) {
-        m->ray_variant = k;
+        m->ray_variant[0] = m->ray_variant[1] = k;
         for (int r = 0; r <= reps; ++r) {
           if (r == 1) CK(cudaEventRecord(m->ev0, m->stream));
           enqueue_iteration(m, a, jacobi, 0, 2, quiet, off, launches);
@@ -2535,16 +2557,15 @@ mrf_status mrf_autotune_flags(mrf_map* m, int reps, int flags, double* ms_out, i
         CK(cudaMemcpyAsync(m->d_belief.p, snap + nv, nv, cudaMemcpyDeviceToDevice, m->stream));
         CK(cudaMemcpyAsync(m->pair_m.p, snap + 2 * nv, npb, cudaMemcpyDeviceToDevice, m->stream));
       }
-      m->ray_variant = keep;
-      m->ray_variant_chosen = keep_chosen;
+      m->ray_variant[0] = keep[0];
+      m->ray_variant[1] = keep[1];
       sync(m);
     }
     int best = 0;
     for (int k = 1; k < NV; ++k)
       if (ms[k] < ms[best]) best = k;
     for (int k = 0; k < NV && k < cap; ++k) ms_out[k] = ms[k];
-    m->ray_variant = best;
-    m->ray_variant_chosen = true;
+    m->ray_variant[0] = m->ray_variant[1] = best;
     drop_graphs(m);
     // then the pair reduction's variant with that ray kernel
     if (m->n_inc > 0) {

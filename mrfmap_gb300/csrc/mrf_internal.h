@@ -245,6 +245,8 @@ cudaError_t launch_pair_prepare_loud(const BpArrays& a, const uint32_t* prefix, 
                                      uint32_t n, cudaStream_t s);
 // ray-kernel variants (register budget x load policy; identical arithmetic)
 int ray_bp_variants();
+// whether a variant takes its rays from the SM regions
+bool ray_bp_regions(int variant);
 // resident blocks per SM of a variant of the persistent ray kernel (queried once)
 int ray_bp_resident_blocks(int variant, int half_streams, int quiet);
 // fp32 -> fp16, round to nearest

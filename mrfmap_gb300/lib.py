@@ -38,7 +38,7 @@ EXPORTS = ["mrf_create", "mrf_destroy", "mrf_release_cached_memory", "mrf_last_e
            "mrf_set_pose", "mrf_infer", "mrf_infer_converge", "mrf_warm_start", "mrf_warm_start_device",
            "mrf_warm_features", "mrf_read_messages", "mrf_write_messages", "mrf_rebuild_logodds", "mrf_net_num_params", "mrf_net_workspace_bytes", "mrf_net_forward",
            "mrf_net_gradients", "mrf_net_adam",
-           "mrf_ray_variants", "mrf_set_ray_variant",
+           "mrf_ray_variants", "mrf_set_ray_variant", "mrf_set_ray_variant_flags", "mrf_get_ray_variant_flags",
            "mrf_autotune", "mrf_reset_state", "mrf_likelihood_view", "mrf_likelihood",
            "mrf_likelihood_device", "mrf_likelihood_device_noalloc", "mrf_num_bricks", "mrf_read_bricks", "mrf_read_logodds",
            "mrf_num_nodes", "mrf_read_nodes", "mrf_load_map", "mrf_view_incidences",
@@ -128,6 +128,8 @@ def load(path: str | None = None):
                           C.c_float, C.c_float, C.c_int, C.c_void_p], C.c_int),
         "mrf_ray_variants": ([], C.c_int),
         "mrf_set_ray_variant": ([vp, C.c_int], C.c_int),
+        "mrf_set_ray_variant_flags": ([vp, C.c_int, C.c_int], C.c_int),
+        "mrf_get_ray_variant_flags": ([vp, C.c_int, ip], C.c_int),
         "mrf_autotune": ([vp, C.c_int, C.POINTER(C.c_double), C.c_int, ip], C.c_int),
         "mrf_reset_state": ([vp], C.c_int),
         "mrf_likelihood_view": ([vp, C.c_int, fp, fp], C.c_int),
@@ -363,8 +365,19 @@ class MRFMap:
         and ln q gathers in the ray kernel)."""
         _check(self._L.mrf_set_precision(self._h, mode))
 
-    def set_ray_variant(self, variant: int):
-        _check(self._L.mrf_set_ray_variant(self._h, variant))
+    def set_ray_variant(self, variant: int, flags: int | None = None):
+        """For every launch, or for the launches of the schedule in flags
+        (JACOBI: those over several views, else those over one)."""
+        if flags is None:
+            _check(self._L.mrf_set_ray_variant(self._h, variant))
+        else:
+            _check(self._L.mrf_set_ray_variant_flags(self._h, flags, variant))
+
+    def ray_variant(self, flags: int = 0) -> int:
+        """The variant that the launches of the schedule in flags run."""
+        v = C.c_int()
+        _check(self._L.mrf_get_ray_variant_flags(self._h, flags, C.byref(v)))
+        return v.value
 
     def autotune(self, reps: int = 3, flags: int = 0):
         """Times every ray-kernel variant on this map (iterations of the
@@ -398,7 +411,8 @@ class MRFMap:
         _check(self._L.mrf_set_pair_variant(self._h, variant))
 
     def tuning(self):
-        """(ray-kernel variant, home share, pair-reduction variant) in use."""
+        """(ray-kernel variant of launches over one view, home share,
+        pair-reduction variant) in use."""
         v, h, p = C.c_int(), C.c_int(), C.c_int()
         _check(self._L.mrf_get_tuning(self._h, C.byref(v), C.byref(h), C.byref(p)))
         return v.value, h.value, p.value
