@@ -51,8 +51,7 @@ typedef enum {
                                captured CUDA graph of one iteration */
 #define MRF_FULL_RAYS 64    /* read every ray's whole Pre range in every iteration
                                (no static prefixes from their quiet sums; by default
-                               a call of 8 or more iterations, of 4 or more once the
-                               current lists were split for one, takes them from the
+                               a call of 8 or more iterations takes them from the
                                third iteration on when the quiet incidences are at
                                least half of the Pre incidences and average at
                                least 48 per ray) */

@@ -876,17 +876,23 @@ void emit_loud_lists(mrf_map* m) {
 // their quiet sums from its third iteration on.  Per iteration that saves the
 // gathers of the quiet incidences; it costs a pass over the static prefixes
 // per call (the quiet sums), and two more when the current build has no loud
-// lists yet: the call must be long enough for either (8 x 640x480 at 1 cm:
-// 0.10 ms a view and iteration saved, 0.17 and 0.36 spent), the quiet
-// incidences at least half of the Pre incidences, and on average enough per
-// ray to outweigh the records (5 x 160x120 at 4 cm, 70 a ray: iteration 0.19
-// -> 0.16 ms; 32 views of 8 scenes at 2 cm, 100 a ray: 1.43 -> 1.24).
+// lists yet.  The two paths round differently, so the rule looks at the build
+// and the call only, not at whether an earlier call has made the lists: a call
+// gives the same bits whatever came before it.  Hence one count of iterations,
+// from which a first call about breaks even: 4 views of 640x480, first call and
+// repeated call, ms in full and with the sums: at 1 cm (382 quiet incidences a
+// ray) 7 iterations 9.56 and 9.50, 9.54 and 8.10; 8 iterations 10.82 and 10.34,
+// 10.81 and 8.95; at 2 cm (190) 8 iterations 5.32 and 5.70, 5.26 and 4.82; 12
+// iterations 7.90 and 7.68, 7.80 and 6.76.  The quiet incidences must be at
+// least half of the Pre incidences, and on average enough per ray to outweigh
+// the records (5 x 160x120 at 4 cm, 70 a ray: iteration 0.19 -> 0.16 ms; 32
+// views of 8 scenes at 2 cm, 100 a ray: 1.43 -> 1.24).
 constexpr int64_t kQuietPerRay = 48;
-constexpr int64_t kQuietIters = 4, kQuietItersNew = 8;
+constexpr int64_t kQuietIters = 8;
 bool quiet_path(mrf_map* m, int64_t iters, int flags) {
   const bool force = (flags & MRF_QUIET_PREFIX) != 0;
   if ((flags & MRF_FULL_RAYS) || m->n_inc <= 0 || m->npix_total <= 0) return false;
-  if (iters < (force ? 3 : (m->loud_list_version == m->built_version ? kQuietIters : kQuietItersNew))) return false;
+  if (iters < (force ? 3 : kQuietIters)) return false;
   const int64_t pre = m->stats.n_inc_pre_bp, k4 = m->stats.n_inc_from_k4, rays = m->stats.n_rays_bp;
   if (!force && (rays <= 0 || pre - k4 < kQuietPerRay * rays)) return false;  // no count needed
   if (m->loud_count_version != m->built_version) {
