@@ -373,9 +373,10 @@ def ray_kernel_bytes(st, iters, half=False):
       once per call, the quiet sums of the static prefixes [0, k4): per
         incidence pair id, fp32 length and gather (8 + g); per ray 16 B;
       every later iteration (fast path): per incidence from k4 on 4 + l + g;
-        per loud prefix incidence pair id, fp32 length, position and gather
-        (10 + g); per dynamic incidence +8 B; per ray 36 B (metadata 16,
-        ray index 4, quiet sums 8, list bounds 8)."""
+        per loud prefix incidence 10 + g (pair id, fp32 length and gather;
+        2 more than an entry takes now, kept so that reports compare); per
+        dynamic incidence +8 B; per ray 36 B (metadata 16, ray index 4,
+        quiet sums and list bounds 16)."""
     g = 2 if half else 4
     ln = 2 if half else 4
     pre, k4, loud = st["n_inc_pre_bp"], st["n_inc_from_k4"], st["n_loud_prefix"]

@@ -300,7 +300,8 @@ void check_device_err(mrf_map* m) {
   int e = read1(m, m->s_err.as<int>());
   if (e) {
     CK(cudaMemsetAsync(m->s_err.p, 0, sizeof(int), m->stream));
-    fail(MRF_ERR_DEVICE, "a kernel raised its error flag (ray longer than 65532 incidences)");
+    fail(MRF_ERR_DEVICE, e & 1 ? "a kernel raised its error flag (ray longer than 65532 incidences)"
+                               : "a kernel raised its error flag (a ray's list does not match its count)");
   }
 }
 
@@ -835,8 +836,8 @@ void view_tiles(mrf_map* m, int c, uint32_t tb) {
 
 // The loud lists of the static prefixes of every live view's queued rays
 // (npix pixel records in meta): counts per ray, one scan over all pixels,
-// then the lists (pair id, length, position) -- the data the ray kernel's
-// fast path gathers every iteration, and room for the quiet sums.
+// then the lists (pair id, length) -- the data the ray kernel's fast path
+// gathers every iteration, and room for the quiet sums.
 void count_loud_lists(mrf_map* m) {
   const int64_t npix = m->npix_total;
   m->loud_off.reserve((size_t)(npix + 1) * 4, false, m->stream);
@@ -885,8 +886,11 @@ void emit_loud_lists(mrf_map* m) {
 // 10.81 and 8.95; at 2 cm (190) 8 iterations 5.32 and 5.70, 5.26 and 4.82; 12
 // iterations 7.90 and 7.68, 7.80 and 6.76.  The quiet incidences must be at
 // least half of the Pre incidences, and on average enough per ray to outweigh
-// the records (5 x 160x120 at 4 cm, 70 a ray: iteration 0.19 -> 0.16 ms; 32
-// views of 8 scenes at 2 cm, 100 a ray: 1.43 -> 1.24).
+// the records.  12 iterations in full and with the sums, ms: 5 x 160x120 with
+// 107 a ray 1.56 and 1.43, with 71 1.19 and 1.11, with 53 1.01 and 1.04; 4 x
+// 640x480 with 94 5.26 and 5.05, with 62 4.51 and 4.49, with 47 4.16 and 4.23.
+// Near the line a long call gains a few per cent and a short one loses as much
+// (one iteration with 47 a ray 0.342 and 0.320, with 53 0.080 and 0.078).
 constexpr int64_t kQuietPerRay = 48;
 constexpr int64_t kQuietIters = 8;
 bool quiet_path(mrf_map* m, int64_t iters, int flags) {
@@ -936,8 +940,8 @@ void rebuild_lists(mrf_map* m, OldPairs& old) {
   DBuf& old_vox = old.vox;
   DBuf& old_m = old.m;
   const std::vector<View>& old_views = old.views;
-  // 1. counts of every pixel of every live view, one scan per view ->
-  //    offsets (totals in 64 bits: a wrapped total would size the arenas
+  // 1. counts of every pixel of every live view, one scan over all of them
+  //    -> offsets (totals in 64 bits: a wrapped total would size the arenas
   //    too small for the emit pass)
   std::vector<int> live;
   for (int c = 0; c < V; ++c) {
@@ -1012,9 +1016,8 @@ void rebuild_lists(mrf_map* m, OldPairs& old) {
   m->pair_dm.reserve(pb * 4, false, m->stream);
   CK(launch_fill_f32(m->pair_m.as<float>(), pair_total, 0.0f, m->stream));
   {
-    // tile carries of the pair update: enough for any view or all of them;
-    // first pair of every tile, per view (Gauss-Seidel) and over all views
-    // (Jacobi)
+    // first pair of every tile of the pair update, per view (Gauss-Seidel)
+    // and over all views (Jacobi)
     int64_t tiles = (int64_t)pair_update_tiles((uint32_t)std::min<int64_t>(dperm_total, 0xFFFFFFF0ll)) + V + 1;
     m->tile_first.reserve((size_t)(2 * tiles + 2) * 4, false, m->stream);
     uint32_t tb = 0;
@@ -1183,8 +1186,7 @@ void append_lists(mrf_map* m) {
   m->pair_q.reserve(pb * 4, false, m->stream);
   m->pair_dm.reserve(pb * 4, false, m->stream);
   CK(launch_fill_f32(m->pair_m.as<float>() + pair0, pair_total - pair0, 0.0f, m->stream));
-  // tiles of the new views at the end of tile_first; the carries sized for
-  // the largest launch
+  // tiles of the new views at the end of tile_first
   {
     int64_t need = m->tile_end;
     for (int c = m->built_views; c < V; ++c) need += pair_update_tiles(m->views[c].n_dperm) + 1;
