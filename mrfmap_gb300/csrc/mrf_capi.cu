@@ -1278,9 +1278,10 @@ void build_jacobi_csr(mrf_map* m) {
 void ensure_built(mrf_map* m);
 
 // the all-view structures (Jacobi queues and tiles, the voxel CSR) need
-// one full build with no retired views' data in the arenas
+// one full build with no retired views' data in the arenas: also where the
+// lists are out of date, whose next build might append
 void ensure_compact(mrf_map* m) {
-  if (m->holes || m->appended) {
+  if (m->holes || m->appended || m->built_version != m->version) {
     m->needs_full = true;
     m->version++;
   }
